@@ -423,8 +423,8 @@ typedef struct lvg_stats {
    * run: with the local-moving phase replayed as one graph, a dynamic-frontier
    * run that ends after one pass waits once). */
   uint64_t host_syncs;
-  /* Aggregated levels whose local-moving iterations after the first ran as
-   * one graph launch (lvg_tuning.level_graphs). */
+  /* Local-moving phases whose iterations (all, or those after the first) ran
+   * as one launch (lvg_tuning.level_graphs). */
   uint64_t level_graphs;
 } lvg_stats;
 /* Enable (1) or disable (0) per-launch event timing for calls on g. */
@@ -465,11 +465,13 @@ typedef struct lvg_tuning {
                                   to the previous bin's empties the bin. Entries 0, 10 and 11
                                   are 0 (bin 10 ends at degree 8192, the hubs' threshold).
                                   Same results in deterministic mode (default all 0) */
-  int      level_graphs;       /* 1: on every aggregated level, the local-moving iterations after
-                                  the first run as one CUDA graph launch (a conditional while
-                                  node with the stop test on the device) built for that level;
-                                  0: one launch sequence and one synchronisation per iteration
-                                  (same results; default 1) */
+  int      level_graphs;       /* 1: a level's local-moving phase runs as one launch with the stop
+                                  test on the device: a cooperative kernel that sweeps every
+                                  colour class of every iteration, or, on levels it does not serve
+                                  (resident hub tables, hub_chunk above 4096), the iterations
+                                  after the first as one CUDA graph (a conditional while node)
+                                  built for that level; 0: one launch sequence and one
+                                  synchronisation per iteration (same results; default 1) */
   int      small_regs;         /* registers a thread of the fused launch of degree bins 1-6
                                   (fused_small): 32 (8 resident blocks per SM, some values kept
                                   in local memory) or 64 (4 blocks per SM, none); default 64 */

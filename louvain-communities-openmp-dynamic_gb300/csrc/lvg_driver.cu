@@ -51,6 +51,7 @@ void read_counters(lvg_graph *g) {
     LVG_CUDA(cudaMemsetAsync(&g->ctr.p->err, 0, sizeof(unsigned), g->stream));
     if (e & ERR_BAD_ID) throw Error(LVG_EINVAL, "prior membership id >= span (err=" + std::to_string(e) + ")");
     if (e & ERR_WORKLIST) throw Error(LVG_ECUDA, "worklist append outside its degree bin (stale degree bins)");
+    if (e & ERR_BARRIER) throw Error(LVG_ETIMEOUT, "a grid barrier of the local-moving phase was given up");
     throw Error(LVG_ETIMEOUT, "device hash table overflow guard tripped (err=" + std::to_string(e) + ")");
   }
 }
@@ -68,7 +69,9 @@ void compute_bins(lvg_graph *g, Level &lv, const uint32_t *deg, uint32_t *list, 
 // Chunked work of degree bin 11 (see HubPlan): hubs in colour order, each
 // hub's edges cut into chunks of the graph's hub_chunk edges, each with a
 // partial region of the chunk's size. Built on the host from the hubs'
-// degrees (synchronises).
+// degrees (synchronises once), in one pinned block that goes up in one copy: a
+// batch apply rebuilds it, and eight copies from pageable vectors took most of
+// its 0.15 ms on a scale-22 R-MAT graph.
 void build_hub_plan(lvg_graph *g, Level &lv, HubPlanBuffers &hb) {
   cudaStream_t s = g->stream;
   HubPlan &P = lv.hub;
@@ -82,71 +85,102 @@ void build_hub_plan(lvg_graph *g, Level &lv, HubPlanBuffers &hb) {
   P.hub_begin[K] = H;
   P.hubs = H;
   if (!H) return;
-  hb.hub_vertex.ensure(H);
-  hb.degs.ensure(H);
+  hb.verts_degs.ensure(2 * H);
   for (int k = 0; k < K; ++k) {
     const size_t n = lv.bucket_size(k, NUM_BINS - 1);
     if (n)
-      LVG_CUDA(cudaMemcpyAsync(hb.hub_vertex.p + P.hub_begin[k], lv.bins + lv.bucket_begin(k, NUM_BINS - 1),
+      LVG_CUDA(cudaMemcpyAsync(hb.verts_degs.p + P.hub_begin[k], lv.bins + lv.bucket_begin(k, NUM_BINS - 1),
                                n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   }
-  launch_gather_u32(hb.hub_vertex.p, H, lv.deg, hb.degs.p, s);
-  std::vector<uint32_t> degs(H), verts(H), first(H + 1);
-  LVG_CUDA(cudaMemcpyAsync(degs.data(), hb.degs.p, H * 4, cudaMemcpyDeviceToHost, s));
-  LVG_CUDA(cudaMemcpyAsync(verts.data(), hb.hub_vertex.p, H * 4, cudaMemcpyDeviceToHost, s));
-  host_sync(g);
-  std::vector<uint4> chunks;
-  std::vector<uint64_t> parts, toff(H);
-  std::vector<uint8_t> tlog(H);
-  std::vector<uint32_t> pages;
-  uint64_t part = 0;
+  launch_gather_u32(hb.verts_degs.p, H, lv.deg, hb.verts_degs.p + H, s);
+  if (hb.hverts_degs.n < 2 * H) LVG_CUDA(cudaStreamSynchronize(s));  // (before a pinned block in use is freed)
+  hb.hverts_degs.ensure(2 * H);
+  LVG_CUDA(cudaMemcpyAsync(hb.hverts_degs.p, hb.verts_degs.p, 2 * H * 4, cudaMemcpyDeviceToHost, s));
+  host_sync(g);  // (and the pinned block's last upload is done)
+  const uint32_t *verts = hb.hverts_degs.p, *degs = verts + H;
+  const uint32_t step = g->tuning.hub_chunk;
+  // sizes: chunks, spill pages (tables of at least twice the degree in whole
+  // pages), merge tasks (hash partitions of at most about 8192 distinct
+  // communities: a task's table has 16384 slots)
+  size_t nch = 0, npages = 0, nmerge = 0;
+  auto table_log = [&](uint32_t d) {
+    int lg = SPILL_PAGE_LOG;
+    while ((uint64_t(1) << lg) < 2ull * d) ++lg;
+    return lg;
+  };
+  for (size_t h = 0; h < H; ++h) {
+    nch += (degs[h] + step - 1) / step;
+    npages += size_t(1) << (table_log(degs[h]) - SPILL_PAGE_LOG);
+    nmerge += (degs[h] + 8191) / 8192;
+  }
+  size_t bytes = 0;
+  auto place = [&](size_t n, size_t elem) {
+    const size_t at = bytes;
+    bytes += (n * elem + 15) / 16 * 16;
+    return at;
+  };
+  const size_t a_chunk = place(nch, 16), a_part = place(nch, 8), a_toff = place(H, 8), a_seg = place(H, 8),
+               a_merge = place(nmerge, 8), a_first = place(H + 1, 4), a_parts = place(H, 4), a_page = place(npages, 4),
+               a_tlog = place(H, 1);
+  hb.hpack.ensure(bytes);
+  hb.pack.ensure(bytes);
+  uint8_t *hp = hb.hpack.p;
+  auto *chunk = reinterpret_cast<uint4 *>(hp + a_chunk);
+  auto *chunk_part = reinterpret_cast<uint64_t *>(hp + a_part);
+  auto *toff = reinterpret_cast<uint64_t *>(hp + a_toff);
+  auto *seg_off = reinterpret_cast<uint64_t *>(hp + a_seg);
+  auto *merge = reinterpret_cast<uint2 *>(hp + a_merge);
+  auto *first = reinterpret_cast<uint32_t *>(hp + a_first);
+  auto *parts = reinterpret_cast<uint32_t *>(hp + a_parts);
+  auto *page = reinterpret_cast<uint32_t *>(hp + a_page);
+  uint8_t *tlog = hp + a_tlog;
+  size_t c = 0, pg = 0, mt = 0;
+  uint64_t part = 0, seg = 0;
   for (int k = 0; k < K; ++k) {
-    P.chunk_begin[k] = chunks.size();
+    P.chunk_begin[k] = c;
+    P.merge_begin[k] = mt;
+    P.page_begin[k] = pg;
     uint64_t slots = 0;  // the class's spill tables, back to back
-    P.page_begin[k] = pages.size();
     for (size_t h = P.hub_begin[k]; h < P.hub_begin[k + 1]; ++h) {
-      int lg = SPILL_PAGE_LOG;
-      while ((uint64_t(1) << lg) < 2ull * degs[h]) ++lg;
+      const int lg = table_log(degs[h]);
       tlog[h] = uint8_t(lg);
       toff[h] = slots;
       slots += uint64_t(1) << lg;
-      pages.insert(pages.end(), size_t(1) << (lg - SPILL_PAGE_LOG), uint32_t(h));
-      first[h] = uint32_t(chunks.size());
-      const uint32_t step = g->tuning.hub_chunk;
+      for (size_t i = 0; i < size_t(1) << (lg - SPILL_PAGE_LOG); ++i) page[pg++] = uint32_t(h);
+      first[h] = uint32_t(c);
       for (uint32_t lo = 0; lo < degs[h]; lo += step) {
-        chunks.push_back(make_uint4(uint32_t(h), lo, std::min<uint32_t>(degs[h], lo + step), verts[h]));
-        parts.push_back(part + lo);
+        chunk_part[c] = part + lo;
+        chunk[c++] = make_uint4(uint32_t(h), lo, std::min<uint32_t>(degs[h], lo + step), verts[h]);
       }
       part += degs[h];
+      const uint32_t R = (degs[h] + 8191) / 8192;
+      parts[h] = R;
+      seg_off[h] = seg;
+      seg += uint64_t(c - first[h]) * (R + 1);
+      for (uint32_t r = 0; r < R; ++r) merge[mt++] = make_uint2(uint32_t(h), r);
     }
     P.spill_slots = std::max<size_t>(P.spill_slots, slots);
     P.class_slots[k] = slots;
   }
-  P.page_begin[K] = pages.size();
-  P.chunk_begin[K] = chunks.size();
-  first[H] = uint32_t(chunks.size());
-  P.chunks = chunks.size();
+  P.page_begin[K] = pg;
+  P.chunk_begin[K] = c;
+  P.merge_begin[K] = mt;
+  P.seg_total = seg;
+  first[H] = uint32_t(c);
+  P.chunks = c;
   P.part = part;
-  hb.hub_first.ensure(H + 1);
-  hb.chunk.ensure(chunks.size());
-  hb.chunk_part.ensure(chunks.size());
-  hb.hub_toff.ensure(H);
-  hb.hub_tlog.ensure(H);
-  LVG_CUDA(cudaMemcpyAsync(hb.hub_toff.p, toff.data(), H * 8, cudaMemcpyHostToDevice, s));
-  LVG_CUDA(cudaMemcpyAsync(hb.hub_tlog.p, tlog.data(), H, cudaMemcpyHostToDevice, s));
-  hb.page_hub.ensure(pages.size());
-  LVG_CUDA(cudaMemcpyAsync(hb.page_hub.p, pages.data(), pages.size() * 4, cudaMemcpyHostToDevice, s));
-  LVG_CUDA(cudaMemcpyAsync(hb.hub_first.p, first.data(), (H + 1) * 4, cudaMemcpyHostToDevice, s));
-  LVG_CUDA(cudaMemcpyAsync(hb.chunk.p, chunks.data(), chunks.size() * sizeof(uint4), cudaMemcpyHostToDevice, s));
-  LVG_CUDA(cudaMemcpyAsync(hb.chunk_part.p, parts.data(), parts.size() * 8, cudaMemcpyHostToDevice, s));
-  host_sync(g);
-  P.hub_vertex = hb.hub_vertex.p;
-  P.hub_first = hb.hub_first.p;
-  P.chunk = hb.chunk.p;
-  P.chunk_part = hb.chunk_part.p;
-  P.hub_toff = hb.hub_toff.p;
-  P.hub_tlog = hb.hub_tlog.p;
-  P.page_hub = hb.page_hub.p;
+  LVG_CUDA(cudaMemcpyAsync(hb.pack.p, hp, bytes, cudaMemcpyHostToDevice, s));
+  const uint8_t *dp = hb.pack.p;
+  P.hub_vertex = hb.verts_degs.p;
+  P.hub_first = reinterpret_cast<const uint32_t *>(dp + a_first);
+  P.chunk = reinterpret_cast<const uint4 *>(dp + a_chunk);
+  P.chunk_part = reinterpret_cast<const uint64_t *>(dp + a_part);
+  P.hub_toff = reinterpret_cast<const uint64_t *>(dp + a_toff);
+  P.hub_tlog = dp + a_tlog;
+  P.page_hub = reinterpret_cast<const uint32_t *>(dp + a_page);
+  P.hub_parts = reinterpret_cast<const uint32_t *>(dp + a_parts);
+  P.seg_off = reinterpret_cast<const uint64_t *>(dp + a_seg);
+  P.merge = reinterpret_cast<const uint2 *>(dp + a_merge);
 }
 
 // Colour classes of a run: the options' count, else 16 (deterministic), else
@@ -657,6 +691,86 @@ void capture_iteration(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot
   g->iter_key = key;
 }
 
+// The chunked hubs' partial results (both the launch-by-launch path and the
+// phase kernel).
+void ensure_hub_buffers(lvg_graph *g, const Level &lv) {
+  Workspace &W = *g->ws;
+  W.chunk_cnt.ensure(lv.hub.chunks);
+  W.part_key.ensure(lv.hub.part);
+  W.part_val.ensure(lv.hub.part);
+  if (W.hub_over.n < lv.hub.hubs) {  // the merge resets each mark it reads
+    W.hub_over.ensure(lv.hub.hubs);
+    LVG_CUDA(cudaMemsetAsync(W.hub_over.p, 0, W.hub_over.n, g->stream));
+    W.hub_best.ensure(lv.hub.hubs);
+    LVG_CUDA(cudaMemsetAsync(W.hub_best.p, 0, W.hub_best.n * 8, g->stream));
+  }
+}
+
+// Enqueue a level's whole local-moving phase as one launch of the phase
+// kernel (lvg_phase.cu) and the read-back of its counters. False, having
+// enqueued nothing, when the level takes the launch-by-launch path.
+bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const tot_t *tot,
+                          const uint8_t *fa, double M, float kr, int L, double E, bool sync, const UnionCall *uc,
+                          bool listed, bool from_prior) {
+  Workspace &W = *g->ws;
+  cudaStream_t s = g->stream;
+  if (g->profiling || !g->tuning.level_graphs || L <= 0) return false;
+  // resident hub tables are kept by the launch-by-launch kernels; a frontier
+  // run of one class starts from lists of its few marked vertices there
+  if (W.ht_now.key || listed) return false;
+  const HubPlan &P = lv.hub;
+  // Asynchronous runs from a prior on a level with hubs keep the launches: in
+  // which order a class's degree bins see each other's moves differs there,
+  // and with it the outcome by more (1.4 % of the memberships of a scale-22
+  // R-MAT graph) than two runs of one order differ (0.2-0.7 %).
+  if (P.hubs && from_prior && !sync) return false;
+  if (P.hubs && (g->tuning.hub_chunk > PHASE_HUB_CHUNK || lv.bin_maxdeg[NUM_BINS - 1] > PHASE_MAX_DEGREE)) return false;
+  const uint32_t grid = phase_grid(lv);
+  if (!grid) return false;
+  PhaseArgs a{};
+  a.off = lv.off; a.deg = lv.deg; a.key = lv.key; a.w = lv.w; a.bins = lv.bins;
+  a.vcom = com; a.ctot = ctot; a.vaff = W.vaff.p; a.fa = fa; a.vtot = tot;
+  W.phase_ctl.ensure(1);
+  a.ctr = g->ctr.p; a.ctl = W.phase_ctl.p;
+  a.kr = kr; a.colors = lv.colors; a.L = L; a.M = M; a.E = E;
+  a.cap = phase_list_cap(lv, grid);
+  if (!phase_lists_fit(a.cap)) {
+    W.phase_mv.ensure(size_t(grid) * a.cap);
+    W.phase_list.ensure(size_t(grid) * a.cap);
+    a.gmv = W.phase_mv.p;
+    a.glist = W.phase_list.p;
+  }
+  if (P.hubs) {
+    ensure_hub_buffers(g, lv);
+    W.hub_segs.ensure(P.seg_total);
+    if (W.hub_done.n < P.hubs) {  // (left zero by the merges)
+      W.hub_done.ensure(P.hubs);
+      LVG_CUDA(cudaMemsetAsync(W.hub_done.p, 0, W.hub_done.n * 4, s));
+    }
+    W.hub_move.ensure(P.hubs);
+    a.hub_vertex = P.hub_vertex; a.hub_first = P.hub_first; a.hub_parts = P.hub_parts; a.seg_off = P.seg_off;
+    a.chunk = P.chunk; a.chunk_part = P.chunk_part; a.merge = P.merge;
+    a.chunk_cnt = W.chunk_cnt.p; a.part_key = W.part_key.p; a.part_val = reinterpret_cast<uint32_t *>(W.part_val.p);
+    a.segs = W.hub_segs.p; a.hub_kd = W.hub_kd.p; a.hub_best = W.hub_best.p;
+    a.hub_done = W.hub_done.p; a.hub_move = W.hub_move.p;
+    for (int k = 0; k <= lv.colors; ++k) {
+      a.chunk_begin[k] = uint32_t(P.chunk_begin[k]);
+      a.merge_begin[k] = uint32_t(P.merge_begin[k]);
+    }
+  }
+  if (uc) {
+    a.gid = lv.gid; a.gkr = uc->kr; a.gzero = lv.gbase; a.gfix = uc->fix; a.gact = uc->gact;
+    a.graphs = uint32_t(uc->n); a.gctl = uc->ctl; a.gM = uc->M; a.itcap = uc->L;
+  }
+  for (int i = 0; i <= lv.colors * NUM_BINS; ++i) a.start[i] = uint32_t(lv.bin_start[i]);
+  launch_fill_bytes(W.phase_ctl.p, 0, sizeof(PhaseCtl), s);
+  launch_phase(sync, lv.unit, lv.whole && g->total_weight < 2147483648.0, grid, a, s);
+  ++g->stats.move_launches;
+  ++g->stats.level_graphs;
+  LVG_CUDA(cudaMemcpyAsync(g->hctr.p, g->ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));
+  return true;
+}
+
 // louvainMoveOmpW (inc/louvain.hxx:588-609). Returns the iteration count, 0
 // if the first iteration found nothing to gain. Each iteration sweeps the
 // colour classes in order (enqueue_iteration). For the uploaded level the
@@ -674,7 +788,7 @@ struct PhaseEnd {
 int move_phase(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const tot_t *tot, const uint8_t *fa,
                double M, float kr, int L, double E, bool sync, int fused, const UnionCall *uc = nullptr,
                bool iso_clear = false, PhaseEnd *end = nullptr, bool capture = true,
-               const std::function<void()> *tail = nullptr, bool *tail_done = nullptr) {
+               const std::function<void()> *tail = nullptr, bool *tail_done = nullptr, bool from_prior = false) {
   if (tail_done) *tail_done = false;
   Workspace &W = *g->ws;
   cudaStream_t s = g->stream;
@@ -690,6 +804,19 @@ int move_phase(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const 
       iso.n[k] = lv.bucket_size(k, 0);
     }
     launch_clear_isolated_multi(iso, W.vaff.p, fa, s);
+  }
+  if (enqueue_phase_kernel(g, lv, com, ctot, tot, fa, M, kr, L, E, sync, uc, iso_clear && K == 1,
+                           from_prior)) {
+    if (tail) {
+      (*tail)();
+      if (tail_done) *tail_done = true;
+    }
+    host_sync(g);
+    if (g->hctr.p->err) read_counters(g);  // raises the device error
+    const int l = int(g->hctr.p->dev_iters);
+    const double el = uc ? 0.0 : g->hctr.p->dev_el;  // graph unions: each graph's el is in its GraphCtl
+    if (end) { end->l = l; end->el = el; }
+    return (l > 1 || el != 0) ? l : 0;
   }
   // Global fallback regions of the large-degree bins (9-11): each launch's
   // blocks get 2^glog2[b] slots, enough for the bin's largest degree.
@@ -708,17 +835,7 @@ int move_phase(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const 
     W.gkeys.ensure(need);
     W.gvals.ensure(need);
   }
-  if (lv.hub.hubs) {
-    W.chunk_cnt.ensure(lv.hub.chunks);
-    W.part_key.ensure(lv.hub.part);
-    W.part_val.ensure(lv.hub.part);
-    if (W.hub_over.n < lv.hub.hubs) {  // the merge resets each mark it reads
-      W.hub_over.ensure(lv.hub.hubs);
-      LVG_CUDA(cudaMemsetAsync(W.hub_over.p, 0, W.hub_over.n, s));
-      W.hub_best.ensure(lv.hub.hubs);
-      LVG_CUDA(cudaMemsetAsync(W.hub_best.p, 0, W.hub_best.n * 8, s));
-    }
-  }
+  if (lv.hub.hubs) ensure_hub_buffers(g, lv);
   const bool base = lv.off == g->base.off;
   IterKey key{};
   if (base) {
@@ -837,6 +954,7 @@ Level aggregate(lvg_graph *g, const Level &lv, const uint32_t *com, size_t CN, i
   nl.span = nl.order = CN;
   nl.off = nb.off.p; nl.deg = nb.deg.p; nl.key = nb.key.p; nl.w = nb.w.p; nl.ex = nullptr;
   nl.gid = ngid; nl.gbase = ngbase;
+  nl.whole = lv.whole;
   // Community -> members CSR and row capacities.
   LVG_CUDA(cudaMemsetAsync(W.csize.p, 0, (CN + 1) * sizeof(uint32_t), s));
   LVG_CUDA(cudaMemsetAsync(W.ccur.p, 0, (CN + 1) * sizeof(uint32_t), s));
@@ -1132,7 +1250,8 @@ void run(lvg_graph *g, int method, const DBatch &b, StateRef prior, StateRef out
         SpillScope spill(g, lv, method == LVG_METHOD_STATIC);
         HubTabScope hts(g, first && tabs ? tout : nullptr);  // kept up to date by the first pass's moves
         m = move_phase(g, lv, com, ctot, tot, first ? fa : nullptr, M, kr, L, E, sync, fused, nullptr, ends,
-                       nullptr, true, first && r == rep - 1 ? &tail : nullptr, &tail_done);
+                       nullptr, true, first && r == rep - 1 ? &tail : nullptr, &tail_done,
+                       method != LVG_METHOD_STATIC);
       }
       tl_ev.push_back({a0, tail_done ? tail_ev : g->events.record(s)});
       l += std::max(m, 1);
@@ -1643,6 +1762,7 @@ void init_graph(lvg_graph *g, size_t span, size_t order, size_t X, const uint64_
   read_counters(g);
   g->total_weight = g->hctr.p->fp64[0];
   b.unit = X > 0 && g->hctr.p->nonunit == 0;
+  b.whole = X > 0 && g->hctr.p->nonwhole == 0;
 }
 
 // ---------------------------------------------------------------- batch apply
@@ -1792,10 +1912,11 @@ void apply_plan(lvg_graph *g, const PlanCounts &pc) {
   launch_finish_rows(g->off.p, g->deg.p, g->cap.p, g->key.p, g->w.p, rows, nrows, g->u_plan.p, g->u_grow.p,
                      g->u_gpos.p, pool, s);
   g->pool_cursor += GROW;
-  if (b.unit && ni) {  // an insertion of another weight ends the unit-weight fast path
-    LVG_CUDA(cudaMemsetAsync(&g->ctr.p->nonunit, 0, sizeof(unsigned long long), s));
+  static_assert(offsetof(Counters, nonwhole) == offsetof(Counters, nonunit) + sizeof(unsigned long long), "");
+  if (b.whole && ni) {  // an insertion of another weight ends the unit-weight (whole-weight) fast path
+    LVG_CUDA(cudaMemsetAsync(&g->ctr.p->nonunit, 0, 2 * sizeof(unsigned long long), s));
     launch_count_nonunit(iw, ni, g->ctr.p, s);
-    LVG_CUDA(cudaMemcpyAsync(&g->hctr.p->nonunit, &g->ctr.p->nonunit, sizeof(unsigned long long),
+    LVG_CUDA(cudaMemcpyAsync(&g->hctr.p->nonunit, &g->ctr.p->nonunit, 2 * sizeof(unsigned long long),
                              cudaMemcpyDeviceToHost, s));
   }
   if (ex) {
@@ -1803,7 +1924,10 @@ void apply_plan(lvg_graph *g, const PlanCounts &pc) {
     LVG_CUDA(cudaMemcpyAsync(g->hupd.p + UPD_ORDER, g->upd.p + UPD_ORDER, 8, cudaMemcpyDeviceToHost, s));
   }
   LVG_CUDA(cudaStreamSynchronize(s));
-  if (b.unit && ni && g->hctr.p->nonunit) b.unit = false;
+  if (b.whole && ni) {
+    b.unit = b.unit && !g->hctr.p->nonunit;
+    b.whole = !g->hctr.p->nonwhole;
+  }
   b.edges = size_t((long long)b.edges + edge_delta);
   if (ex) b.order = g->hupd.p[UPD_ORDER];
   g->total_weight += wdelta;

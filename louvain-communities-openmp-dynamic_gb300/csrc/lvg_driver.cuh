@@ -22,11 +22,10 @@ namespace lvg {
 extern thread_local std::string g_err;  // the calling thread's last error (lvg_last_error)
 
 struct HubPlanBuffers {
-  DBuf<uint32_t> hub_vertex, hub_first, degs;
-  DBuf<uint4> chunk;
-  DBuf<uint64_t> chunk_part, hub_toff;
-  DBuf<uint8_t> hub_tlog;
-  DBuf<uint32_t> page_hub;
+  DBuf<uint32_t> verts_degs;  // [2 hubs] vertex ids, degrees
+  DBuf<uint8_t> pack;         // every other array of the plan
+  HBuf<uint32_t> hverts_degs;
+  HBuf<uint8_t> hpack;
 };
 
 struct LevelBuffers {
@@ -60,6 +59,11 @@ struct Workspace {
   DBuf<float> spill_vals;
   bool spill_now = false;  // the iteration being enqueued spills overflowing hubs
   bool first_sweep = false;  // static Louvain's first iteration (every neighbour a singleton)
+  // the phase kernel's shared words, and its blocks' lists when they are too
+  // long for shared memory
+  DBuf<PhaseCtl> phase_ctl;
+  DBuf<uint2> phase_mv;
+  DBuf<uint32_t> phase_list, hub_segs, hub_done, hub_move;
   // resident hub tables: build scratch, and the tables the first pass of the
   // run being enqueued keeps up to date (key == nullptr: none)
   DBuf<uint64_t> ht_soff;

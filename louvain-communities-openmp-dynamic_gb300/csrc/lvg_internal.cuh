@@ -103,6 +103,16 @@ struct HubPlan {
   size_t spill_slots = 0;
   size_t class_slots[MAX_COLORS] = {};
   size_t page_begin[MAX_COLORS + 1] = {};
+  // The phase kernel's merges (lvg_phase.cu): hub h's communities fall into
+  // hub_parts[h] hash partitions, one merge task (hub, partition) each (class
+  // k's tasks: merge[merge_begin[k] .. merge_begin[k+1])); chunk c of hub h
+  // keeps its partitions' bounds at seg_off[h] + (c - hub_first[h]) *
+  // (hub_parts[h] + 1), seg_total words in all.
+  const uint32_t *hub_parts = nullptr;
+  const uint64_t *seg_off = nullptr;
+  const uint2 *merge = nullptr;
+  size_t merge_begin[MAX_COLORS + 1] = {};
+  size_t seg_total = 0;
 };
 constexpr int SPILL_PAGE_LOG = 15;
 
@@ -127,6 +137,10 @@ struct Level {
   // integers in FP32 below 2^24 whatever the order, so the results are those
   // of the weighted path bit for bit.
   bool unit = false;
+  // Every edge weight is a whole number and they sum to less than 2^31 (a
+  // level aggregated from unit weights, or an uploaded level of counts): the
+  // phase kernel then adds them as integers, exactly.
+  bool whole = false;
   // Vertices grouped by (colour class, degree bin), ascending id within a
   // group: group (k, b) is bins[bin_start[k*NUM_BINS+b] .. bin_start[k*NUM_BINS+b+1]).
   uint32_t *bins = nullptr;
@@ -160,6 +174,7 @@ struct Counters {
   unsigned int ds_long;                       // delta-screening sources with more than 32 insertions
   uint32_t ds_chunks;                         // delta-screening neighbour chunks of the high-degree vertices
   unsigned long long nonunit;                 // edge weights other than 1 (count_nonunit)
+  unsigned long long nonwhole;                // and those that are no whole number in [0, 2^24]
   unsigned int dev_iters;                     // iterations run by the device-side loop (iter_end_kernel)
   double dev_el;                              // its last iteration's el
   // Worklists of the first local-moving iteration filled by df_start_kernel
@@ -298,6 +313,69 @@ struct MoveArgs {
   HubTabView ht;
 };
 
+// Shared words of a phase kernel's blocks (lvg_phase.cu), zeroed before the
+// launch. Each triple takes turns: over grid barriers (bar) or iterations.
+struct PhaseCtl {
+  unsigned long long bar[3];      // arrivals (low word) and moves (high word) of a barrier
+  unsigned long long fix[3];      // an iteration's gain sum
+  unsigned long long gactive[3];  // graph unions: graphs still moving
+  unsigned long long aborted;     // a block gave a wait up
+};
+
+// Arguments of the phase kernel: a level's whole local-moving phase.
+struct PhaseArgs {
+  const uint64_t *off;
+  const uint32_t *deg;
+  const uint32_t *key;
+  const float *w;
+  const uint32_t *bins;  // Level::bins
+  uint32_t *vcom;
+  tot_t *ctot;
+  uint8_t *vaff;
+  const uint8_t *fa;
+  const tot_t *vtot;
+  Counters *ctr;
+  PhaseCtl *ctl;
+  float kr;
+  int colors, L;
+  double M, E;
+  uint32_t cap;       // list slots of a block
+  uint2 *gmv;         // [grid * cap] moves and lists of blocks that do not fit
+  uint32_t *glist;    // shared memory
+  // hubs (HubPlan), and their partial results
+  const uint32_t *hub_vertex, *hub_first, *hub_parts;
+  const uint64_t *seg_off;
+  const uint4 *chunk;
+  const uint64_t *chunk_part;
+  const uint2 *merge;
+  uint32_t *chunk_cnt, *part_key, *part_val, *segs;
+  float *hub_kd;                // [span]
+  unsigned long long *hub_best; // [hubs] zero between uses, as hub_done
+  uint32_t *hub_done, *hub_move;
+  // graph unions (nullptr for one graph), as MoveArgs
+  const uint32_t *gid;
+  const float *gkr;
+  const uint32_t *gzero;
+  unsigned long long *gfix;
+  uint8_t *gact;
+  uint32_t graphs;
+  GraphCtl *gctl;
+  const double *gM;
+  int itcap;          // iterations of a graph of the union
+  uint32_t start[MAX_BUCKETS + 1];  // Level::bin_start
+  uint32_t chunk_begin[MAX_COLORS + 1], merge_begin[MAX_COLORS + 1];  // hub chunks and merge tasks of a class
+};
+// Hub chunks (lvg_tuning::hub_chunk) up to this many edges fit the phase
+// kernel's table and leave room for the partitions' counters.
+constexpr uint32_t PHASE_HUB_CHUNK = 4096;
+constexpr uint64_t PHASE_MAX_DEGREE = 8192ull * 16384ull;  // partitions the counters hold
+// Blocks and list slots per block a level's phase kernel takes (0 blocks: the
+// device cannot launch cooperatively).
+uint32_t phase_grid(const Level &lv);
+uint32_t phase_list_cap(const Level &lv, uint32_t grid);
+void launch_phase(bool sync, bool unit, bool whole, uint32_t grid, const PhaseArgs &a, cudaStream_t s);
+bool phase_lists_fit(uint32_t cap);  // the lists stay in shared memory
+
 // Arguments of the aggregation kernels (inc/louvain.hxx:897-912, 987-992).
 struct AggArgs {
   const uint64_t *off;   // input level
@@ -371,7 +449,8 @@ void launch_iter_begin(unsigned long long *el_fix, uint32_t *wl_count, int n, cu
 void launch_fill_f32(float *p, size_t n, float v, cudaStream_t s);
 void launch_init_static(const Level &g, uint32_t *ucom, tot_t *utot, tot_t *ctot, cudaStream_t s);
 void launch_total_weight(const float *w, size_t n, Counters *ctr, cudaStream_t s);  // -> ctr->fp64[0]
-// ctr->nonunit += the count of w[0..n) other than 1.0f.
+// ctr->nonunit += the count of w[0..n) other than 1.0f; ctr->nonwhole += those
+// that are not whole numbers in [0, 2^24].
 void launch_count_nonunit(const float *w, size_t n, Counters *ctr, cudaStream_t s);
 // louvainVertexWeightsOmpW / louvainCommunityWeightsOmpW in FP64 (the C-ABI utilities).
 void launch_vertex_weights_f64(const Level &g, double *vtot, cudaStream_t s);

@@ -68,12 +68,20 @@ __global__ void init_static_kernel(const uint64_t *off, const uint32_t *deg, con
   }
 }
 
-__global__ void count_nonunit_kernel(const float *w, size_t m, unsigned long long *dst) {
-  unsigned long long c = 0;
-  GRID_STRIDE(i, m) c += w[i] != 1.0f;
+__global__ void count_nonunit_kernel(const float *w, size_t m, unsigned long long *dst, unsigned long long *nonwhole) {
+  unsigned long long c = 0, x = 0;
+  GRID_STRIDE(i, m) {
+    const float f = w[i];
+    c += f != 1.0f;
+    x += !(f >= 0.f && f <= 16777216.f && f == rintf(f));
+  }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+  for (int o = 16; o > 0; o >>= 1) {
+    c += __shfl_xor_sync(0xffffffffu, c, o);
+    x += __shfl_xor_sync(0xffffffffu, x, o);
+  }
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(dst, c);
+  if ((threadIdx.x & 31) == 0 && x) atomicAdd(nonwhole, x);
 }
 
 __global__ void total_weight_kernel(const float *w, size_t m, double *dst) {
@@ -1045,7 +1053,7 @@ void launch_community_weights_f64(const uint32_t *q, const double *vtot, size_t 
 
 void launch_count_nonunit(const float *w, size_t n, Counters *ctr, cudaStream_t s) {
   if (!n) return;
-  count_nonunit_kernel<<<grid_for(n, 256), 256, 0, s>>>(w, n, &ctr->nonunit);
+  count_nonunit_kernel<<<grid_for(n, 256), 256, 0, s>>>(w, n, &ctr->nonunit, &ctr->nonwhole);
   LVG_CHECK_LAUNCH();
 }
 

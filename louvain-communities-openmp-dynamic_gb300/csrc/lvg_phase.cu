@@ -1,0 +1,995 @@
+// lvg_phase.cu — a level's whole local-moving phase in one kernel
+// (louvainMoveOmpW, inc/louvain.hxx:588-609: every iteration, every colour
+// class, the stop test).
+//
+// What bounds a level of up to a few million edges is not its work but the
+// chain of steps: 16 colour classes an iteration, each of them a compaction,
+// a fork onto five streams, a kernel per degree bin, a join and (deterministic
+// mode) two more kernels, at 3-8 us a launch even inside a CUDA graph. Here
+// one cooperative launch of at most a block per SM stays on the GPU for the
+// phase; a class is two grid barriers (one in asynchronous mode), and every
+// block serves all degree bins of its share of the class.
+//
+// A class's vertices (Level::bins, grouped by degree bin) are dealt to the
+// blocks in small chunks, heaviest bins first. Per class a block
+//   1. lists the active ones among its vertices per bin (the flags as they
+//      are when the class starts);
+//   2. decides them: hubs (degree above 8192) chunk by chunk on many blocks,
+//      merged behind a further barrier; degree <= 32 by a tile of 4/8/16/32
+//      lanes that groups equal communities with warp matches and needs no
+//      table; degree 33-128 by a warp, 129-512 by four warps, 513-2048 by
+//      eight, above by the whole block, each with an open-addressing table of
+//      twice the degree in shared memory;
+//   3. deterministic mode: waits until every block has decided, then commits
+//      its own decisions (community, totals) and marks the movers' neighbours.
+//      Asynchronous mode commits at once.
+// Where every weight is 1, or a whole number (the aggregated levels of a
+// unit-weight graph), the tables add with integer shared-memory atomics
+// (native) instead of FP32 ones (a compare-and-swap loop); the sums are exact,
+// so the gains are those of exact FP32 sums.
+//
+// Measured on a GB300, deterministic static runs, launches -> this kernel: 2K
+// vertices 4.1 -> 1.8 ms, 131K-vertex planted partition 13 -> 4.3 ms, R-MAT
+// scale 20 20.4 -> 13.0 ms, scale 23 126 -> 76 ms (its two large levels' moving
+// 44 + 37 -> 21 + 20 ms). A class of a small level takes about 9 us: 1 to list,
+// 3-4 to decide, 1 to commit, 2 a barrier; of a large one, what its gathers
+// take (ncu, scale 21: warps wait at the groups' barriers and on gathers, 19 %
+// of issue slots busy).
+// Tried and dropped: tables of 1.5x instead of 2x to 4x the degree on half
+// blocks (the longest probe of a warp decides: 21 -> 29 ms), one code copy for
+// all group sizes (20.7 -> 21.6 ms), the next vertex's offset and degree
+// fetched ahead (no gain).
+#include <algorithm>
+#include <type_traits>
+
+#include "lvg_internal.cuh"
+
+namespace lvg {
+namespace {
+
+constexpr int PB = 1024;                  // threads per block
+constexpr int PW = PB / 32;               // warps per block
+constexpr uint32_t LOG_BLOCK = 14;        // shared slots of a block's vertex (log2)
+constexpr uint32_t TABLE_WORDS = 2u << LOG_BLOCK;  // keys and values
+constexpr uint32_t LIST_CAP = 1920;       // listed vertices a block keeps in shared memory
+constexpr uint32_t MERGE_FULL = 8192;     // partial entries of a hub that one block merges at once
+// One wait of the grid barrier gives up after this many polls (seconds; a
+// class takes microseconds), flags ERR_BARRIER and ends the kernel.
+constexpr uint32_t BARRIER_POLLS = 1u << 24;
+
+// The level's weights: any FP32, all 1, or whole numbers whose total is below 2^31.
+enum Weights { FLOATS, UNIT, WHOLE };
+template <int MODE>
+using Sum = typename std::conditional<MODE == FLOATS, float, uint32_t>::type;
+__device__ __forceinline__ uint32_t bits(float x) { return __float_as_uint(x); }
+__device__ __forceinline__ uint32_t bits(uint32_t x) { return x; }
+template <int MODE>
+__device__ __forceinline__ Sum<MODE> of_bits(uint32_t x) {
+  if constexpr (MODE == FLOATS) return __uint_as_float(x);
+  else return x;
+}
+// Weight of edge i.
+template <int MODE>
+__device__ __forceinline__ Sum<MODE> weight(const PhaseArgs &a, uint64_t i) {
+  if constexpr (MODE == FLOATS) return __ldcs(a.w + i);
+  else if constexpr (MODE == WHOLE) return __float2uint_rn(__ldcs(a.w + i));
+  else return 1u;
+}
+
+struct Shared {
+  uint32_t off[MAX_BUCKETS];   // [class][bin]: the block's first list slot of the bin
+  uint32_t pos[MAX_BUCKETS];   // [class][bin]: the bin's first position dealt to the block
+  uint32_t tot[MAX_COLORS];    // the block's list slots of a class
+  uint32_t cnt[NUM_BINS];      // listed vertices per bin of the current class
+  uint32_t edges[NUM_BINS];    // scanned edges of the current iteration
+  unsigned long long sv[NUM_BINS], se[NUM_BINS];  // the phase's vertices and edges
+  unsigned long long moves;
+  uint32_t redk[PW], redg[PW], redc[PW];
+  uint32_t next;               // next warp-sized unit of work of the class
+  uint32_t nmv, nbig;          // moves of the class; those with long rows
+  uint32_t hubmv;              // hubs moved by the block's merges
+  uint32_t over, bad, stop;
+  uint32_t any;                // some block moved a vertex before the last barrier that counts moves
+  unsigned long long sum;      // the iteration's gain sum, or the union's graphs still moving
+};
+
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+
+// Barrier number n of the grid (the launch is cooperative, so all blocks are
+// resident). A barrier's word counts the arrivals below and `moves` above, so
+// the waiting poll also tells whether any block moved a vertex (S.any); three
+// words take turns, block 0 clearing the next one (whose last readers have all
+// arrived at the barrier before this one). `sum` (optional) is read behind the
+// barrier into S.sum. False when a wait was given up, here or in another
+// block: every thread of every block then returns.
+__device__ __forceinline__ bool grid_barrier(const PhaseArgs &a, Shared &S, uint32_t n, uint32_t moves,
+                                             const unsigned long long *sum) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    if (gridDim.x == 1) {
+      S.any = moves;
+    } else {
+      if (blockIdx.x == 0) a.ctl->bar[(n + 1) % 3] = 0;
+      __threadfence();
+      unsigned long long *word = &a.ctl->bar[n % 3];
+      atomicAdd(word, 1ull + (static_cast<unsigned long long>(moves) << 32));
+      unsigned long long v;
+      uint32_t polls = 0;
+      while (uint32_t(v = ld_acquire(word)) < gridDim.x) {
+        ++polls;
+        if (polls >= BARRIER_POLLS || ((polls & 255u) == 0 && ld_acquire(&a.ctl->aborted))) {
+          atomicExch(&a.ctl->aborted, 1ull);
+          atomicOr(&a.ctr->err, ERR_BARRIER);
+          S.stop = 1;
+          break;
+        }
+      }
+      __threadfence();
+      S.any = uint32_t(v >> 32);
+    }
+    if (sum) S.sum = *reinterpret_cast<const volatile unsigned long long *>(sum);
+  }
+  __syncthreads();
+  return !S.stop;
+}
+
+// A barrier over the n threads (whole warps) of group `id`.
+__device__ __forceinline__ void group_sync(uint32_t id, uint32_t n) {
+  if (n == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+
+// The lanes of a warp holding the same key (grp) sum their weights in lane
+// order; every one of them gets the sum.
+template <class V>
+__device__ __forceinline__ V match_sum(unsigned grp, bool some, V w, int lane) {
+  const unsigned most = __reduce_max_sync(0xffffffffu, some ? unsigned(__popc(grp)) : 0u);
+  V sum = 0;
+  unsigned rem = some ? grp : 0u;
+  for (unsigned it = 0; it < most; ++it) {
+    const int src = rem ? __ffs(rem) - 1 : lane;
+    const V x = __shfl_sync(0xffffffffu, w, src);
+    if (rem) sum += x;
+    rem &= rem - 1u;
+  }
+  return sum;
+}
+
+template <class V>
+__device__ __forceinline__ V warp_sum(V x) {
+  if constexpr (std::is_same<V, uint32_t>::value) {
+    return __reduce_add_sync(0xffffffffu, x);
+  } else {
+#pragma unroll
+    for (int sh = 16; sh > 0; sh >>= 1) x += __shfl_xor_sync(0xffffffffu, x, sh);
+    return x;
+  }
+}
+
+// Add w to community c's slot of a table of 2^lg slots (linear probing).
+// False when every slot holds another key. Not the aggregation tables' hash
+// (hash_hi): an aggregated row is stored in the order of that one, so a chunk
+// of a hub's row would crowd into one stretch of slots (40 us of probing a
+// chunk, against 3).
+template <class V>
+__device__ __forceinline__ bool add(uint32_t *keys, uint32_t *vals, uint32_t lg, uint32_t c, V w) {
+  const uint32_t mask = (1u << lg) - 1u;
+  uint32_t s = (c * 0x85EBCA6Bu) >> (32u - lg);
+  for (uint32_t p = 0; p <= mask; ++p) {
+    uint32_t k = keys[s];
+    if (k == EMPTY) {
+      k = atomicCAS(&keys[s], EMPTY, c);
+      if (k == EMPTY) k = c;
+    }
+    if (k == c) {
+      atomicAdd(reinterpret_cast<V *>(&vals[s]), w);
+      return true;
+    }
+    s = (s + 1u) & mask;
+  }
+  return false;
+}
+
+// add() of FP32 weights by the lanes of a converged warp (c == EMPTY: nothing
+// to add). An FP32 shared-memory atomic retries while other lanes use its
+// address, and the neighbours of a large vertex share few communities: up to
+// three communities that four lanes or more hold are summed over the warp
+// first. (Whole weights need none of this: the hardware adds integers.)
+__device__ __forceinline__ bool add_warp(uint32_t *keys, uint32_t *vals, uint32_t lg, uint32_t c, float w, int lane) {
+  bool fine = true;
+  unsigned todo = __ballot_sync(0xffffffffu, c != EMPTY);
+  for (int r = 0; r < 3 && __popc(todo) >= 8; ++r) {
+    const int src = __ffs(todo) - 1;
+    const uint32_t key = __shfl_sync(0xffffffffu, c, src);
+    const unsigned same = __ballot_sync(0xffffffffu, c == key);
+    todo &= ~same;
+    if (__popc(same) < 4) continue;
+    const float sum = warp_sum<float>(c == key ? w : 0.f);
+    if (lane == src) fine &= add<float>(keys, vals, lg, c, sum);
+    if (c == key) c = EMPTY;
+  }
+  if (c != EMPTY) fine &= add<float>(keys, vals, lg, c, w);
+  return fine;
+}
+
+// R/(2M), the community that is never a target, and the graph of vertex u.
+struct Of {
+  float kr;
+  uint32_t zero, g;
+  __device__ __forceinline__ Of(const PhaseArgs &a, uint32_t u) : kr(a.kr), zero(0), g(0) {
+    if (a.gid) {
+      g = a.gid[u];
+      kr = a.gkr[g];
+      zero = a.gzero[g];
+    }
+  }
+};
+
+// The hash partition (of R) of a hub's community. Every bit of the id takes
+// part (two multiply-and-shift rounds), so that no pattern of ids gathers in
+// one partition; unlike the tables' slots, which are the high bits of one
+// multiplication.
+__device__ __forceinline__ uint32_t hub_part(uint32_t c, uint32_t R) {
+  c = (c ^ (c >> 16)) * 0x7FEB352Du;
+  c = (c ^ (c >> 15)) * 0x846CA68Bu;
+  return __umulhi(c ^ (c >> 16), R);
+}
+
+// A vertex's best gain into its iteration's sum: the thread's for one graph
+// (flushed once an iteration), the graph's for a union.
+__device__ __forceinline__ void add_gain(const PhaseArgs &a, unsigned long long &fix, const Of &G, float bg) {
+  if (a.gfix) atomicAdd(&a.gfix[G.g], gain_to_fix(bg));
+  else fix += gain_to_fix(bg);
+}
+
+// Graph unions, once an iteration: graph i's own stop test (as
+// iter_control_kernel).
+__device__ __forceinline__ void phase_control(const PhaseArgs &a, uint32_t i, uint32_t slot) {
+  if (!a.gact[i]) return;
+  const double el = double(a.gfix[i]) / GAIN_FIX / a.gM[i];
+  a.gfix[i] = 0;
+  GraphCtl &c = a.gctl[i];
+  c.el = el;
+  c.it += 1;
+  if (el <= a.E || c.it >= uint32_t(a.itcap)) a.gact[i] = 0;
+  else atomicAdd(&a.ctl->gactive[slot], 1ull);
+}
+
+// Mark the neighbours row[0..m) of u (thread t of n), four in flight.
+__device__ __forceinline__ void mark_row(const PhaseArgs &a, uint32_t u, uint64_t o, uint32_t m, uint32_t t, uint32_t n) {
+  for (uint32_t j = t; j < m; j += 4 * n) {
+    uint32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = j + k * n < m ? __ldcs(a.key + o + j + k * n) : u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (v[k] != u) a.vaff[v[k]] = 1;
+  }
+}
+
+// One thread: vertex u of community d leaves for c.
+template <bool SYNC>
+__device__ __forceinline__ void commit(const PhaseArgs &a, Shared &S, uint2 *mv, uint32_t u, uint32_t d, uint32_t c,
+                                       double wu) {
+  const uint32_t i = atomicAdd(&S.nmv, 1u);
+  if constexpr (SYNC) {
+    mv[i] = make_uint2(u, c);
+  } else {
+    atomicAdd(&a.ctot[d], -wu);
+    atomicAdd(&a.ctot[c], wu);
+    a.vcom[u] = c;
+  }
+}
+
+// Two rounds of 32/T vertices of degree <= T (T = 4, 8, 16, 32), one per tile
+// of the warp: list[first ..), those at `n` and beyond idle; both rounds'
+// loads are in flight together (a vertex is a chain of five dependent
+// gathers). Each lane holds one neighbour; equal communities of a tile are
+// grouped by a warp match.
+constexpr int TILE_ROUNDS = 2;
+template <bool SYNC, int MODE>
+__device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uint2 *mv, const uint32_t *list,
+                                              uint32_t first, uint32_t n, uint32_t T, int bin,
+                                              unsigned long long &fix) {
+  constexpr int N = TILE_ROUNDS;
+  using V = Sum<MODE>;
+  const int lane = threadIdx.x & 31;
+  const uint32_t tl = lane & (T - 1);
+  const unsigned tmask = (T == 32 ? 0xffffffffu : ((1u << T) - 1u) << (lane & ~(T - 1)));
+  uint32_t u[N], dg[N], d[N], v[N], c[N];
+  double wu[N], td[N];
+  V w[N];
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    const uint32_t i = first + r * (32 / T) + lane / T;
+    u[r] = i < n ? list[i] : EMPTY;
+  }
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    dg[r] = 0;
+    d[r] = EMPTY;
+    wu[r] = 0.0;
+    v[r] = u[r];
+    w[r] = 0;
+    if (u[r] != EMPTY) {
+      const uint64_t o = a.off[u[r]];
+      dg[r] = a.deg[u[r]];
+      d[r] = a.vcom[u[r]];
+      wu[r] = a.vtot[u[r]];
+      if (tl < dg[r]) {
+        v[r] = __ldcs(a.key + o + tl);
+        w[r] = weight<MODE>(a, o + tl);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    c[r] = v[r] != u[r] ? a.vcom[v[r]] : EMPTY;
+    td[r] = u[r] != EMPTY ? a.ctot[d[r]] : 0.0;
+  }
+  V kc[N], kd[N];
+  double tc[N];
+  unsigned lead = 0;
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    kd[r] = 0;
+    if (c[r] == d[r]) {
+      kd[r] = w[r];
+      c[r] = EMPTY;
+    }
+    const unsigned grp = __match_any_sync(0xffffffffu, c[r]) & tmask;
+    const bool is = c[r] != EMPTY && (grp & ((1u << lane) - 1u)) == 0u;
+    lead |= unsigned(is) << r;
+    tc[r] = is ? a.ctot[c[r]] : 0.0;
+    if constexpr (MODE == UNIT) {
+      kc[r] = __popc(grp);
+      kd[r] = __popc(__ballot_sync(0xffffffffu, kd[r] != 0u) & tmask);
+    } else {
+      kc[r] = match_sum<V>(grp, c[r] != EMPTY, w[r], lane);
+      for (uint32_t sh = T >> 1; sh; sh >>= 1) kd[r] += __shfl_xor_sync(0xffffffffu, kd[r], sh);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < N; ++r) {
+    const Of G(a, u[r] != EMPTY ? u[r] : 0u);
+    float bg = 0.f;
+    uint32_t bc = EMPTY;
+    if ((lead >> r) & 1u) {
+      const float g = gain_of(float(kc[r]), float(kd[r]), wu[r], __double2float_rn(wu[r]), tc[r], td[r], G.kr);
+      if (g > 0.f) { bg = g; bc = c[r]; }
+    }
+    for (uint32_t sh = T >> 1; sh; sh >>= 1) {
+      const float og = __shfl_xor_sync(0xffffffffu, bg, sh);
+      const uint32_t oc = __shfl_xor_sync(0xffffffffu, bc, sh);
+      if (better(og, oc, bg, bc)) { bg = og; bc = oc; }
+    }
+    const bool moved = bc != EMPTY && bc != G.zero;
+    if (u[r] != EMPTY && tl == 0) {
+      if (bc != EMPTY) add_gain(a, fix, G, bg);
+      if (moved) commit<SYNC>(a, S, mv, u[r], d[r], bc, wu[r]);
+      atomicAdd(&S.edges[bin], dg[r]);
+    }
+    if constexpr (!SYNC) {
+      if (moved && v[r] != u[r]) a.vaff[v[r]] = 1;
+      if (u[r] != EMPTY && tl == 0) a.vaff[u[r]] = 0;
+    }
+  }
+}
+
+// Sum the weights of the neighbours row[0..m) of u per community into a table
+// of 2^lg slots by the n threads of a group (thread t); those in u's own
+// community d are summed in the return value (each thread its share).
+template <int MODE>
+__device__ __forceinline__ Sum<MODE> scan_row(const PhaseArgs &a, Shared &S, uint32_t u, uint64_t o, uint32_t m,
+                                              uint32_t d, uint32_t t, uint32_t n, uint32_t *keys, uint32_t *vals,
+                                              uint32_t lg) {
+  using V = Sum<MODE>;
+  const int lane = threadIdx.x & 31;
+  V kd = 0;
+  bool fine = true;
+  constexpr int U = 4;  // edges of a lane in flight
+  for (uint32_t base = t - lane; base < m; base += U * n) {
+    uint32_t v[U], c[U];
+    V w[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const uint32_t j = base + k * n + lane;
+      v[k] = j < m ? __ldcs(a.key + o + j) : u;
+      w[k] = j < m ? weight<MODE>(a, o + j) : V(0);
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) c[k] = v[k] != u ? a.vcom[v[k]] : EMPTY;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (c[k] == d) { kd += w[k]; c[k] = EMPTY; }
+      if constexpr (MODE == FLOATS) fine &= add_warp(keys, vals, lg, c[k], w[k], lane);
+      else if (c[k] != EMPTY) fine &= add<V>(keys, vals, lg, c[k], MODE == UNIT ? 1u : w[k]);
+    }
+  }
+  if (!fine) S.bad = 1;  // (a table has twice as many slots as neighbours)
+  return kd;
+}
+
+// The best move of u over the communities of a table (kd: the weight to its
+// own community), by the n threads of a group whose first warp is w0: the
+// largest gain (positive, so its bits order as the floats), then the lowest
+// id. Four slots of a thread in flight: their communities' totals are gathers.
+template <int MODE>
+__device__ __forceinline__ void best_of_table(const PhaseArgs &a, Shared &S, const uint32_t *keys, const uint32_t *vals,
+                                              uint32_t slots, uint32_t t, uint32_t n, uint32_t id, int w0, float kd,
+                                              double wu, double td, float kr, uint32_t &gb, uint32_t &bc) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const float wuf = __double2float_rn(wu);
+  float bg = 0.f;
+  bc = EMPTY;
+  constexpr int U = 4;
+  for (uint32_t s = t; s < slots; s += U * n) {
+    uint32_t c[U];
+    double tc[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) c[k] = s + k * n < slots ? keys[s + k * n] : EMPTY;
+#pragma unroll
+    for (int k = 0; k < U; ++k) tc[k] = c[k] != EMPTY ? a.ctot[c[k]] : 0.0;
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (c[k] == EMPTY) continue;
+      const float kc = float(of_bits<MODE>(vals[s + k * n]));
+      const float g = gain_of(kc, kd, wu, wuf, tc[k], td, kr);
+      if (g > 0.f && better(g, c[k], bg, bc)) { bg = g; bc = c[k]; }
+    }
+  }
+  gb = __reduce_max_sync(0xffffffffu, __float_as_uint(bg));
+  bc = __reduce_min_sync(0xffffffffu, __float_as_uint(bg) == gb ? bc : EMPTY);
+  if (n > 32) {
+    if (lane == 0) { S.redg[wid] = gb; S.redc[wid] = bc; }
+    group_sync(id, n);
+    gb = 0;
+    bc = EMPTY;
+    for (uint32_t k = 0; k < (n >> 5); ++k) {
+      const uint32_t og = S.redg[w0 + k], oc = S.redc[w0 + k];
+      if (og > gb || (og == gb && oc < bc)) { gb = og; bc = oc; }
+    }
+  } else {
+    __syncwarp();
+  }
+}
+
+// One vertex by the n threads (1, 4, 8 or 32 warps, thread t) of a group, with
+// a table of twice its degree (at most 2^lgmax slots).
+template <bool SYNC, int MODE>
+__device__ __forceinline__ void group_vertex(const PhaseArgs &a, Shared &S, uint2 *mv, uint32_t u, uint32_t t,
+                                             uint32_t n, uint32_t id, uint32_t *table, uint32_t lgmax, int bin,
+                                             unsigned long long &fix) {
+  using V = Sum<MODE>;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int w0 = wid - int(t >> 5);  // the group's first warp
+  const uint64_t o = a.off[u];
+  const uint32_t dg = a.deg[u];
+  const uint32_t d = a.vcom[u];
+  const double wu = a.vtot[u], td = a.ctot[d];
+  const Of G(a, u);
+  const uint32_t lg = min(lgmax, uint32_t(ceil_log2(2ull * dg)));
+  uint32_t *keys = table, *vals = table + (1u << lg);
+  for (uint32_t s = t; s < (1u << lg); s += n) { keys[s] = EMPTY; vals[s] = 0u; }
+  group_sync(id, n);
+  V kd = warp_sum<V>(scan_row<MODE>(a, S, u, o, dg, d, t, n, keys, vals, lg));
+  if (lane == 0) S.redk[wid] = bits(kd);
+  group_sync(id, n);  // the table and the sums are complete
+  kd = 0;
+  for (uint32_t k = 0; k < (n >> 5); ++k) kd += of_bits<MODE>(S.redk[w0 + k]);
+  uint32_t gb, bc;
+  best_of_table<MODE>(a, S, keys, vals, 1u << lg, t, n, id, w0, float(kd), wu, td, G.kr, gb, bc);
+  const bool moved = bc != EMPTY && bc != G.zero;
+  if (t == 0) {
+    if (bc != EMPTY) add_gain(a, fix, G, __uint_as_float(gb));
+    if (moved) commit<SYNC>(a, S, mv, u, d, bc, wu);
+    atomicAdd(&S.edges[bin], dg);
+  }
+  if constexpr (!SYNC) {
+    if (moved) mark_row(a, u, o, dg, t, n);
+    if (t == 0) a.vaff[u] = 0;
+  }
+}
+
+// ---- hubs (degree above 8192), in two steps with a grid barrier between.
+// Step 1, a block per chunk of a hub's edges: the chunk's communities are
+// counted in the block's table and written out as (community, weight) pairs,
+// grouped by the hub's `parts` hash partitions of the communities (segs: the
+// groups' bounds), so that step 2 splits a hub of many communities over
+// blocks. chunk_cnt is EMPTY for a hub that is not active.
+template <int MODE>
+__device__ __forceinline__ void hub_chunk(const PhaseArgs &a, Shared &S, uint32_t ci, uint32_t *table) {
+  using V = Sum<MODE>;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint4 ch = a.chunk[ci];
+  const uint32_t u = ch.w, h = ch.x;
+  if (threadIdx.x == 0) {
+    S.over = a.vaff[u] && (!a.fa || a.fa[u]) && (!a.gact || a.gact[a.gid[u]]);
+    S.next = 0;
+  }
+  __syncthreads();
+  if (!S.over) {  // (block-uniform)
+    __syncthreads();
+    if (threadIdx.x == 0) a.chunk_cnt[ci] = EMPTY;
+    return;
+  }
+  const uint32_t m = ch.z - ch.y, d = a.vcom[u];
+  const uint32_t lg = max(1u, uint32_t(ceil_log2(2ull * m))), slots = 1u << lg;
+  uint32_t *keys = table, *vals = table + slots, *pc = table + 2 * slots;
+  const uint32_t R = a.hub_parts[h];
+  for (uint32_t s = threadIdx.x; s < slots; s += PB) { keys[s] = EMPTY; vals[s] = 0u; }
+  for (uint32_t r = threadIdx.x; r < R; r += PB) pc[r] = 0;
+  __syncthreads();
+  const V kd = warp_sum<V>(scan_row<MODE>(a, S, u, a.off[u] + ch.y, m, d, threadIdx.x, PB, keys, vals, lg));
+  if (lane == 0) S.redk[wid] = bits(kd);
+  __syncthreads();
+  uint32_t *pk = a.part_key + a.chunk_part[ci];
+  uint32_t *pv = a.part_val + a.chunk_part[ci];
+  // (lanes of one partition take their places together: the counters are few
+  // and hot)
+  if (R > 1) {
+    for (uint32_t s = threadIdx.x; s - lane < slots; s += PB) {
+      const uint32_t c = s < slots ? keys[s] : EMPTY;
+      const uint32_t r = c != EMPTY ? hub_part(c, R) : EMPTY;
+      const unsigned grp = __match_any_sync(0xffffffffu, r);
+      if (r != EMPTY && (grp & ((1u << lane) - 1u)) == 0u) atomicAdd(&pc[r], uint32_t(__popc(grp)));
+    }
+    __syncthreads();
+    uint32_t *seg = a.segs + a.seg_off[h] + size_t(ci - a.hub_first[h]) * (R + 1);
+    if (wid == 0) {  // exclusive prefix of the partitions' counts
+      uint32_t carry = 0;
+      for (uint32_t r0 = 0; r0 < R; r0 += 32) {
+        const uint32_t r = r0 + lane, x = r < R ? pc[r] : 0u;
+        uint32_t inc = x;
+#pragma unroll
+        for (int sh = 1; sh < 32; sh <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, inc, sh);
+          if (lane >= sh) inc += y;
+        }
+        if (r < R) { pc[r] = carry + inc - x; seg[r] = carry + inc - x; }
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      if (lane == 0) { seg[R] = carry; S.next = carry; }
+    }
+    __syncthreads();
+  }
+  for (uint32_t s = threadIdx.x; s - lane < slots; s += PB) {
+    const uint32_t c = s < slots ? keys[s] : EMPTY;
+    const uint32_t r = c == EMPTY ? EMPTY : R > 1 ? hub_part(c, R) : 0u;
+    const unsigned grp = __match_any_sync(0xffffffffu, r);
+    const int leader = __ffs(grp) - 1;
+    uint32_t at = 0;
+    if (r != EMPTY && lane == leader) at = atomicAdd(R > 1 ? &pc[r] : &S.next, uint32_t(__popc(grp)));
+    at = __shfl_sync(0xffffffffu, at, leader) + __popc(grp & ((1u << lane) - 1u));
+    if (r != EMPTY) { pk[at] = c; pv[at] = vals[s]; }
+  }
+  if (threadIdx.x == 0) {
+    V k = 0;
+    for (int x = 0; x < PW; ++x) k += of_bits<MODE>(S.redk[x]);
+    if (k != V(0)) atomicAdd(reinterpret_cast<V *>(&a.hub_kd[u]), k);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    a.chunk_cnt[ci] = S.next;
+    S.next = 0;
+  }
+}
+
+// Step 2, a block per (hub, partition): the partition's pairs of all chunks
+// are merged in the block's table and its best move goes to hub_best; the
+// block that completes the hub takes its decision (hub_move: the community it
+// goes to, EMPTY if it stays). A hub whose pairs all fit one table is merged
+// by the block of partition 0 alone. A hub that was marked while its chunks
+// ran (asynchronous mode: some chunks skipped it) waits for the next
+// iteration.
+template <bool SYNC, int MODE>
+__device__ __forceinline__ void hub_merge(const PhaseArgs &a, Shared &S, uint2 task, uint32_t *table,
+                                          unsigned long long &fix) {
+  using V = Sum<MODE>;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const uint32_t h = task.x, r = task.y, R = a.hub_parts[h];
+  const uint32_t u = a.hub_vertex[h];
+  const uint32_t c0 = a.hub_first[h], nc = a.hub_first[h + 1] - c0;
+  if (threadIdx.x == 0) { S.next = 0; S.over = 0; }
+  __syncthreads();
+  {
+    uint32_t sum = 0;
+    bool stale = false;
+    for (uint32_t c = threadIdx.x; c < nc; c += PB) {
+      const uint32_t x = a.chunk_cnt[c0 + c];
+      stale |= x == EMPTY;
+      sum += x == EMPTY ? 0u : x;
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0 && sum) atomicAdd(&S.next, sum);
+    if (stale) S.over = 1;
+  }
+  __syncthreads();
+  const uint32_t P = S.next;
+  const bool stale = S.over != 0, single = R == 1 || P <= MERGE_FULL;
+  __syncthreads();
+  if (stale || (single && r > 0)) {  // (block-uniform)
+    if (stale && r == 0 && threadIdx.x == 0) {
+      a.hub_move[h] = EMPTY;
+      a.hub_kd[u] = 0.f;
+    }
+    if (threadIdx.x == 0) S.next = 0;
+    return;
+  }
+  const uint32_t lg = single ? max(1u, uint32_t(ceil_log2(2ull * P))) : LOG_BLOCK, slots = 1u << lg;
+  uint32_t *keys = table, *vals = table + slots;
+  for (uint32_t s = threadIdx.x; s < slots; s += PB) { keys[s] = EMPTY; vals[s] = 0u; }
+  const uint32_t d = a.vcom[u];
+  const double wu = a.vtot[u], td = a.ctot[d];
+  const V kd = of_bits<MODE>(__float_as_uint(a.hub_kd[u]));
+  const Of G(a, u);
+  __syncthreads();
+  bool fine = true;
+  // a warp per (chunk, piece of its pairs): 128 pairs at a time, `pieces`
+  // warps to a chunk (as many as its pairs are likely to need)
+  const uint32_t pieces = single ? min(32u, max(1u, P / (nc * 128u) + 1)) : min(32u, 32u / R + 1);
+  for (uint32_t x = wid; x < nc * pieces; x += PW) {
+    const uint32_t c = x / pieces, piece = x - c * pieces;
+    const uint64_t p = a.chunk_part[c0 + c];
+    uint32_t b = 0, e = 0;
+    if (single) {
+      e = a.chunk_cnt[c0 + c];
+    } else {
+      const uint32_t *seg = a.segs + a.seg_off[h] + size_t(c) * (R + 1);
+      b = seg[r];
+      e = seg[r + 1];
+    }
+    for (uint32_t q = b + piece * 128u + lane; q - lane < e; q += pieces * 128u) {
+      uint32_t k4[4], v4[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const bool in = q + 32 * k < e;
+        k4[k] = in ? a.part_key[p + q + 32 * k] : EMPTY;
+        v4[k] = in ? a.part_val[p + q + 32 * k] : 0u;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k4[k] != EMPTY) fine &= add<V>(keys, vals, lg, k4[k], of_bits<MODE>(v4[k]));
+    }
+  }
+  if (!fine) S.bad = 1;
+  __syncthreads();
+  uint32_t gb, bc;
+  best_of_table<MODE>(a, S, keys, vals, slots, threadIdx.x, PB, 0, 0, float(kd), wu, td, G.kr, gb, bc);
+  if (threadIdx.x == 0) {
+    bool last = true;
+    if (!single) {
+      if (bc != EMPTY) atomicMax(&a.hub_best[h], (static_cast<unsigned long long>(gb) << 32) | (0xFFFFFFFFu - bc));
+      __threadfence();
+      last = atomicAdd(&a.hub_done[h], 1u) == R - 1;
+      if (last) {
+        __threadfence();
+        const unsigned long long best = atomicExch(&a.hub_best[h], 0ull);
+        gb = uint32_t(best >> 32);
+        bc = best ? 0xFFFFFFFFu - uint32_t(best) : EMPTY;
+        a.hub_done[h] = 0;
+      }
+    }
+    if (last) {
+      const bool moved = bc != EMPTY && bc != G.zero;
+      if (bc != EMPTY) add_gain(a, fix, G, __uint_as_float(gb));
+      a.hub_move[h] = moved ? bc : EMPTY;
+      a.hub_kd[u] = 0.f;
+      a.vaff[u] = 0;
+      S.cnt[NUM_BINS - 1] += 1;
+      S.edges[NUM_BINS - 1] += a.deg[u];
+      if (moved) {
+        S.hubmv += 1;
+        if constexpr (!SYNC) {
+          atomicAdd(&a.ctot[d], -wu);
+          atomicAdd(&a.ctot[bc], wu);
+          a.vcom[u] = bc;
+        }
+      }
+    }
+    S.next = 0;
+  }
+}
+
+// log2 of the vertices a block takes of a bin at a time (dealt in turn).
+__host__ __device__ constexpr uint32_t chunk_log(int b) { return b <= 2 ? 5 : b == 3 ? 4 : b == 4 ? 3 : b <= 6 ? 2 : 0; }
+
+template <bool SYNC, int MODE>
+__global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ PhaseArgs a) {
+  extern __shared__ __align__(16) uint32_t table[];  // TABLE_WORDS, then the moves, then the list
+  __shared__ Shared S;
+  const uint32_t tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const uint32_t G = gridDim.x, bid = blockIdx.x;
+  const int K = a.colors;
+  const bool in_smem = a.cap <= LIST_CAP;
+  uint2 *mv = in_smem ? reinterpret_cast<uint2 *>(table + TABLE_WORDS) : a.gmv + size_t(bid) * a.cap;
+  uint32_t *list = in_smem ? table + TABLE_WORDS + 2 * LIST_CAP : a.glist + size_t(bid) * a.cap;
+  // the block's share of every class: bins in descending order, the chunks of
+  // all of them dealt to the blocks in turn
+  for (int k = int(tid); k < K; k += PB) {
+    uint32_t q = 0, items = 0;  // chunks of the bins before, the block's list slots of them
+    for (int b = NUM_BINS - 2; b >= 1; --b) {
+      const uint32_t n = a.start[k * NUM_BINS + b + 1] - a.start[k * NUM_BINS + b];
+      const uint32_t chunks = (n + (1u << chunk_log(b)) - 1) >> chunk_log(b);
+      const uint32_t r = q % G;
+      const uint32_t first = bid >= r ? bid - r : bid + G - r;  // the block's first chunk of the bin
+      S.off[k * NUM_BINS + b] = items;
+      S.pos[k * NUM_BINS + b] = first << chunk_log(b);
+      if (first < chunks) items += ((chunks - first + G - 1) / G) << chunk_log(b);
+      q += chunks;
+    }
+    S.tot[k] = items;
+  }
+  if (tid < NUM_BINS) { S.sv[tid] = 0; S.se[tid] = 0; S.edges[tid] = 0; S.cnt[tid] = 0; }
+  if (tid == 0) { S.moves = 0; S.nmv = 0; S.nbig = 0; S.hubmv = 0; S.bad = 0; S.stop = 0; S.next = 0; }
+  __syncthreads();
+  uint32_t nbar = 0;  // barriers so far
+  double el = 0.0;
+  unsigned long long fix = 0;  // the thread's share of the iteration's gain sum
+  unsigned long long sum = 0;
+  uint32_t l = 0;
+  while (l < uint32_t(a.L)) {
+    // what ends an iteration: its gain sum, or the graphs of the union still moving
+    const unsigned long long *total = a.gfix ? &a.ctl->gactive[l % 3] : &a.ctl->fix[l % 3];
+    for (int k = 0; k < K; ++k) {
+      const bool last = k == K - 1;
+      // ---- 1. the block's active vertices of the class, per bin
+      const uint32_t tot = S.tot[k];
+      const uint32_t *off = S.off + k * NUM_BINS;
+      for (uint32_t t0 = tid - lane; t0 < tot; t0 += PB) {
+        const uint32_t t = t0 + lane;
+        int b = -1;
+        uint32_t u = 0, rank = 0;
+        if (t < tot) {
+          b = 1;
+#pragma unroll
+          for (int x = 2; x < NUM_BINS - 1; ++x)
+            if (t < off[x - 1]) b = x;
+          const uint32_t j = t - off[b], lgc = chunk_log(b);
+          const uint32_t p = S.pos[k * NUM_BINS + b] + (((j >> lgc) * G) << lgc) + (j & ((1u << lgc) - 1u));
+          const uint32_t s0 = a.start[k * NUM_BINS + b];
+          if (p < a.start[k * NUM_BINS + b + 1] - s0) {
+            u = a.bins[s0 + p];
+            if (!a.vaff[u] || (a.fa && !a.fa[u]) || (a.gact && !a.gact[a.gid[u]])) b = -1;
+            else if (SYNC) a.vaff[u] = 0;  // (marks of this class come after every block has decided)
+          } else {
+            b = -1;
+          }
+        }
+        const unsigned grp = __match_any_sync(0xffffffffu, b);
+        const int leader = __ffs(grp) - 1;
+        if (b >= 0 && int(lane) == leader) rank = atomicAdd(&S.cnt[b], uint32_t(__popc(grp)));
+        rank = __shfl_sync(0xffffffffu, rank, leader);
+        if (b >= 0) list[off[b] + rank + __popc(grp & ((1u << lane) - 1u))] = u;
+      }
+      __syncthreads();
+      // ---- 2. decide them
+      const uint32_t ch0 = a.chunk_begin[k], nch = a.chunk_begin[k + 1] - ch0;
+      for (uint32_t t = G - 1 - bid; t < nch; t += G) {  // (from the last block: the first ones have the heaviest lists)
+        hub_chunk<MODE>(a, S, ch0 + t, table);
+        __syncthreads();
+      }
+      const uint32_t c10 = S.cnt[10], c9 = S.cnt[9];
+      for (uint32_t i = 0; i < c10; ++i) {
+        group_vertex<SYNC, MODE>(a, S, mv, list[off[10] + i], tid, PB, 0, table, LOG_BLOCK, 10, fix);
+        __syncthreads();
+      }
+      if (c9) {
+        const uint32_t g = wid >> 3;
+        for (uint32_t i = g; i < c9; i += 4)
+          group_vertex<SYNC, MODE>(a, S, mv, list[off[9] + i], tid & 255u, 256, 9 + g, table + g * 8192u, 12, 9, fix);
+        __syncthreads();
+      }
+      // four-warp vertices (tables in the first half of the area), then
+      // whoever is free takes warp-sized units: degree 33-128 (tables in the
+      // second half), then tiles
+      const uint32_t c8 = S.cnt[8], c7 = S.cnt[7];
+      for (uint32_t i = wid >> 2; i < c8 + c7; i += PW / 4) {
+        const int b = i < c8 ? 8 : 7;
+        const uint32_t u = i < c8 ? list[off[8] + i] : list[off[7] + i - c8];
+        group_vertex<SYNC, MODE>(a, S, mv, u, tid & 127u, 128, 1 + (wid >> 2), table + (wid >> 2) * 2048u, 10, b, fix);
+      }
+      {
+        constexpr uint32_t N = TILE_ROUNDS;
+        const uint32_t n6 = S.cnt[6], n5 = n6 + S.cnt[5], n4 = n5 + (S.cnt[4] + N - 1) / N,
+                       n3 = n4 + (S.cnt[3] + 2 * N - 1) / (2 * N), n2 = n3 + (S.cnt[2] + 4 * N - 1) / (4 * N),
+                       n1 = n2 + (S.cnt[1] + 8 * N - 1) / (8 * N);
+        for (;;) {
+          uint32_t x = 0;
+          if (lane == 0) x = atomicAdd(&S.next, 1u);
+          x = __shfl_sync(0xffffffffu, x, 0);
+          if (x >= n1) break;
+          if (x < n5) {
+            const int b = x < n6 ? 6 : 5;
+            const uint32_t u = x < n6 ? list[off[6] + x] : list[off[5] + x - n6];
+            group_vertex<SYNC, MODE>(a, S, mv, u, lane, 32, 0, table + TABLE_WORDS / 2 + wid * 512u, 8, b, fix);
+          } else {
+            const int b = x < n4 ? 4 : x < n3 ? 3 : x < n2 ? 2 : 1;
+            const uint32_t x0 = x < n4 ? n5 : x < n3 ? n4 : x < n2 ? n3 : n2;
+            const uint32_t T = 2u << b;
+            tile_vertices<SYNC, MODE>(a, S, mv, list + off[b], (x - x0) * (N * 32 / T), S.cnt[b], T, b, fix);
+          }
+        }
+      }
+      __syncthreads();
+      if (nch) {  // (the same for every block)
+        if (tid == 0) S.next = 0;
+        if (!grid_barrier(a, S, nbar++, 0, nullptr)) return;
+        const uint32_t m0 = a.merge_begin[k], m1 = a.merge_begin[k + 1];
+        for (uint32_t t = m0 + bid; t < m1; t += G) {
+          hub_merge<SYNC, MODE>(a, S, a.merge[t], table, fix);
+          __syncthreads();
+        }
+      }
+      const uint32_t nmv = S.nmv, moves = nmv + S.hubmv;
+      if (tid == 0) {
+        S.next = 0;
+        S.moves += moves;
+        if (last && bid == 0) { a.ctl->fix[(l + 1) % 3] = 0; a.ctl->gactive[(l + 1) % 3] = 0; }
+      }
+      if (last && !a.gfix) {
+#pragma unroll
+        for (int sh = 16; sh > 0; sh >>= 1) fix += __shfl_xor_sync(0xffffffffu, fix, sh);
+        if (lane == 0 && fix) atomicAdd(&a.ctl->fix[l % 3], fix);
+        fix = 0;
+      }
+      if (tid < NUM_BINS) {
+        S.sv[tid] += S.cnt[tid];
+        S.cnt[tid] = 0;
+        if (last) { S.se[tid] += S.edges[tid]; S.edges[tid] = 0; }
+      }
+      if (!grid_barrier(a, S, nbar++, moves, last ? total : nullptr)) return;
+      const bool any = S.any != 0;  // some block moved a vertex (the same for every block)
+      // ---- 3. commit the decisions, mark the movers' neighbours
+      if constexpr (SYNC) {
+        if (any) {
+          // eight lanes per move; rows above 256 entries by 256 threads
+          uint32_t *big = table;
+          const uint32_t sl = tid & 7u;
+          for (uint32_t i = tid >> 3; i < nmv; i += PB / 8) {
+            const uint2 m = mv[i];
+            const uint64_t o = a.off[m.x];
+            const uint32_t dg = a.deg[m.x];
+            if (sl == 0) {
+              const uint32_t d = a.vcom[m.x];
+              const double wu = a.vtot[m.x];
+              atomicAdd(&a.ctot[d], -wu);
+              atomicAdd(&a.ctot[m.y], wu);
+              a.vcom[m.x] = m.y;
+              if (dg > 256) big[atomicAdd(&S.nbig, 1u)] = m.x;
+            }
+            if (dg <= 256) mark_row(a, m.x, o, dg, sl, 8);
+          }
+          __syncthreads();
+          const uint32_t nbig = S.nbig;
+          for (uint32_t i = wid >> 3; i < nbig; i += PW / 8) mark_row(a, big[i], a.off[big[i]], a.deg[big[i]], tid & 255u, 256);
+          for (uint32_t t = G - 1 - bid; t < nch; t += G) {  // the moved hubs' chunks
+            const uint4 ch = a.chunk[ch0 + t];
+            const uint32_t c = a.hub_move[ch.x], u = ch.w;
+            if (c == EMPTY) continue;
+            if (ch.y == 0 && tid == 0) {
+              const uint32_t d = a.vcom[u];
+              const double wu = a.vtot[u];
+              atomicAdd(&a.ctot[d], -wu);
+              atomicAdd(&a.ctot[c], wu);
+              a.vcom[u] = c;
+            }
+            mark_row(a, u, a.off[u] + ch.y, ch.z - ch.y, tid, PB);
+          }
+        }
+      } else {
+        // the moved hubs' neighbours, by the blocks of their chunks
+        for (uint32_t t = G - 1 - bid; t < nch; t += G) {
+          const uint4 ch = a.chunk[ch0 + t];
+          if (a.hub_move[ch.x] != EMPTY) mark_row(a, ch.w, a.off[ch.w] + ch.y, ch.z - ch.y, tid, PB);
+        }
+      }
+      if (last && a.gfix)  // graph unions: each graph's own stop test
+        for (uint32_t i = bid * PB + tid; i < a.graphs; i += G * PB) phase_control(a, i, l % 3);
+      __syncthreads();
+      if (tid == 0) { S.nbig = 0; S.nmv = 0; S.hubmv = 0; }
+      if ((SYNC && any) || (last && a.gfix)) {
+        if (!grid_barrier(a, S, nbar++, 0, last && a.gfix ? total : nullptr)) return;
+      } else {
+        __syncthreads();
+      }
+    }
+    // ---- the stop test (el <= E), the same value in every block
+    sum = S.sum;
+    __syncthreads();
+    ++l;
+    if (a.gfix) {
+      if (sum == 0ull) break;
+    } else {
+      el = double(sum) / GAIN_FIX / a.M;
+      if (el <= a.E) break;
+    }
+  }
+  if (bid == 0 && tid == 0) {
+    a.ctr->dev_iters = l;
+    a.ctr->dev_el = el;
+    if (a.gfix) a.ctr->gactive = uint32_t(sum);
+  }
+  if (tid < NUM_BINS && S.sv[tid]) {
+    atomicAdd(&a.ctr->bin_vertices[tid], S.sv[tid]);
+    atomicAdd(&a.ctr->vertices, S.sv[tid]);
+    atomicAdd(&a.ctr->bin_edges[tid], S.se[tid]);
+    atomicAdd(&a.ctr->edges, S.se[tid]);
+  }
+  if (tid == 0) {
+    if (S.moves) atomicAdd(&a.ctr->moves, S.moves);
+    if (S.bad) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
+  }
+}
+
+constexpr size_t SMEM = (size_t(TABLE_WORDS) + 3 * LIST_CAP) * sizeof(uint32_t);
+
+template <bool SYNC, int MODE>
+void launch(uint32_t grid, const PhaseArgs &a, cudaStream_t s) {
+  static const bool configured = [] {  // (thread-safe, once)
+    LVG_CUDA(cudaFuncSetAttribute(phase_kernel<SYNC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM)));
+    return true;
+  }();
+  (void)configured;
+  void *args[] = {const_cast<PhaseArgs *>(&a)};
+  LVG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(phase_kernel<SYNC, MODE>), dim3(grid), dim3(PB), args,
+                                       SMEM, s));
+  ++launch_counter();
+}
+
+}  // namespace
+
+bool phase_lists_fit(uint32_t cap) { return cap <= LIST_CAP; }
+
+// Enough blocks for the largest class's warps of work (a block's vertex
+// counts 32 of them, a tile-sized one its share of a warp) to be about one per
+// warp, at most one block per SM: fewer blocks make the barriers cheaper.
+uint32_t phase_grid(const Level &lv) {
+  static const bool coop = [] {
+    int dev = 0, c = 0;
+    LVG_CUDA(cudaGetDevice(&dev));
+    LVG_CUDA(cudaDeviceGetAttribute(&c, cudaDevAttrCooperativeLaunch, dev));
+    return c != 0;
+  }();
+  if (!coop) return 0;
+  static const uint32_t share[NUM_BINS] = {0, 4, 8, 16, 32, 32, 32, 128, 128, 256, 1024, 1024};  // 1/32 warps
+  uint64_t most = 0;
+  for (int k = 0; k < lv.colors; ++k) {
+    uint64_t units = 0;
+    for (int b = 1; b < NUM_BINS - 1; ++b) units += uint64_t(lv.bucket_size(k, b)) * share[b];
+    units += uint64_t(lv.hub.chunk_begin[k + 1] - lv.hub.chunk_begin[k]) * share[NUM_BINS - 1];  // (a block per chunk)
+    most = std::max(most, units / 32);
+  }
+  return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(device_sms()), (most + PW / 2 - 1) / (PW / 2))));
+}
+
+uint32_t phase_list_cap(const Level &lv, uint32_t grid) {
+  uint64_t cap = 1;
+  for (int k = 0; k < lv.colors; ++k) {
+    uint64_t items = 0;
+    for (int b = 1; b < NUM_BINS - 1; ++b) {
+      const uint64_t chunks = (lv.bucket_size(k, b) + (size_t(1) << chunk_log(b)) - 1) >> chunk_log(b);
+      items += ((chunks + grid - 1) / grid) << chunk_log(b);
+    }
+    cap = std::max(cap, items);
+  }
+  return uint32_t(cap);
+}
+
+void launch_phase(bool sync, bool unit, bool whole, uint32_t grid, const PhaseArgs &a, cudaStream_t s) {
+  if (sync) {
+    if (unit) launch<true, UNIT>(grid, a, s);
+    else if (whole) launch<true, WHOLE>(grid, a, s);
+    else launch<true, FLOATS>(grid, a, s);
+  } else {
+    if (unit) launch<false, UNIT>(grid, a, s);
+    else if (whole) launch<false, WHOLE>(grid, a, s);
+    else launch<false, FLOATS>(grid, a, s);
+  }
+}
+
+}  // namespace lvg
