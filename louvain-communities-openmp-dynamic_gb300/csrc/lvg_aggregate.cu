@@ -14,13 +14,15 @@
 // by the driver (launch_next_vertex_weights), not re-summed here.
 //
 // Communities are binned by total degree like vertices in the move kernels:
-// sub-warp tiles / warps with shared tables for small communities, blocks
-// with shared tables (and a global-memory fallback when a community has too
-// many distinct neighbours) for large ones. Inside a tile, the members' edge
-// lists are flattened with a tile prefix scan over member degrees, so lanes
-// stay busy whatever the member degrees are. Internal edges (into the
+// sub-warp tiles / warps with shared tables for total degrees up to 128, where
+// the members' edge lists are flattened with a tile prefix scan over member
+// degrees, so lanes stay busy whatever the member degrees are; blocks of 64 to
+// 1024 threads with shared tables up to 8192, where a few lanes take a member
+// and warps the pieces of a long row; chunks on many blocks above. Internal edges (into the
 // community itself, the hottest key) are summed privately per lane and added
 // once.
+#include <type_traits>
+
 #include "lvg_internal.cuh"
 
 namespace lvg {
@@ -190,274 +192,393 @@ __global__ void __launch_bounds__(TILE_BLOCK) agg_tile_kernel(AggArgs a) {
   }
 }
 
-__device__ __forceinline__ bool smem_add_budget(uint32_t *keys, float *vals, int log2cap, uint32_t c, float w,
-                                                unsigned *used, unsigned limit) {
-  const uint32_t mask = (1u << log2cap) - 1u;
-  uint32_t s = hash_hi(c, log2cap);
-  for (uint32_t probe = 0; probe <= mask; ++probe) {
+// ------------------------------------------------------------ groups of warps
+
+// How a level's weights add up: any FP32, all 1, or whole numbers whose total
+// is below 2^31 (integer shared-memory atomics are native, FP32 ones are a
+// compare-and-swap loop; the integer sums are exact and rounded to FP32 once).
+enum Weights { FLOATS, UNIT, WHOLE };
+template <int MODE>
+using Sum = typename std::conditional<MODE == FLOATS, float, uint32_t>::type;
+template <int MODE>
+__device__ __forceinline__ Sum<MODE> weight(const AggArgs &a, uint64_t i) {
+  if constexpr (MODE == FLOATS) return __ldcs(a.w + i);
+  else if constexpr (MODE == WHOLE) return __float2uint_rn(__ldcs(a.w + i));
+  else return 1u;
+}
+template <int MODE>
+__device__ __forceinline__ float value(uint32_t bits) {
+  if constexpr (MODE == FLOATS) return __uint_as_float(bits);
+  else return float(bits);
+}
+
+// Add w to community c's slot of a table (linear probing from slot s). False
+// when every slot holds another community. `claims` counts the slots taken.
+template <class V>
+__device__ __forceinline__ bool sum_add(uint32_t *keys, uint32_t *vals, uint32_t slots, uint32_t s, uint32_t c, V w,
+                                        uint32_t &claims) {
+  for (uint32_t p = 0; p < slots; ++p) {
     uint32_t k = keys[s];
-    if (k == c) { atomicAdd(&vals[s], w); return true; }
     if (k == EMPTY) {
-      if (atomicAdd(used, 1u) >= limit) return false;
-      uint32_t prev = atomicCAS(&keys[s], EMPTY, c);
-      if (prev == EMPTY || prev == c) { atomicAdd(&vals[s], w); return true; }
+      k = atomicCAS(&keys[s], EMPTY, c);
+      if (k == EMPTY) {
+        k = c;
+        ++claims;
+      }
     }
-    s = (s + 1u) & mask;
+    if (k == c) {
+      atomicAdd(reinterpret_cast<V *>(&vals[s]), w);
+      return true;
+    }
+    s = (s + 1u) & (slots - 1u);
   }
   return false;
 }
+template <class V>
+__device__ __forceinline__ bool sum_add(uint32_t *keys, uint32_t *vals, uint32_t slots, uint32_t s, uint32_t c, V w) {
+  uint32_t claims = 0;
+  return sum_add(keys, vals, slots, s, c, w, claims);
+}
 
-// One block per community (total degree > 512); each warp flattens a
-// 32-member chunk at a time. The community is merged in a shared table of
-// 2^LOGS slots with a claim budget (half the slots); a community with more
-// distinct neighbour communities is redone with a table in its block's
-// region of global memory (2^a.glog2 slots). The table holds
-// min(total degree, community count) * 2 slots rounded up to a power of two.
-template <int B, int LOGS>
-__global__ void __launch_bounds__(B) agg_block_kernel(AggArgs a) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  __shared__ uint32_t s_cnt;
-  __shared__ unsigned s_used;
-  __shared__ int s_over;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint32_t *skeys = reinterpret_cast<uint32_t *>(smem);
-  float *svals = reinterpret_cast<float *>(smem + (size_t(1) << LOGS) * sizeof(uint32_t));
-  uint32_t *gkeys = a.gkeys ? a.gkeys + (size_t(blockIdx.x) << a.glog2) : nullptr;
-  float *gvals = a.gvals ? a.gvals + (size_t(blockIdx.x) << a.glog2) : nullptr;
+// Visit the edges [e0, e1) of the members cmem[m0..m1), counted along the
+// members in order (mpre; nullptr: every edge; `total` edges in all), by the
+// whole block: one to eight lanes per member by the members' mean degree, rows
+// of more than LONG_ROW edges put aside (long_o, long_n; at most MAXLONG of
+// them, the others visited by their own lanes) and then taken in pieces of 128
+// edges, a warp each. Edges into `self` are summed in self_w,
+// the others go to add(community, weight). Ends without a barrier.
+constexpr uint32_t LONG_ROW = 64;
+template <int MODE, int B, int MAXLONG, class Add>
+__device__ __forceinline__ void visit(const AggArgs &a, const uint64_t *mpre, uint64_t e0, uint64_t e1, uint32_t total, uint32_t m0,
+                                      uint32_t m1, uint32_t self, Sum<MODE> &self_w, uint64_t *long_o, uint32_t *long_n,
+                                      uint32_t *nlong, Add add) {
+  constexpr int U = 4;  // edges of a lane in flight
+  auto run = [&](uint64_t o, uint32_t n, uint32_t t, uint32_t step) {
+    for (uint32_t j = t; j < n; j += U * step) {
+      uint32_t c[U];
+      Sum<MODE> w[U];
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        const bool in = j + k * step < n;
+        c[k] = in ? __ldcs(a.key + o + j + k * step) : EMPTY;
+        w[k] = in ? weight<MODE>(a, o + j + k * step) : Sum<MODE>(0);
+      }
+#pragma unroll
+      for (int k = 0; k < U; ++k) c[k] = c[k] != EMPTY ? a.vcom[c[k]] : EMPTY;
+#pragma unroll
+      for (int k = 0; k < U; ++k) {
+        if (c[k] == self) self_w += w[k];
+        else if (c[k] != EMPTY) add(c[k], MODE == UNIT ? Sum<MODE>(1) : w[k]);  // (the constant 1: counted per address)
+      }
+    }
+  };
+  const uint32_t mean = total / (m1 - m0);
+  const uint32_t lgl = mean >= 8 ? 3u : mean >= 4 ? 2u : mean >= 2 ? 1u : 0u, L = 1u << lgl;
+  const uint32_t sl = threadIdx.x & (L - 1u), lead = threadIdx.x & 31u & ~(L - 1u);
+  for (uint32_t m = m0 + (threadIdx.x >> lgl); m < m1; m += B >> lgl) {
+    const uint32_t u = a.cmem[m];
+    uint64_t o = a.off[u];
+    uint32_t n = a.deg[u];
+    if (mpre) {  // only the part of the row inside [e0, e1)
+      const uint64_t f = mpre[m], l = f + n;
+      const uint64_t lo = f > e0 ? f : e0, hi = l < e1 ? l : e1;
+      o += lo - f;
+      n = hi > lo ? uint32_t(hi - lo) : 0u;
+    }
+    uint32_t at = MAXLONG;
+    if (n > LONG_ROW) {
+      if (sl == 0) at = atomicAdd(nlong, 1u);
+      at = __shfl_sync(((1u << L) - 1u) << lead, at, lead);
+    }
+    if (at < MAXLONG) {
+      if (sl == 0) { long_o[at] = o; long_n[at] = n; }
+    } else {
+      run(o, n, sl, L);
+    }
+  }
+  __syncthreads();
+  const uint32_t nl = min(*nlong, uint32_t(MAXLONG));
+  constexpr uint32_t W = B / 32;
+  for (uint32_t i = 0; i < nl; ++i) {
+    const uint32_t n = long_n[i];
+    for (uint32_t p = ((threadIdx.x >> 5) + W - i % W) % W; p * 128u < n; p += W)
+      run(long_o[i] + p * 128u, min(128u, n - p * 128u), threadIdx.x & 31u, 32);
+  }
+}
+
+// One block per community of total degree 129-8192: its members' edges summed
+// per neighbour community in a shared table of twice its total degree (at most
+// 2^LOGS slots, or twice the community count where that is less), then written
+// out as the row. Each of the three steps is a chain of gathers, so the blocks
+// are small where the communities are (64 threads up to total degree 256):
+// several communities per SM at different steps. Measured on level 0 of an
+// R-MAT scale-23 run against one warp per 32 members, a claim counter and an
+// HBM fallback table: total degree 129-512 1.5 -> 0.9 ms, 513-2048 8.7 -> 1.1
+// ms, 2049-8192 7.0 -> 0.9 ms. (Long rows in pieces, not a row per warp: 5.6 ->
+// 1.0 ms for the last.)
+template <int MODE, int B, int LOGS>
+__global__ void __launch_bounds__(B) agg_group_kernel(AggArgs a) {
+  extern __shared__ __align__(16) uint32_t tab[];
+  constexpr int MAXLONG = (1 << LOGS) / (2 * int(LONG_ROW)) + 1;
+  __shared__ uint64_t long_o[MAXLONG];
+  __shared__ uint32_t long_n[MAXLONG];
+  __shared__ uint32_t s_cnt, s_nlong;
+  const int lane = threadIdx.x & 31;
   unsigned long long nread = 0;
   bool ok = true;
   for (uint32_t i = blockIdx.x; i < a.count; i += gridDim.x) {
     const uint32_t c = a.list[i];
     const uint32_t m0 = a.coff[c], m1 = a.coff[c + 1];
     const uint64_t y0 = a.yoff[c], tdeg = a.yoff[c + 1] - y0;
-    const uint64_t want = 2ull * (tdeg < a.cn ? tdeg : a.cn);
-    int lg = min(LOGS, max(1, ceil_log2(want)));
-    uint32_t ccap = 1u << lg;
-    for (uint32_t s = threadIdx.x; s < ccap; s += B) { skeys[s] = EMPTY; svals[s] = 0.f; }
-    if (threadIdx.x == 0) { s_cnt = 0; s_used = 0; s_over = 0; }
+    const int lg = min(LOGS, max(5, ceil_log2(2ull * (tdeg < a.cn ? tdeg : a.cn))));
+    const uint32_t slots = 1u << lg;
+    uint32_t *keys = tab, *vals = tab + slots;
+    for (uint32_t s = threadIdx.x; s < slots; s += B) { keys[s] = EMPTY; vals[s] = 0u; }
+    if (threadIdx.x == 0) { s_cnt = 0; s_nlong = 0; }
     __syncthreads();
-    const unsigned limit = ccap >> 1;
-    float self_w = 0.f;
-    uint64_t nr = 0;
-    for (uint32_t b0 = m0 + uint32_t(wid) * 32; b0 < m1; b0 += B) {
-      const uint32_t b1 = b0 + 32 < m1 ? b0 + 32 : m1;
-      nr += visit_members<32>(a, b0, b1, lane, 0xffffffffu, c, self_w, [&](uint32_t k, float w) {
-        if (smem_add_budget(skeys, svals, lg, k, w, &s_used, limit)) return true;
-        s_over = 1;
-        return false;
-      });
-    }
-    __syncthreads();
-    uint32_t *keys = skeys;
-    float *vals = svals;
-    if (s_over) {
-      lg = min(a.glog2, max(1, ceil_log2(want)));
-      ccap = 1u << lg;
-      keys = gkeys;
-      vals = gvals;
-      if (!keys) { ok = false; ccap = 0; }
-      for (uint32_t s = threadIdx.x; s < ccap; s += B) { keys[s] = EMPTY; vals[s] = 0.f; }
-      __syncthreads();
-      self_w = 0.f;
-      nr = 0;
-      if (keys)
-        for (uint32_t b0 = m0 + uint32_t(wid) * 32; b0 < m1; b0 += B) {
-          const uint32_t b1 = b0 + 32 < m1 ? b0 + 32 : m1;
-          nr += visit_members<32>(a, b0, b1, lane, 0xffffffffu, c, self_w, [&](uint32_t k, float w) {
-            ok &= table_add(keys, vals, lg, k, w);
-            return true;
-          });
-        }
-    }
-    nread += nr;
+    Sum<MODE> self_w = 0;
+    visit<MODE, B, MAXLONG>(a, nullptr, 0, 0, uint32_t(tdeg), m0, m1, c, self_w, long_o, long_n, &s_nlong,
+                            [&](uint32_t k, Sum<MODE> w) { ok &= sum_add(keys, vals, slots, hash_hi(k, lg), k, w); });
+    if (threadIdx.x == 0) nread += tdeg;
     // internal weight: one insertion per warp
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) self_w += __shfl_xor_sync(0xffffffffu, self_w, o);
-    if (lane == 0 && self_w != 0.f && ccap) ok &= table_add(keys, vals, lg, c, self_w);
+    if (lane == 0 && self_w != Sum<MODE>(0)) ok &= sum_add(keys, vals, slots, hash_hi(c, lg), c, self_w);
     __syncthreads();
-    for (uint32_t s0 = 0; s0 < ccap; s0 += B) {
-      const uint32_t s = s0 + threadIdx.x;
-      const uint32_t k = s < ccap ? keys[s] : EMPTY;
-      const bool has = k != EMPTY;
-      const unsigned bal = __ballot_sync(0xffffffffu, has);
+    for (uint32_t s = threadIdx.x; s - lane < slots; s += B) {
+      const uint32_t k = s < slots ? keys[s] : EMPTY;
+      const unsigned bal = __ballot_sync(0xffffffffu, k != EMPTY);
       uint32_t base = 0;
       if (lane == 0 && bal) base = atomicAdd(&s_cnt, uint32_t(__popc(bal)));
       base = __shfl_sync(0xffffffffu, base, 0);
-      if (has) {
-        const uint32_t r = __popc(bal & ((1u << lane) - 1u));
-        const float v = vals[s];
-        a.ykey[y0 + base + r] = k;
-        a.yw[y0 + base + r] = v;
+      if (k != EMPTY) {
+        const uint64_t y = y0 + base + __popc(bal & ((1u << lane) - 1u));
+        a.ykey[y] = k;
+        a.yw[y] = value<MODE>(vals[s]);
       }
     }
     __syncthreads();
     if (threadIdx.x == 0) a.ydeg[c] = s_cnt;
-    __syncthreads();
   }
-  if (lane != 0) nread = 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) nread += __shfl_xor_sync(0xffffffffu, nread, o);
-  const bool bad = __any_sync(0xffffffffu, !ok);
-  if (lane == 0) {
-    if (nread) atomicAdd(&a.ctr->agg_edges, nread);
-    if (bad) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
-  }
+  if (threadIdx.x == 0 && nread) atomicAdd(&a.ctr->agg_edges, nread);
+  if (!ok) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
 }
 
 // ------------------------------------------------------------ communities above total degree 8192
 //
-// A community's members' edges, flattened in member order, are the range
-// [mpre[m0], mpre[m1]) of the member-degree prefix mpre. The largest
-// communities (after the first pass of a power-law graph, a handful hold
-// most of the edges) are cut into AGG_CHUNK-edge chunks, one block each; a
-// block merges its chunk in a listed shared table with warp-aggregated
-// inserts and adds the distinct (community, weight) pairs to the community's
-// table in global memory, which agg_gfinish_kernel then writes out as the
-// community's row. Each block finds the member of every edge of a batch by a
-// binary search over the batch's window of member prefixes in shared memory.
+// A community's members' edges, counted along the members in order, are the
+// range [mpre[m0], mpre[m1]) of the member-degree prefix mpre. The largest
+// communities (after the first pass of a power-law graph, a handful hold most
+// of the edges) are cut into AGG_CHUNK-edge chunks, a run of consecutive ones
+// per block. A block sums its chunks per neighbour community in a shared table,
+// as many as leave room for the next chunk's communities, and writes the
+// (community, weight) pairs out as a list grouped by the community's hash
+// partition (parts: as many as leave about AGG_PART distinct communities each;
+// seg: the groups' bounds). A second kernel, a block per (community,
+// partition), sums a partition's pairs of all lists the same way and appends
+// them to the row. No table in global memory: its atomics (two per pair) took
+// longer than both kernels. Measured on an R-MAT scale-23 run against such
+// tables: level 0 4.7 -> 2.9 ms, scale 18 2.4 -> 0.1 ms (too few chunks to hide
+// the atomics); a fixed eight lanes per list in the merge took 11 ms where a
+// community has two partitions.
+// Partitions take every bit of the id (two multiply-and-shift rounds), unlike
+// the tables' slots.
+__device__ __forceinline__ uint32_t part_of(uint32_t c, uint32_t R) {
+  c = (c ^ (c >> 16)) * 0x7FEB352Du;
+  c = (c ^ (c >> 15)) * 0x846CA68Bu;
+  return __umulhi(c ^ (c >> 16), R);
+}
+// Table slots by a hash that is not the rows' order: the rows of an aggregated
+// level are stored in the order of hash_hi, and a chunk of one would crowd
+// into one stretch of slots.
+constexpr int CHUNK_LOGS = 13, MERGE_LOGS = 14;
+static_assert((1u << CHUNK_LOGS) == 2 * AGG_CHUNK, "a chunk's communities fill half its table");
+static_assert((1u << MERGE_LOGS) == 2 * AGG_PART, "a partition's communities fill about half its table");
+__device__ __forceinline__ uint32_t chunk_slot(uint32_t c) { return (c * 0x85EBCA6Bu) >> (32 - CHUNK_LOGS); }
 
-template <int B, int LOGS>
+// A warp finds the last m in [lo, hi) with mpre[m] <= e, 32 probes a step.
+__device__ __forceinline__ uint32_t member_of(const uint64_t *mpre, uint32_t lo, uint32_t hi, uint64_t e) {
+  const uint32_t lane = threadIdx.x & 31u;
+  while (hi - lo > 1) {
+    const uint32_t step = (hi - lo + 31) / 32;
+    const uint64_t x = uint64_t(lo) + uint64_t(lane + 1) * step;
+    const unsigned m = __ballot_sync(0xffffffffu, x < hi && mpre[x] <= e);
+    lo += __popc(m) * step;
+    hi = min(hi, lo + step);
+  }
+  return lo;
+}
+
+template <int MODE, int B>
 __global__ void __launch_bounds__(B) agg_chunk_kernel(AggArgs a, AggChunks ch) {
-  extern __shared__ __align__(16) uint8_t smem[];
-  constexpr uint32_t CS = 1u << LOGS;
-  __shared__ uint64_t win[B + 1];
-  __shared__ unsigned s_used;
-  __shared__ uint32_t s_mi;
-  uint32_t *skeys = reinterpret_cast<uint32_t *>(smem);
-  float *svals = reinterpret_cast<float *>(smem + size_t(CS) * 4);
-  uint32_t *slist = reinterpret_cast<uint32_t *>(smem + size_t(CS) * 8);
-  for (uint32_t s2 = threadIdx.x; s2 < CS; s2 += B) { skeys[s2] = EMPTY; svals[s2] = 0.f; }
-  const uint2 cj = ch.chunk[blockIdx.x];  // (community slot, chunk index)
-  const uint32_t j = cj.x;
+  extern __shared__ __align__(16) uint32_t tab[];  // keys, values, partition counters
+  constexpr uint32_t CS = 1u << CHUNK_LOGS;
+  constexpr int MAXLONG = int(AGG_CHUNK / LONG_ROW) + 1;
+  __shared__ uint64_t long_o[MAXLONG];
+  __shared__ uint32_t long_n[MAXLONG];
+  __shared__ uint32_t s_nlong, s_m[2], s_used, s_list;
+  uint32_t *keys = tab, *vals = tab + CS, *pc = tab + 2 * CS;
+  const int lane = threadIdx.x & 31;
+  const uint4 cr = ch.run[blockIdx.x];  // (community slot, first chunk, chunks)
+  const uint32_t j = cr.x, R = ch.parts[j];
   const uint32_t c = ch.comm[j];
   const uint32_t m0 = a.coff[c], m1 = a.coff[c + 1];
   const uint64_t ebeg = ch.mpre[m0], eend = ch.mpre[m1];
-  const uint64_t e0 = ebeg + uint64_t(cj.y) * AGG_CHUNK;
-  const uint64_t e1 = min(eend, e0 + AGG_CHUNK);
-  uint32_t *gk = ch.gkeys + ch.toff[j];
-  float *gv = ch.gvals + ch.toff[j];
-  const int glg = ch.tlog[j];
-  const unsigned limit = CS >> 1;
-  if (threadIdx.x == 0) {
-    s_used = 0;
-    // the member holding edge e0: the last m in [m0, m1) with mpre[m] <= e0
-    uint32_t lo = m0, hi = m1 - 1;
-    while (lo < hi) {
-      const uint32_t mid = lo + (hi - lo + 1) / 2;
-      if (ch.mpre[mid] <= e0) lo = mid; else hi = mid - 1;
-    }
-    s_mi = lo;
-  }
-  __syncthreads();
-  unsigned long long nread = 0;
+  uint32_t from = cr.y;  // the first chunk in the table
   bool ok = true;
-  uint64_t base = e0;
-  while (base < e1) {  // block-uniform
-    const uint32_t mi = s_mi;
-    const uint32_t nw = min(uint32_t(B), m1 - mi);  // members staged: mi .. mi+nw-1
-    for (uint32_t t = threadIdx.x; t <= nw; t += B) win[t] = ch.mpre[mi + t];
-    __syncthreads();
-    // this pass of the loop: edges [base, stop), all inside the staged members
-    const uint64_t stop = min(e1, min(base + B, win[nw]));
-    const uint64_t e = base + threadIdx.x;
-    uint32_t key = EMPTY;
-    float w = 0.f;
-    if (e < stop) {
-      uint32_t lo = 0, hi = nw - 1;  // last window entry <= e
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (win[mid] <= e) lo = mid; else hi = mid - 1;
-      }
-      const uint32_t u = a.cmem[mi + lo];
-      const uint64_t x = a.off[u] + (e - win[lo]);
-      key = a.vcom[__ldcs(a.key + x)];
-      w = __ldcs(a.w + x);
-      ++nread;
+  for (uint32_t k = cr.y; k < cr.y + cr.z; ++k) {
+    const uint64_t e0 = ebeg + uint64_t(k) * AGG_CHUNK;
+    const uint64_t e1 = min(eend, e0 + AGG_CHUNK);
+    if (from == k) {
+      for (uint32_t s = threadIdx.x; s < CS; s += B) { keys[s] = EMPTY; vals[s] = 0u; }
+      for (uint32_t r = threadIdx.x; r < R; r += B) pc[r] = 0;
+      if (threadIdx.x == 0) s_used = 0;
     }
-    agg_warp_insert(key, w, [&](uint32_t k, float v) {
-      // the shared table while its claim budget lasts, then the global one
-      const uint32_t mask = CS - 1u;
-      uint32_t sl = hash_hi(k, LOGS);
-      for (uint32_t probe = 0; probe <= mask; ++probe) {
-        const uint32_t kk = skeys[sl];
-        if (kk == k) { atomicAdd(&svals[sl], v); return true; }
-        if (kk == EMPTY) {
-          const unsigned r = atomicAdd(&s_used, 1u);
-          if (r >= limit) break;
-          const uint32_t prev = atomicCAS(&skeys[sl], EMPTY, k);
-          if (prev == EMPTY) { slist[r] = sl; atomicAdd(&svals[sl], v); return true; }
-          slist[r] = EMPTY;
-          if (prev == k) { atomicAdd(&svals[sl], v); return true; }
-        }
-        sl = (sl + 1u) & mask;
-      }
-      ok &= table_add(gk, gv, glg, k, v);
-      return true;
-    });
-    __syncthreads();  // every thread has read win[] and s_mi
-    // the next round starts at the member holding edge `stop`
-    if (threadIdx.x == 0) {
-      if (stop < win[nw]) {
-        uint32_t lo = 0, hi = nw - 1;
-        while (lo < hi) {
-          const uint32_t mid = (lo + hi + 1) >> 1;
-          if (win[mid] <= stop) lo = mid; else hi = mid - 1;
-        }
-        s_mi = mi + lo;
-      } else {
-        s_mi = mi + nw;  // past the staged members (also when they had no edges left)
-      }
+    if (threadIdx.x == 0) s_nlong = 0;
+    if (threadIdx.x < 64) {  // the members holding the chunk's first and last edge
+      const uint32_t m = member_of(ch.mpre, m0, m1, threadIdx.x < 32 ? e0 : e1 - 1);
+      if (lane == 0) s_m[threadIdx.x >> 5] = m;
     }
-    base = stop;
     __syncthreads();
-  }
-  // the shared table into the community's global table
-  const unsigned nl = min(s_used, limit);
-  for (unsigned i = threadIdx.x; i < nl; i += B) {
-    const uint32_t sl = slist[i];
-    if (sl != EMPTY) ok &= table_add(gk, gv, glg, skeys[sl], svals[sl]);
-  }
-  const int lane = threadIdx.x & 31;
+    Sum<MODE> self_w = 0;
+    uint32_t claims = 0;
+    visit<MODE, B, MAXLONG>(a, ch.mpre, e0, e1, uint32_t(e1 - e0), s_m[0], s_m[1] + 1, c, self_w, long_o, long_n, &s_nlong,
+                            [&](uint32_t x, Sum<MODE> w) { ok &= sum_add(keys, vals, CS, chunk_slot(x), x, w, claims); });
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) nread += __shfl_xor_sync(0xffffffffu, nread, o);
-  const bool bad = __any_sync(0xffffffffu, !ok);
-  if (lane == 0) {
-    if (nread) atomicAdd(&a.ctr->agg_edges, nread);
-    if (bad) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
+    for (int o = 16; o > 0; o >>= 1) self_w += __shfl_xor_sync(0xffffffffu, self_w, o);
+    if (lane == 0 && self_w != Sum<MODE>(0)) ok &= sum_add(keys, vals, CS, chunk_slot(c), c, self_w, claims);
+    claims = __reduce_add_sync(0xffffffffu, claims);
+    if (lane == 0 && claims) atomicAdd(&s_used, claims);
+    __syncthreads();
+    // room for another chunk: at most 5/8 of the slots taken after it
+    if (k + 1 < cr.y + cr.z && s_used <= CS / 8) {
+      __syncthreads();
+      continue;
+    }
+    // the pairs, grouped by partition: counts, their prefix, places (lanes of
+    // one partition take theirs together)
+    for (uint32_t s = threadIdx.x; s < CS; s += B) {  // (whole warps)
+      const uint32_t r = keys[s] != EMPTY ? part_of(keys[s], R) : EMPTY;
+      const unsigned grp = __match_any_sync(0xffffffffu, r);
+      if (r != EMPTY && (grp & ((1u << lane) - 1u)) == 0u) atomicAdd(&pc[r], uint32_t(__popc(grp)));
+    }
+    if (threadIdx.x == 0) {
+      s_list = atomicAdd(&ch.nlist[j], 1u);
+      ch.list_at[ch.list_off[j] + s_list] = from;
+    }
+    __syncthreads();
+    uint32_t *seg = ch.seg + ch.seg_off[j] + uint64_t(s_list) * (R + 1);
+    if (threadIdx.x < 32) {
+      uint32_t carry = 0;
+      for (uint32_t r0 = 0; r0 < R; r0 += 32) {
+        const uint32_t r = r0 + lane, x = r < R ? pc[r] : 0u;
+        uint32_t inc = x;
+#pragma unroll
+        for (int sh = 1; sh < 32; sh <<= 1) {
+          const uint32_t y = __shfl_up_sync(0xffffffffu, inc, sh);
+          if (lane >= sh) inc += y;
+        }
+        if (r < R) { pc[r] = carry + inc - x; seg[r] = carry + inc - x; }
+        carry += __shfl_sync(0xffffffffu, inc, 31);
+      }
+      if (lane == 0) seg[R] = carry;
+    }
+    __syncthreads();
+    const uint64_t p0 = ch.part_off[j] + uint64_t(from) * AGG_CHUNK;
+    for (uint32_t s = threadIdx.x; s < CS; s += B) {
+      const uint32_t x = keys[s];
+      const uint32_t r = x != EMPTY ? part_of(x, R) : EMPTY;
+      const unsigned grp = __match_any_sync(0xffffffffu, r);
+      const int leader = __ffs(grp) - 1;
+      uint32_t at = 0;
+      if (r != EMPTY && lane == leader) at = atomicAdd(&pc[r], uint32_t(__popc(grp)));
+      at = __shfl_sync(0xffffffffu, at, leader) + __popc(grp & ((1u << lane) - 1u));
+      if (r != EMPTY) ch.pairs[p0 + at] = make_uint2(x, vals[s]);
+    }
+    __syncthreads();
+    from = k + 1;
   }
+  if (threadIdx.x == 0) {
+    const uint64_t e0 = ebeg + uint64_t(cr.y) * AGG_CHUNK;
+    atomicAdd(&a.ctr->agg_edges, (unsigned long long)(min(eend, e0 + uint64_t(cr.z) * AGG_CHUNK) - e0));
+  }
+  if (!ok) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
 }
 
-// The global tables of the chunked communities into their rows: a thread
-// per slot, output positions by a warp-aggregated cursor per community
-// (ydeg).
-__global__ void agg_gfinish_kernel(AggArgs a, AggChunks ch, uint64_t slots) {
+template <int MODE, int B>
+__global__ void __launch_bounds__(B) agg_merge_kernel(AggArgs a, AggChunks ch) {
+  extern __shared__ __align__(16) uint32_t tab[];
+  constexpr uint32_t CS = 1u << MERGE_LOGS;
+  __shared__ uint32_t s_n, s_at;
+  uint32_t *keys = tab, *vals = tab + CS;
   const int lane = threadIdx.x & 31;
-  for (uint64_t base = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * 32; base < slots;
-       base += uint64_t(gridDim.x) * blockDim.x) {
-    const uint64_t t = base + lane;
-    uint32_t jj = EMPTY, k = EMPTY;
-    float v = 0.f;
-    if (t < slots) {
-      uint32_t lo = 0, hi = ch.n - 1;  // the community whose region holds slot t
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (ch.toff[mid] <= t) lo = mid; else hi = mid - 1;
-      }
-      k = ch.gkeys[t];
-      if (k != EMPTY) { jj = lo; v = ch.gvals[t]; }
+  const uint2 task = ch.merge[blockIdx.x];  // (community slot, partition)
+  const uint32_t j = task.x, r = task.y, R = ch.parts[j];
+  const uint32_t c = ch.comm[j];
+  const uint32_t nc = ch.nlist[j];
+  const uint32_t *list_at = ch.list_at + ch.list_off[j];
+  for (uint32_t s = threadIdx.x; s < CS; s += B) { keys[s] = EMPTY; vals[s] = 0u; }
+  if (threadIdx.x == 0) s_n = 0;
+  __syncthreads();
+  bool ok = true;
+  // L lanes per list's group of pairs, about a quarter of the pairs a group
+  // has where every community of a chunk differs (a community of two
+  // partitions has few large groups, one of hundreds thousands of small ones),
+  // the next group's bounds loaded ahead
+  const uint32_t want = AGG_CHUNK / (4u * R);
+  const uint32_t L = min(256u, max(8u, want ? 1u << (31 - __clz(want)) : 0u));
+  const uint32_t sl = threadIdx.x & (L - 1u), step = B / L;
+  const uint32_t *seg = ch.seg + ch.seg_off[j] + r;
+  const uint2 *p = ch.pairs + ch.part_off[j];
+  uint32_t k = threadIdx.x / L;
+  uint32_t b = 0, e = 0, f = 0;
+  if (k < nc) { b = seg[uint64_t(k) * (R + 1)]; e = seg[uint64_t(k) * (R + 1) + 1]; f = list_at[k]; }
+  for (; k < nc; k += step) {
+    uint32_t nb = 0, ne = 0, nf = 0;
+    if (k + step < nc) {
+      nb = seg[uint64_t(k + step) * (R + 1)];
+      ne = seg[uint64_t(k + step) * (R + 1) + 1];
+      nf = list_at[k + step];
     }
-    const unsigned grp = __match_any_sync(0xffffffffu, jj);
-    const int leader = __ffs(grp) - 1;
+    const uint2 *g = p + uint64_t(f) * AGG_CHUNK;
+    for (uint32_t q = b + sl; q < e; q += 4 * L) {  // four pairs of a lane in flight
+      uint2 x[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) x[u] = q + u * L < e ? __ldcs(g + q + u * L) : make_uint2(EMPTY, 0u);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (x[u].x == EMPTY) continue;
+        Sum<MODE> w;
+        if constexpr (MODE == FLOATS) w = __uint_as_float(x[u].y);
+        else w = x[u].y;
+        ok &= sum_add(keys, vals, CS, hash_hi(x[u].x, MERGE_LOGS), x[u].x, w);
+      }
+    }
+    b = nb;
+    e = ne;
+    f = nf;
+  }
+  __syncthreads();
+  uint32_t mine = 0;
+  for (uint32_t s = threadIdx.x; s < CS; s += B) mine += keys[s] != EMPTY;
+  mine = __reduce_add_sync(0xffffffffu, mine);
+  if (lane == 0 && mine) atomicAdd(&s_n, mine);
+  __syncthreads();
+  if (threadIdx.x == 0) s_at = s_n ? atomicAdd(&a.ydeg[c], s_n) : 0u;  // the partition's place in the row
+  __syncthreads();
+  const uint64_t y0 = a.yoff[c];
+  for (uint32_t s = threadIdx.x; s < CS; s += B) {
+    const uint32_t k = keys[s];
+    const unsigned bal = __ballot_sync(0xffffffffu, k != EMPTY);
     uint32_t at = 0;
-    const uint32_t c = jj != EMPTY ? ch.comm[jj] : 0u;
-    if (jj != EMPTY && lane == leader) at = atomicAdd(&a.ydeg[c], uint32_t(__popc(grp)));
-    at = __shfl_sync(grp, at, leader);
-    if (jj != EMPTY) {
-      const uint64_t y = a.yoff[c] + at + __popc(grp & ((1u << lane) - 1u));
-      a.ykey[y] = k;
-      a.yw[y] = v;
+    if (lane == 0 && bal) at = atomicAdd(&s_at, uint32_t(__popc(bal)));
+    at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
+    if (k != EMPTY) {
+      a.ykey[y0 + at] = k;
+      a.yw[y0 + at] = value<MODE>(vals[s]);
     }
   }
+  if (!ok) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
 }
 
 __global__ void comm_tdeg_kernel(const uint32_t *list, size_t n, const uint64_t *yoff, uint64_t *out) {
@@ -500,15 +621,50 @@ void launch_tile(const AggArgs &a, cudaStream_t s) {
   LVG_CHECK_LAUNCH();
 }
 
-template <int B, int LOGS>
-void launch_big(const AggArgs &a, cudaStream_t s) {
+template <int MODE, int B, int LOGS>
+void launch_group(const AggArgs &a, cudaStream_t s) {
   const size_t smem = (size_t(1) << LOGS) * 8;
-  auto k = agg_block_kernel<B, LOGS>;
-  static bool configured = false;
-  if (!configured) { set_smem(k, smem); configured = true; }
-  unsigned grid = unsigned(global_table_blocks(a.count));
+  auto k = agg_group_kernel<MODE, B, LOGS>;
+  // as many blocks as fit the device (queried once; thread-safe)
+  static const unsigned resident = [&] {
+    set_smem(k, smem);
+    int per_sm = 0;
+    LVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, B, smem));
+    return unsigned(per_sm > 0 ? per_sm : 1) * unsigned(sms());
+  }();
+  const unsigned grid = a.count < resident ? a.count : resident;
   if (!grid) return;
   k<<<grid, B, smem, s>>>(a);
+  LVG_CHECK_LAUNCH();
+}
+
+template <int MODE>
+void launch_groups(int b, const AggArgs &a, cudaStream_t s) {
+  switch (b) {
+    case 7: launch_group<MODE, 64, 9>(a, s); break;
+    case 8: launch_group<MODE, 128, 10>(a, s); break;
+    case 9: launch_group<MODE, 256, 12>(a, s); break;
+    case 10: launch_group<MODE, 1024, 14>(a, s); break;
+    default: break;
+  }
+}
+
+constexpr int AGG_CHUNK_B = 512, AGG_MERGE_B = 1024;
+template <int MODE>
+void launch_chunks(const AggArgs &a, const AggChunks &ch, size_t runs, size_t merges, uint32_t max_parts,
+                   cudaStream_t s) {
+  const size_t smem1 = (size_t(1) << CHUNK_LOGS) * 8, smem2 = (size_t(1) << MERGE_LOGS) * 8;
+  auto k1 = agg_chunk_kernel<MODE, AGG_CHUNK_B>;
+  auto k2 = agg_merge_kernel<MODE, AGG_MERGE_B>;
+  static const bool configured = [&] {
+    set_smem(k1, smem1 + size_t(AGG_MAX_PARTS) * 4);
+    set_smem(k2, smem2);
+    return true;
+  }();
+  (void)configured;
+  k1<<<unsigned(runs), AGG_CHUNK_B, smem1 + size_t(max_parts) * 4, s>>>(a, ch);  // (the partitions' counters behind)
+  LVG_CHECK_LAUNCH();
+  k2<<<unsigned(merges), AGG_MERGE_B, smem2, s>>>(a, ch);
   LVG_CHECK_LAUNCH();
 }
 
@@ -526,15 +682,12 @@ void launch_member_degrees(const uint32_t *cmem, const uint32_t *deg, size_t n, 
   LVG_CHECK_LAUNCH();
 }
 
-constexpr int AGG_CHUNK_B = 256, AGG_CHUNK_LOGS = 11;
-
-void launch_aggregate_chunks(const AggArgs &a, const AggChunks &ch, size_t chunks, uint64_t slots, cudaStream_t s) {
-  if (!chunks) return;
-  const size_t smem = (size_t(1) << AGG_CHUNK_LOGS) * 10;  // keys, values, claimed list
-  agg_chunk_kernel<AGG_CHUNK_B, AGG_CHUNK_LOGS><<<unsigned(chunks), AGG_CHUNK_B, smem, s>>>(a, ch);
-  LVG_CHECK_LAUNCH();
-  agg_gfinish_kernel<<<grid_for(slots, 256), 256, 0, s>>>(a, ch, slots);
-  LVG_CHECK_LAUNCH();
+void launch_aggregate_chunks(const AggArgs &a, const AggChunks &ch, size_t runs, size_t merges, uint32_t max_parts,
+                             cudaStream_t s) {
+  if (!runs) return;
+  if (a.unit) launch_chunks<UNIT>(a, ch, runs, merges, max_parts, s);
+  else if (a.whole) launch_chunks<WHOLE>(a, ch, runs, merges, max_parts, s);
+  else launch_chunks<FLOATS>(a, ch, runs, merges, max_parts, s);
 }
 
 void launch_aggregate_bin(int b, const AggArgs &a, cudaStream_t s) {
@@ -545,12 +698,11 @@ void launch_aggregate_bin(int b, const AggArgs &a, cudaStream_t s) {
     case 4: launch_tile<32, 64>(a, s); break;
     case 5: launch_tile<32, 128>(a, s); break;
     case 6: launch_tile<32, 256>(a, s); break;
-    case 7: launch_tile<32, 512>(a, s); break;
-    case 8: launch_tile<32, 1024>(a, s); break;
-    case 9: launch_big<256, 12>(a, s); break;
-    case 10: launch_big<512, 13>(a, s); break;
-    case 11: launch_big<512, 13>(a, s); break;
-    default: break;
+    default:
+      if (a.unit) launch_groups<UNIT>(b, a, s);
+      else if (a.whole) launch_groups<WHOLE>(b, a, s);
+      else launch_groups<FLOATS>(b, a, s);
+      break;
   }
 }
 

@@ -969,83 +969,106 @@ Level aggregate(lvg_graph *g, const Level &lv, const uint32_t *com, size_t CN, i
   launch_community_scatter(lv, com, W.csize.p, W.ccur.p, W.cmem.p, s);
   // Empty communities never reach a kernel: zero their rows first.
   LVG_CUDA(cudaMemsetAsync(nl.deg, 0, CN * sizeof(uint32_t), s));
-  // Global fallback regions of bins 9-10 (bin 11 is chunked below).
-  int glog2[NUM_BINS] = {};
-  size_t need = 0;
-  for (int b = 9; b < NUM_BINS - 1; ++b) {
-    const size_t cnt = cb[b + 1] - cb[b];
-    if (!cnt) continue;
-    glog2[b] = global_table_log2(std::min<uint64_t>(cmax[b], CN));
-    need = std::max(need, size_t(global_table_blocks(cnt)) << glog2[b]);
-  }
-  if (need) {
-    W.gkeys.ensure(need);
-    W.gvals.ensure(need);
-  }
+  AggArgs a{};
+  a.off = lv.off; a.deg = lv.deg; a.key = lv.key; a.w = lv.w;
+  a.vcom = com; a.coff = W.csize.p; a.cmem = W.cmem.p;
+  a.yoff = nl.off; a.ydeg = nl.deg; a.ykey = nl.key; a.yw = nl.w;
+  a.ctr = g->ctr.p; a.cn = uint32_t(CN);
+  a.whole = lv.whole && g->total_weight < 2147483648.0;  // (no integer sum overflows)
+  a.unit = lv.unit && a.whole;
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   if (g->profiling) e0 = g->events.record(s);
-  for (int b = 1; b < NUM_BINS - 1; ++b) {
+  // the bins are independent (disjoint rows): the block bins on side streams
+  // beside the tiles and the chunked communities
+  ensure_aux(g);
+  LVG_CUDA(cudaEventRecord(g->fork_ev, s));
+  for (int i = 0; i < 4; ++i) LVG_CUDA(cudaStreamWaitEvent(g->aux[i], g->fork_ev, 0));
+  for (int b = NUM_BINS - 2; b >= 1; --b) {
     const size_t cnt = cb[b + 1] - cb[b];
     if (!cnt) continue;
-    AggArgs a;
-    a.off = lv.off; a.deg = lv.deg; a.key = lv.key; a.w = lv.w;
-    a.vcom = com; a.coff = W.csize.p; a.cmem = W.cmem.p;
     a.list = W.cbins.p + cb[b];
     a.count = uint32_t(cnt);
-    a.yoff = nl.off; a.ydeg = nl.deg; a.ykey = nl.key; a.yw = nl.w;
-    a.ctr = g->ctr.p; a.cn = uint32_t(CN);
-    a.gkeys = need ? W.gkeys.p : nullptr; a.gvals = need ? W.gvals.p : nullptr; a.glog2 = glog2[b];
-    launch_aggregate_bin(b, a, s);
+    launch_aggregate_bin(b, a, g->aux[b == 10 ? 0 : b == 9 ? 1 : b >= 7 ? 2 : 3]);
     ++g->stats.aggregate_launches;
   }
   // communities above total degree 8192: chunks of AGG_CHUNK edges over many
-  // blocks, merged in per-community tables in HBM
+  // blocks, merged by hash partitions of their neighbour communities
   if (const size_t n11 = cb[NUM_BINS] - cb[NUM_BINS - 1]) {
     const uint32_t *list = W.cbins.p + cb[NUM_BINS - 1];
-    uint32_t members = 0;
-    LVG_CUDA(cudaMemcpyAsync(&members, W.csize.p + CN, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     W.agg_tdeg.ensure(n11);
     launch_comm_tdeg(list, n11, nl.off, W.agg_tdeg.p, s);
-    std::vector<uint64_t> tdeg(n11);
-    LVG_CUDA(cudaMemcpyAsync(tdeg.data(), W.agg_tdeg.p, n11 * 8, cudaMemcpyDeviceToHost, s));
+    if (W.agg_htdeg.n < n11 + 1) LVG_CUDA(cudaStreamSynchronize(s));
+    W.agg_htdeg.ensure(n11 + 1);
+    LVG_CUDA(cudaMemcpyAsync(W.agg_htdeg.p, W.agg_tdeg.p, n11 * 8, cudaMemcpyDeviceToHost, s));
+    LVG_CUDA(cudaMemcpyAsync(W.agg_htdeg.p + n11, W.csize.p + CN, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     host_sync(g);
+    const uint64_t *tdeg = W.agg_htdeg.p;
+    const uint32_t members = *reinterpret_cast<const uint32_t *>(W.agg_htdeg.p + n11);
     W.mpre.ensure(size_t(members) + 1);
     launch_member_degrees(W.cmem.p, lv.deg, members, W.mpre.p, s);
     exclusive_scan_u64(W.mpre.p, W.mpre.p, members, W.mpre.p + members, W.scan64.p, s);
-    std::vector<uint2> chunks;
-    std::vector<uint64_t> toff(n11 + 1, 0);
-    std::vector<int> tlog(n11);
+    auto chunks_of = [](uint64_t d) { return (d + AGG_CHUNK - 1) / AGG_CHUNK; };
+    auto parts_of = [&](uint64_t d) {
+      return std::min<uint64_t>((std::min<uint64_t>(d, CN) + AGG_PART - 1) / AGG_PART, AGG_MAX_PARTS);
+    };
+    uint64_t nch = 0, nrun = 0, nm = 0, max_parts = 0;
+    for (size_t j = 0; j < n11; ++j) nch += chunks_of(tdeg[j]);
+    // chunks a block takes in a run: longer lists to merge from, as long as
+    // every SM's three blocks get a few runs
+    const uint64_t len = std::max<uint64_t>(1, std::min<uint64_t>(16, nch / (uint64_t(device_sms()) * 12)));
     for (size_t j = 0; j < n11; ++j) {
-      const uint64_t want = 2 * std::min<uint64_t>(tdeg[j], CN);
-      int lg = 1;
-      while ((uint64_t(1) << lg) < want) ++lg;
-      tlog[j] = lg;
-      toff[j + 1] = toff[j] + (uint64_t(1) << lg);
-      for (uint64_t k = 0; k * AGG_CHUNK < tdeg[j]; ++k) chunks.push_back(make_uint2(uint32_t(j), uint32_t(k)));
+      nrun += (chunks_of(tdeg[j]) + len - 1) / len;
+      nm += parts_of(tdeg[j]);
+      max_parts = std::max<uint64_t>(max_parts, parts_of(tdeg[j]));
     }
-    const uint64_t slots = toff[n11];
-    W.agg_chunk.ensure(chunks.size());
-    W.agg_toff.ensure(n11 + 1);
-    W.agg_tlog.ensure(n11);
-    W.agg_gk.ensure(slots);
-    W.agg_gv.ensure(slots);
-    LVG_CUDA(cudaMemcpyAsync(W.agg_chunk.p, chunks.data(), chunks.size() * sizeof(uint2), cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(W.agg_toff.p, toff.data(), (n11 + 1) * 8, cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemcpyAsync(W.agg_tlog.p, tlog.data(), n11 * sizeof(int), cudaMemcpyHostToDevice, s));
-    LVG_CUDA(cudaMemsetAsync(W.agg_gk.p, 0xFF, slots * 4, s));
-    LVG_CUDA(cudaMemsetAsync(W.agg_gv.p, 0, slots * 4, s));
-    AggArgs a;
-    a.off = lv.off; a.deg = lv.deg; a.key = lv.key; a.w = lv.w;
-    a.vcom = com; a.coff = W.csize.p; a.cmem = W.cmem.p;
+    size_t bytes = 0;
+    auto place = [&](size_t n, size_t elem) {
+      const size_t at = bytes;
+      bytes += (n * elem + 15) / 16 * 16;
+      return at;
+    };
+    const size_t a_run = place(nrun, 16), a_merge = place(nm, 8), a_poff = place(n11, 8), a_soff = place(n11, 8),
+                 a_loff = place(n11, 8), a_parts = place(n11, 4);
+    W.agg_hplan.ensure(bytes);  // (its last upload was waited for above)
+    W.agg_plan.ensure(bytes);
+    uint8_t *hp = W.agg_hplan.p;
+    auto *runs = reinterpret_cast<uint4 *>(hp + a_run);
+    auto *merge = reinterpret_cast<uint2 *>(hp + a_merge);
+    auto *poff = reinterpret_cast<uint64_t *>(hp + a_poff), *soff = reinterpret_cast<uint64_t *>(hp + a_soff);
+    auto *loff = reinterpret_cast<uint64_t *>(hp + a_loff);
+    auto *parts = reinterpret_cast<uint32_t *>(hp + a_parts);
+    uint64_t c = 0, m = 0, pairs = 0, seg = 0, lists = 0;
+    for (size_t j = 0; j < n11; ++j) {
+      const uint64_t n = chunks_of(tdeg[j]), R = parts_of(tdeg[j]);
+      for (uint64_t k = 0; k < n; k += len)
+        runs[c++] = make_uint4(uint32_t(j), uint32_t(k), uint32_t(std::min(len, n - k)), 0u);
+      for (uint64_t r = 0; r < R; ++r) merge[m++] = make_uint2(uint32_t(j), uint32_t(r));
+      poff[j] = pairs;
+      soff[j] = seg;
+      loff[j] = lists;
+      parts[j] = uint32_t(R);
+      lists += n;
+      pairs += n * AGG_CHUNK;
+      seg += n * (R + 1);
+    }
+    LVG_CUDA(cudaMemcpyAsync(W.agg_plan.p, hp, bytes, cudaMemcpyHostToDevice, s));
+    W.agg_pairs.ensure(pairs);
+    W.agg_seg.ensure(seg);
+    W.agg_lists.ensure(n11 + lists);
+    LVG_CUDA(cudaMemsetAsync(W.agg_lists.p, 0, n11 * sizeof(uint32_t), s));
     a.list = list;
     a.count = uint32_t(n11);
-    a.yoff = nl.off; a.ydeg = nl.deg; a.ykey = nl.key; a.yw = nl.w;
-    a.ctr = g->ctr.p; a.cn = uint32_t(CN);
-    a.gkeys = nullptr; a.gvals = nullptr; a.glog2 = 0;
-    AggChunks ch{W.agg_chunk.p, list, W.agg_toff.p, W.agg_tlog.p, W.mpre.p, W.agg_gk.p, W.agg_gv.p, uint32_t(n11)};
-    launch_aggregate_chunks(a, ch, chunks.size(), slots, s);
+    const uint8_t *dp = W.agg_plan.p;
+    const AggChunks ch{reinterpret_cast<const uint4 *>(dp + a_run), reinterpret_cast<const uint2 *>(dp + a_merge), list,
+                       reinterpret_cast<const uint32_t *>(dp + a_parts), reinterpret_cast<const uint64_t *>(dp + a_poff),
+                       reinterpret_cast<const uint64_t *>(dp + a_soff), reinterpret_cast<const uint64_t *>(dp + a_loff),
+                       W.mpre.p, W.agg_pairs.p, W.agg_seg.p, W.agg_lists.p, W.agg_lists.p + n11};
+    launch_aggregate_chunks(a, ch, nrun, nm, uint32_t(max_parts), s);
     g->stats.aggregate_launches += 2;
-    host_sync(g);  // the host vectors above are freed next
+  }
+  for (int i = 0; i < 4; ++i) {  // join
+    LVG_CUDA(cudaEventRecord(g->join_ev[i], g->aux[i]));
+    LVG_CUDA(cudaStreamWaitEvent(s, g->join_ev[i], 0));
   }
   if (g->profiling) {
     e1 = g->events.record(s);

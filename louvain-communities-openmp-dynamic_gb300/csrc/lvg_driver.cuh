@@ -70,12 +70,14 @@ struct Workspace {
   DBuf<uint8_t> ht_slg;
   DBuf<uint32_t> ht_skey, ht_scnt, ht_n;
   HubTabView ht_now;
-  // chunked aggregation of the largest communities
-  DBuf<uint64_t> mpre, agg_toff, agg_tdeg;
-  DBuf<uint2> agg_chunk;
-  DBuf<int> agg_tlog;
-  DBuf<uint32_t> agg_gk;
-  DBuf<float> agg_gv;
+  // chunked aggregation of the largest communities: the plan (one pinned block,
+  // uploaded in one copy), the chunks' pairs and their groups' bounds
+  DBuf<uint64_t> mpre, agg_tdeg;
+  DBuf<uint8_t> agg_plan;
+  HBuf<uint8_t> agg_hplan;
+  HBuf<uint64_t> agg_htdeg;
+  DBuf<uint2> agg_pairs;
+  DBuf<uint32_t> agg_seg, agg_lists;
 
   void allocate(size_t S_, size_t X_, cudaStream_t st) {
     S = S_;

@@ -393,25 +393,29 @@ struct AggArgs {
   float *yw;
   uint32_t cn;           // number of communities (distinct keys per row <= cn)
   Counters *ctr;
-  uint32_t *gkeys;
-  float *gvals;
-  int glog2;
+  bool unit, whole;      // Level::unit; Level::whole and a total weight below 2^31
 };
 
 // Aggregation of the communities above total degree 8192 in AGG_CHUNK-edge
-// chunks (lvg_aggregate.cu): community slot j is community comm[j]; its
-// global table holds 2^tlog[j] slots at toff[j] (toff[n] = all slots); mpre
-// is the prefix of member degrees in member-list order.
-constexpr uint32_t AGG_CHUNK = 16384;
+// chunks (lvg_aggregate.cu): community slot j is community comm[j]; mpre is the
+// prefix of member degrees in member-list order. Blocks take runs of its
+// chunks and write lists of (community, weight) pairs: nlist[j] of them (at
+// most a list per chunk), list i from chunk f = list_at[list_off[j] + i] on,
+// its pairs at part_off[j] + f * AGG_CHUNK. Its neighbour communities fall into
+// parts[j] hash partitions (at most AGG_MAX_PARTS), by which a list is grouped:
+// the groups' bounds are at seg_off[j] + i * (parts[j] + 1).
+constexpr uint32_t AGG_CHUNK = 4096;
+constexpr uint32_t AGG_PART = 8192;  // distinct communities a partition is meant to hold
+constexpr uint32_t AGG_MAX_PARTS = 20480;
 struct AggChunks {
-  const uint2 *chunk;     // [chunks] (community slot, chunk index)
-  const uint32_t *comm;   // [n]
-  const uint64_t *toff;   // [n+1]
-  const int *tlog;        // [n]
-  const uint64_t *mpre;   // [members+1]
-  uint32_t *gkeys;        // [toff[n]] EMPTY-initialised
-  float *gvals;           // [toff[n]] zero-initialised
-  uint32_t n;
+  const uint4 *run;          // [runs] (community slot, first chunk, chunks, -)
+  const uint2 *merge;        // [merges] (community slot, partition)
+  const uint32_t *comm;      // [n]
+  const uint32_t *parts;
+  const uint64_t *part_off, *seg_off, *list_off;
+  const uint64_t *mpre;      // [members+1]
+  uint2 *pairs;
+  uint32_t *seg, *nlist, *list_at;  // nlist zeroed
 };
 
 // ---------------------------------------------------------------- scans (lvg_scan.cu)
@@ -551,8 +555,10 @@ void launch_aggregate_bin(int b, const AggArgs &a, cudaStream_t s);
 void launch_comm_tdeg(const uint32_t *list, size_t n, const uint64_t *yoff, uint64_t *out, cudaStream_t s);
 // dst[i] = deg[cmem[i]] for the member list.
 void launch_member_degrees(const uint32_t *cmem, const uint32_t *deg, size_t n, uint64_t *dst, cudaStream_t s);
-// The chunked communities: chunk merges into the global tables, then the rows.
-void launch_aggregate_chunks(const AggArgs &a, const AggChunks &ch, size_t chunks, uint64_t slots, cudaStream_t s);
+// The chunked communities: the chunks' pairs, then the partitions' sums into
+// the rows (max_parts: the largest parts[j]).
+void launch_aggregate_chunks(const AggArgs &a, const AggChunks &ch, size_t runs, size_t merges, uint32_t max_parts,
+                             cudaStream_t s);
 
 // Record a failure message for lvg_last_error() and return `code` (for entry
 // points outside the driver and the C-ABI files).
