@@ -606,8 +606,6 @@ int lvg_community_weights(lvg_graph *g, const uint32_t *membership, const double
   return lvg::guarded([&] {
     LVG_CUDA(cudaSetDevice(g->device));
     const size_t S = g->base.span;
-    for (size_t u = 0; u < S; ++u)
-      if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;
     cudaStream_t s = g->stream;
@@ -629,8 +627,6 @@ int lvg_modularity(lvg_graph *g, const uint32_t *membership, double M, double R,
   return lvg::guarded([&] {
     LVG_CUDA(cudaSetDevice(g->device));
     const size_t S = g->base.span;
-    for (size_t u = 0; u < S; ++u)
-      if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;
     cudaStream_t s = g->stream;
@@ -639,7 +635,7 @@ int lvg_modularity(lvg_graph *g, const uint32_t *membership, double M, double R,
     LVG_CUDA(cudaMemcpyAsync(W.com_next.p, membership, S * 4, cudaMemcpyHostToDevice, s));
     lvg::launch_modularity(g->base, W.com_next.p, W.ctot64.p, g->ctr.p, s);
     lvg::launch_sq_sum(W.ctot64.p, S, g->ctr.p, s);
-    lvg::read_counters(g);
+    lvg::read_counters(g);  // (raises LVG_EINVAL for an id that is no vertex)
     const double intra = g->hctr.p->fp64[1], sq = g->hctr.p->fp64[2];
     *out = intra / (2 * M) - R * sq / (4 * M * M);
     return LVG_OK;
@@ -688,8 +684,6 @@ int lvg_aggregate(lvg_graph *g, const uint32_t *membership, uint32_t *renumbered
   return lvg::guarded([&] {
     LVG_CUDA(cudaSetDevice(g->device));
     const size_t S = g->base.span, X = g->base.edges;
-    for (size_t u = 0; u < S; ++u)
-      if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
     if (X && (!keys || !weights)) throw lvg::Error(LVG_EINVAL, "null keys/weights");
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;

@@ -49,7 +49,7 @@ void read_counters(lvg_graph *g) {
   if (g->hctr.p->err) {
     unsigned e = g->hctr.p->err;
     LVG_CUDA(cudaMemsetAsync(&g->ctr.p->err, 0, sizeof(unsigned), g->stream));
-    if (e & ERR_BAD_ID) throw Error(LVG_EINVAL, "prior membership id >= span (err=" + std::to_string(e) + ")");
+    if (e & ERR_BAD_ID) throw Error(LVG_EINVAL, "membership id >= span (err=" + std::to_string(e) + ")");
     if (e & ERR_WORKLIST) throw Error(LVG_ECUDA, "worklist append outside its degree bin (stale degree bins)");
     if (e & ERR_BARRIER) throw Error(LVG_ETIMEOUT, "a grid barrier of the local-moving phase was given up");
     throw Error(LVG_ETIMEOUT, "device hash table overflow guard tripped (err=" + std::to_string(e) + ")");

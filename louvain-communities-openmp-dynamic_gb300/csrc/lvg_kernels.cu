@@ -1,6 +1,7 @@
 // lvg_kernels.cu — initialisation, batch-update, marking, renumbering,
 // community-CSR and modularity kernels.
 #include <algorithm>
+#include <type_traits>
 
 #include "lvg_internal.cuh"
 
@@ -42,29 +43,90 @@ __global__ void degrees_kernel(const uint64_t *off, uint32_t *deg, size_t n) {
   GRID_STRIDE(u, n) deg[u] = uint32_t(off[u + 1] - off[u]);
 }
 
-// louvainVertexWeightsOmpW (inc/louvain.hxx:210) + louvainInitializeOmpW
-// (:285) for level 0: one warp per vertex (lane-strided rows).
-__global__ void init_static_kernel(const uint64_t *off, const uint32_t *deg, const float *w, const uint8_t *ex,
-                                   size_t n, const uint32_t *gid, const uint32_t *gbase, uint32_t *ucom, tot_t *utot,
-                                   tot_t *ctot) {
-  const size_t warps = size_t(gridDim.x) * blockDim.x / 32;
-  const int lane = threadIdx.x & 31;
-  for (size_t u = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; u < n; u += warps) {
-    const bool has = !ex || ex[u];
-    double s = 0.0;  // FP64, as the reference's vector<W> (exact for integer weights)
-    if (has) {
-      const uint64_t o = off[u];
-      const uint32_t d = deg[u];
-      for (uint32_t j = lane; j < d; j += 32) s += double(w[o + j]);
+// The FP64 sum of a row's weights by eight lanes (sl) of a warp: the value of
+// 32 lanes striding over the row and an xor tree over them (the order of the
+// sum is part of its value), each lane here standing for four of those, which
+// takes 6 FP64 additions a lane beside the row's own instead of 5 on 32 lanes.
+__device__ __forceinline__ double row_sum8(const float *w, uint32_t d, uint32_t sl) {
+  double acc[4] = {0.0, 0.0, 0.0, 0.0};
+  for (uint32_t j = sl; j < d; j += 32) {
+    float x[4];
 #pragma unroll
-      for (int k = 16; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+    for (int q = 0; q < 4; ++q) x[q] = j + 8 * q < d ? __ldcs(w + j + 8 * q) : 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) acc[q] += double(x[q]);
+  }
+  double s = (acc[0] + acc[2]) + (acc[1] + acc[3]);
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffu << (threadIdx.x & 24u), s, o);
+  return s;
+}
+
+// Calls out(u, sum) once for every vertex u with the FP64 sum of its row's
+// weights (0 where absent): eight lanes per vertex; rows above ROW_LONG
+// entries are put aside and taken a warp each.
+constexpr uint32_t ROW_LONG = 512;
+constexpr int ROW_B = 256;
+template <class Out>
+__device__ __forceinline__ void row_sums(const uint64_t *off, const uint32_t *deg, const float *w, const uint8_t *ex,
+                                         size_t n, Out out) {
+  __shared__ uint32_t s_long[ROW_B / 8];
+  __shared__ uint32_t s_n;
+  const uint32_t sl = threadIdx.x & 7u;
+  for (size_t base = size_t(blockIdx.x) * (ROW_B / 8); base < n; base += size_t(gridDim.x) * (ROW_B / 8)) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const size_t u = base + threadIdx.x / 8;
+    if (u < n) {
+      const uint32_t d = !ex || ex[u] ? deg[u] : 0u;
+      if (d > ROW_LONG) {
+        if (sl == 0) s_long[atomicAdd(&s_n, 1u)] = uint32_t(u);
+      } else {
+        const double s = row_sum8(w + off[u], d, sl);
+        if (sl == 0) out(u, s);
+      }
     }
-    if (lane == 0) {
-      // an absent vertex starts in community 0 (of its own graph in a union)
-      ucom[u] = has ? uint32_t(u) : (gid ? gbase[gid[u]] : 0u);
-      utot[u] = s;
-      ctot[u] = s;
+    __syncthreads();
+    for (uint32_t i = threadIdx.x / 32; i < s_n; i += ROW_B / 32) {
+      const uint32_t v = s_long[i], d = deg[v];
+      const float *row = w + off[v];
+      double s = 0.0;
+      for (uint32_t j = threadIdx.x & 31u; j < d; j += 32 * 8) {  // eight loads in flight
+        float x[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x[q] = j + 32 * q < d ? __ldcs(row + j + 32 * q) : 0.f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) s += double(x[q]);
+      }
+      s = warp_sum_d(s);
+      if ((threadIdx.x & 31u) == 0) out(v, s);
     }
+    __syncthreads();
+  }
+}
+
+// louvainVertexWeightsOmpW (inc/louvain.hxx:210) + louvainInitializeOmpW
+// (:285) for level 0. An absent vertex starts in community 0 (of its own graph
+// in a union).
+__device__ __forceinline__ void init_vertex(size_t u, bool has, double s, const uint32_t *gid, const uint32_t *gbase,
+                                            uint32_t *ucom, tot_t *utot, tot_t *ctot) {
+  ucom[u] = has ? uint32_t(u) : (gid ? gbase[gid[u]] : 0u);
+  utot[u] = s;
+  ctot[u] = s;
+}
+__global__ void __launch_bounds__(ROW_B) init_static_kernel(const uint64_t *off, const uint32_t *deg, const float *w,
+                                                            const uint8_t *ex, size_t n, const uint32_t *gid,
+                                                            const uint32_t *gbase, uint32_t *ucom, tot_t *utot,
+                                                            tot_t *ctot) {
+  row_sums(off, deg, w, ex, n, [&](size_t u, double s) { init_vertex(u, !ex || ex[u], s, gid, gbase, ucom, utot, ctot); });
+}
+// A unit-weight level: a vertex's weight is its degree. (R-MAT scale 23: 4.9
+// ms with a warp per row, 0.04 ms without reading the rows.)
+__global__ void init_unit_kernel(const uint32_t *deg, const uint8_t *ex, size_t n, const uint32_t *gid,
+                                 const uint32_t *gbase, uint32_t *ucom, tot_t *utot, tot_t *ctot) {
+  GRID_STRIDE(u, n) {
+    const bool has = !ex || ex[u];
+    init_vertex(u, has, has ? double(deg[u]) : 0.0, gid, gbase, ucom, utot, ctot);
   }
 }
 
@@ -90,20 +152,11 @@ __global__ void total_weight_kernel(const float *w, size_t m, double *dst) {
   block_add_double(s, dst);
 }
 
-// louvainVertexWeightsOmpW in FP64: a warp per row.
-__global__ void vertex_weights_f64_kernel(const uint64_t *off, const uint32_t *deg, const float *w, const uint8_t *ex,
-                                          size_t n, double *vtot) {
-  const size_t warps = size_t(gridDim.x) * blockDim.x / 32;
-  const int lane = threadIdx.x & 31;
-  for (size_t u = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; u < n; u += warps) {
-    double s = 0;
-    if (!ex || ex[u]) {
-      const uint64_t o = off[u];
-      for (uint32_t j = lane; j < deg[u]; j += 32) s += double(w[o + j]);
-      s = warp_sum_d(s);
-    }
-    if (lane == 0) vtot[u] = s;
-  }
+// louvainVertexWeightsOmpW in FP64.
+__global__ void __launch_bounds__(ROW_B) vertex_weights_f64_kernel(const uint64_t *off, const uint32_t *deg,
+                                                                   const float *w, const uint8_t *ex, size_t n,
+                                                                   double *vtot) {
+  row_sums(off, deg, w, ex, n, [&](size_t u, double s) { vtot[u] = s; });
 }
 
 // louvainCommunityWeightsOmpW in FP64: ctot[q[u]] += vtot[u].
@@ -940,29 +993,112 @@ __global__ void count_flags_kernel(const uint8_t *f, size_t n, unsigned long lon
   if ((threadIdx.x & 31) == 0 && c) atomicAdd(dst, c);
 }
 
-// modularityBy (inc/properties.hxx:178-191) in FP64: intra-community weight
-// and per-community totals. One warp per vertex.
-__global__ void modularity_kernel(const uint64_t *off, const uint32_t *deg, const uint32_t *key, const float *w,
-                                  const uint8_t *ex, size_t n, const uint32_t *memb, double *ctot64,
-                                  double *intra) {
-  const size_t warps = size_t(gridDim.x) * blockDim.x / 32;
-  const int lane = threadIdx.x & 31;
-  double in = 0;
-  for (size_t u = (size_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32; u < n; u += warps) {
-    if (ex && !ex[u]) continue;
-    const uint32_t c = memb[u];
-    const uint64_t o = off[u];
-    const uint32_t d = deg[u];
-    double tot = 0;
-    for (uint32_t j = lane; j < d; j += 32) {
-      const double x = w[o + j];
-      tot += x;
-      if (memb[key[o + j]] == c) in += x;
+// modularityBy (inc/properties.hxx:178-191) in FP64: the weight inside the
+// communities and the communities' totals, eight lanes per vertex; rows above
+// MOD_LONG entries are put aside and taken in pieces of 128 entries, a warp
+// each. On a unit-weight level nothing but the neighbour ids is read, and the
+// counts are integers: FP64 additions issue slowly (a warp per row with its
+// FP64 reductions took 4.66 ms on an R-MAT scale-22 graph, this 0.66: bound by the
+// gathers of the neighbours' communities, a 32-byte L2 sector each). The 32
+// vertices of a warp's round whose communities are equal add their weights
+// first (a large community would take an atomic per member on one address).
+// Ids that are no vertex are flagged (ERR_BAD_ID) and left out.
+constexpr uint32_t MOD_LONG = 128;
+constexpr int MOD_B = 256;
+template <bool UNIT>
+__global__ void __launch_bounds__(MOD_B) modularity_kernel(const uint64_t *off, const uint32_t *deg, const uint32_t *key,
+                                                           const float *w, const uint8_t *ex, size_t n,
+                                                           const uint32_t *memb, double *ctot64, double *intra,
+                                                           unsigned int *err) {
+  using A = typename std::conditional<UNIT, unsigned long long, double>::type;
+  __shared__ uint32_t s_long[MOD_B];
+  __shared__ double s_tot[MOD_B];  // a vertex's weight
+  __shared__ uint32_t s_n;
+  const uint32_t sl = threadIdx.x & 7u, lane = threadIdx.x & 31u;
+  A in = 0;
+  bool bad = false;
+  // entries [j, end) by `step` lanes: those inside community c, and the weight of all
+  auto run = [&](uint64_t o, uint32_t j, uint32_t end, uint32_t step, uint32_t c, double &tot) {
+    for (; j < end; j += 4 * step) {
+      uint32_t m[4];
+      float x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const bool is = j + q * step < end;
+        m[q] = is ? __ldcs(key + o + j + q * step) : EMPTY;
+        x[q] = UNIT ? 1.f : (is ? __ldcs(w + o + j + q * step) : 0.f);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) m[q] = m[q] != EMPTY ? memb[m[q]] : EMPTY;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if constexpr (UNIT) {
+          in += m[q] == c;
+        } else {
+          tot += double(x[q]);
+          if (m[q] == c) in += double(x[q]);
+        }
+      }
     }
-    tot = warp_sum_d(tot);
-    if (lane == 0 && tot != 0.0) atomicAdd(&ctot64[c], tot);
+  };
+  // a block takes 256 vertices at a time: their rows, then their totals
+  for (size_t base = size_t(blockIdx.x) * MOD_B; base < n; base += size_t(gridDim.x) * MOD_B) {
+    if (threadIdx.x == 0) s_n = 0;
+    if constexpr (!UNIT) s_tot[threadIdx.x] = 0.0;
+    __syncthreads();
+    for (uint32_t r = threadIdx.x / 8; r < MOD_B && base + r < n; r += MOD_B / 8) {
+      const size_t u = base + r;
+      const uint32_t d = !ex || ex[u] ? deg[u] : 0u, c = memb[u];
+      if (d > MOD_LONG) {
+        if (sl == 0) s_long[atomicAdd(&s_n, 1u)] = r;
+        continue;
+      }
+      double tot = 0.0;
+      run(off[u], sl, d, 8, c, tot);
+      if constexpr (!UNIT) {
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffu << (threadIdx.x & 24u), tot, o);
+        if (sl == 0) s_tot[r] = tot;
+      }
+    }
+    __syncthreads();
+    const uint32_t nl = s_n;
+    constexpr uint32_t W = MOD_B / 32;
+    for (uint32_t i = 0; i < nl; ++i) {
+      const size_t u = base + s_long[i];
+      const uint64_t o = off[u];
+      const uint32_t d = deg[u], c = memb[u];
+      double tot = 0.0;
+      for (uint32_t p = (threadIdx.x / 32 + W - i % W) % W; p * 128u < d; p += W)
+        run(o, p * 128u + lane, min(d, (p + 1) * 128u), 32, c, tot);
+      if constexpr (!UNIT) {
+        tot = warp_sum_d(tot);
+        if (lane == 0 && tot != 0.0) atomicAdd(&s_tot[s_long[i]], tot);
+      }
+    }
+    __syncthreads();
+    {
+      const size_t u = base + threadIdx.x;
+      uint32_t c = EMPTY;
+      double x = 0.0;
+      if (u < n) {
+        c = memb[u];
+        if (c >= n) bad = true;
+        else if (!ex || ex[u]) x = UNIT ? double(deg[u]) : s_tot[threadIdx.x];
+        if (x == 0.0) c = EMPTY;
+      }
+      group_add(ctot64, c, x, int(lane));
+    }
+    __syncthreads();
   }
-  block_add_double(in, intra);
+  if (bad) atomicOr(err, ERR_BAD_ID);
+  if constexpr (UNIT) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) in += __shfl_xor_sync(0xffffffffu, in, o);
+    if (lane == 0 && in) atomicAdd(intra, double(in));  // (exact below 2^53)
+  } else {
+    block_add_double(in, intra);
+  }
 }
 
 __global__ void sq_sum_kernel(const double *x, size_t n, double *dst) {
@@ -1033,14 +1169,17 @@ void launch_fill_f32(float *p, size_t n, float v, cudaStream_t s) {
 
 void launch_init_static(const Level &g, uint32_t *ucom, tot_t *utot, tot_t *ctot, cudaStream_t s) {
   if (!g.span) return;
-  init_static_kernel<<<grid_for(g.span * 32, 256), 256, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, g.gid, g.gbase,
-                                                                 ucom, utot, ctot);
+  if (g.unit)
+    init_unit_kernel<<<grid_for(g.span, 256), 256, 0, s>>>(g.deg, g.ex, g.span, g.gid, g.gbase, ucom, utot, ctot);
+  else
+    init_static_kernel<<<grid_for(g.span * 8, ROW_B), ROW_B, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, g.gid, g.gbase,
+                                                                     ucom, utot, ctot);
   LVG_CHECK_LAUNCH();
 }
 
 void launch_vertex_weights_f64(const Level &g, double *vtot, cudaStream_t s) {
   if (!g.span) return;
-  vertex_weights_f64_kernel<<<grid_for(g.span * 32, 256), 256, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, vtot);
+  vertex_weights_f64_kernel<<<grid_for(g.span * 8, ROW_B), ROW_B, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, vtot);
   LVG_CHECK_LAUNCH();
 }
 
@@ -1285,8 +1424,13 @@ void launch_modularity(const Level &g, const uint32_t *memb, double *ctot64, Cou
   LVG_CUDA(cudaMemsetAsync(&ctr->fp64[1], 0, sizeof(double), s));
   LVG_CUDA(cudaMemsetAsync(ctot64, 0, g.span * sizeof(double), s));
   if (!g.span) return;
-  modularity_kernel<<<grid_for(g.span * 32, 256), 256, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, ctot64,
-                                                               &ctr->fp64[1]);
+  const int grid = grid_for(g.span, MOD_B);
+  if (g.unit)
+    modularity_kernel<true><<<grid, MOD_B, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, ctot64, &ctr->fp64[1],
+                                                   &ctr->err);
+  else
+    modularity_kernel<false><<<grid, MOD_B, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, ctot64,
+                                                    &ctr->fp64[1], &ctr->err);
   LVG_CHECK_LAUNCH();
 }
 
