@@ -12,16 +12,17 @@ namespace {
 // each chunk is copied off the device while the previous one is spread into
 // the (pageable) host arrays by a few threads.
 template <class Dst>
-void copy_out_slices(cudaStream_t s, const void *dev, size_t elem, const std::vector<uint64_t> &vb, Dst dst) {
+void copy_out_slices(cudaStream_t s, UnionStage &st, const void *dev, size_t elem, const std::vector<uint64_t> &vb,
+                     Dst dst) {
   const size_t n = vb.back(), G = vb.size() - 1;
   if (!n) return;
-  const size_t per = std::max<size_t>(1, (size_t(64) << 20) / elem);  // elements per chunk
-  HBuf<uint8_t> stage[2];
-  stage[0].ensure(per * elem);
-  stage[1].ensure(per * elem);
-  cudaEvent_t ev[2];
-  LVG_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
-  LVG_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
+  const size_t per = std::max<size_t>(1, std::min(n, (size_t(16) << 20) / elem));  // elements per chunk
+  HBuf<uint8_t> *stage = st.buf;
+  cudaEvent_t *ev = st.ev;
+  for (int i = 0; i < 2; ++i) {
+    stage[i].ensure(per * elem);
+    if (!ev[i]) LVG_CUDA(cudaEventCreateWithFlags(&ev[i], cudaEventDisableTiming));
+  }
   const size_t chunks = (n + per - 1) / per;
   auto issue = [&](size_t k) {
     const size_t b = k * per, m = std::min(per, n - b);
@@ -53,8 +54,6 @@ void copy_out_slices(cudaStream_t s, const void *dev, size_t elem, const std::ve
     spread(b, std::min(e, b + step));
     for (auto &x : th) x.join();
   }
-  cudaEventDestroy(ev[0]);
-  cudaEventDestroy(ev[1]);
 }
 
 }  // namespace
@@ -468,9 +467,9 @@ int lvg_static_union(lvg_graph *u, const lvg_options *o, lvg_result *results) {
       if (!r->communityWeight) { r->communityWeight = (double *)std::malloc(sp * 8 + 1); r->owned |= 4; }
       if (!r->membership || !r->vertexWeight || !r->communityWeight) throw std::bad_alloc();
     }
-    copy_out_slices(s, U.q.p, 4, U.vb, [&](size_t i) -> void * { return results[i].membership; });
-    copy_out_slices(s, W.utot.p, sizeof(tot_t), U.vb, [&](size_t i) -> void * { return results[i].vertexWeight; });
-    copy_out_slices(s, U.ct.p, sizeof(tot_t), U.vb, [&](size_t i) -> void * { return results[i].communityWeight; });
+    copy_out_slices(s, U.stage, U.q.p, 4, U.vb, [&](size_t i) -> void * { return results[i].membership; });
+    copy_out_slices(s, U.stage, W.utot.p, sizeof(tot_t), U.vb, [&](size_t i) -> void * { return results[i].vertexWeight; });
+    copy_out_slices(s, U.stage, U.ct.p, sizeof(tot_t), U.vb, [&](size_t i) -> void * { return results[i].communityWeight; });
     for (size_t i = 0; i < U.n; ++i) {
       lvg_result *r = &results[i];
       const size_t sp = U.vb[i + 1] - U.vb[i];
@@ -606,6 +605,8 @@ int lvg_community_weights(lvg_graph *g, const uint32_t *membership, const double
   return lvg::guarded([&] {
     LVG_CUDA(cudaSetDevice(g->device));
     const size_t S = g->base.span;
+    for (size_t u = 0; u < S; ++u)
+      if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;
     cudaStream_t s = g->stream;
@@ -684,6 +685,8 @@ int lvg_aggregate(lvg_graph *g, const uint32_t *membership, uint32_t *renumbered
   return lvg::guarded([&] {
     LVG_CUDA(cudaSetDevice(g->device));
     const size_t S = g->base.span, X = g->base.edges;
+    for (size_t u = 0; u < S; ++u)
+      if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
     if (X && (!keys || !weights)) throw lvg::Error(LVG_EINVAL, "null keys/weights");
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;
