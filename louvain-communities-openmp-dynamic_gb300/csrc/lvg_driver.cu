@@ -304,11 +304,12 @@ void ensure_hub_index(lvg_graph *g) {
 // Largest table of a hub: a hub with more than a quarter of this many
 // neighbour communities keeps scanning its edges.
 constexpr int HT_MAX_LOG = 16;
+static_assert((4u * HT_MAX_KEYS) == 1u << HT_MAX_LOG, "");
 
 // Hub tables T of membership q on the current graph version: every hub's
-// neighbours counted per community into a scratch table (at least twice its
-// degree in slots), the distinct communities counted, then each hub's table
-// laid out with four times that many slots (at least 64) and filled.
+// neighbours counted per community into a scratch table (twice its degree in
+// slots, at most 2^HT_MAX_LOG), the distinct communities counted, then each
+// hub's table laid out with four times that many slots (at least 64) and filled.
 void build_hub_tables(lvg_graph *g, const uint32_t *q, HubTables &T) {
   ensure_hub_index(g);
   Workspace &W = *g->ws;
@@ -321,7 +322,7 @@ void build_hub_tables(lvg_graph *g, const uint32_t *q, HubTables &T) {
     std::vector<uint8_t> slg(H);
     for (size_t h = 0; h < H; ++h) {
       int l = 1;
-      while ((uint64_t(1) << l) < 2ull * g->hub_deg_h[h]) ++l;
+      while (l < HT_MAX_LOG && (uint64_t(1) << l) < 2ull * g->hub_deg_h[h]) ++l;
       slg[h] = uint8_t(l);
       soff[h + 1] = soff[h] + (uint64_t(1) << l);
     }
@@ -335,8 +336,8 @@ void build_hub_tables(lvg_graph *g, const uint32_t *q, HubTables &T) {
     LVG_CUDA(cudaMemcpyAsync(W.ht_slg.p, slg.data(), H, cudaMemcpyHostToDevice, s));
     LVG_CUDA(cudaMemsetAsync(W.ht_skey.p, 0xFF, stotal * 4, s));
     LVG_CUDA(cudaMemsetAsync(W.ht_scnt.p, 0, stotal * 4, s));
-    launch_ht_scratch(g->base, q, g->hub_slot.p, W.ht_soff.p, W.ht_slg.p, W.ht_skey.p, W.ht_scnt.p, g->ctr.p, s);
-    launch_ht_count(H, W.ht_soff.p, W.ht_slg.p, W.ht_skey.p, W.ht_n.p, s);
+    LVG_CUDA(cudaMemsetAsync(W.ht_n.p, 0, H * 4, s));
+    launch_ht_scratch(g->base, q, g->hub_slot.p, W.ht_soff.p, W.ht_slg.p, W.ht_skey.p, W.ht_scnt.p, W.ht_n.p, s);
     std::vector<uint32_t> n(H);
     LVG_CUDA(cudaMemcpyAsync(n.data(), W.ht_n.p, H * 4, cudaMemcpyDeviceToHost, s));
     host_sync(g);

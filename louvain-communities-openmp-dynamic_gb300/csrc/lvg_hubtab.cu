@@ -42,6 +42,30 @@ __device__ __forceinline__ bool cnt_add(uint32_t *keys, uint32_t *cnts, int lg, 
   return false;
 }
 
+// cnt_add() into a scratch table, counting the keys that are new to it in *n;
+// a table with more than HT_MAX_KEYS of them is of no use and left as it is.
+__device__ __forceinline__ void scratch_add(uint32_t *keys, uint32_t *cnts, int lg, uint32_t c, uint32_t k,
+                                            uint32_t *n) {
+  const uint32_t mask = (1u << lg) - 1u;
+  uint32_t s = hash_hi(c, lg);
+  for (uint32_t p = 0; p <= mask; ++p) {
+    if ((p & 7u) == 7u && ld_relaxed(n) > HT_MAX_KEYS) return;
+    uint32_t x = ld_relaxed(keys + s);
+    if (x == EMPTY) {
+      x = atomicCAS(keys + s, EMPTY, c);
+      if (x == EMPTY) {
+        x = c;
+        atomicAdd(n, 1u);
+      }
+    }
+    if (x == c) {
+      atomicAdd(cnts + s, k);
+      return;
+    }
+    s = (s + 1u) & mask;
+  }
+}
+
 __global__ void ht_slots_kernel(const uint32_t *hubs, size_t n, uint32_t *slot) {
   GRID_STRIDE(i, n) slot[hubs[i]] = uint32_t(i);
 }
@@ -49,17 +73,18 @@ __global__ void ht_slots_kernel(const uint32_t *hubs, size_t n, uint32_t *slot) 
 // Build step 1: a block per chunk of a hub's edges (the hub plan's chunks, all
 // colour classes). The chunk's neighbours' communities are counted in shared
 // memory first (a hub's neighbours fall into few communities), then added to
-// the hub's scratch table in HBM, which has at least twice the hub's degree in
-// slots and so always has room. A key that finds no slot within HTB_PROBES
-// shared probes goes straight to the scratch table.
+// the hub's scratch table in HBM (twice the hub's degree in slots, at most four
+// times HT_MAX_KEYS: a hub of more communities gets no table). A key that
+// finds no slot within HTB_PROBES shared probes goes straight to the scratch
+// table. The distinct communities are counted on the way (a pass over scratch
+// tables of any size for it, a block per hub, took 1.9 ms on R-MAT scale 24).
 __global__ void __launch_bounds__(HTB_B) ht_scratch_kernel(const uint64_t *off, const uint32_t *key, const uint4 *chunk,
                                                           size_t nchunks, const uint32_t *q, const uint32_t *slot,
                                                           const uint64_t *soff, const uint8_t *slg, uint32_t *skey,
-                                                          uint32_t *scnt, Counters *ctr) {
+                                                          uint32_t *scnt, uint32_t *distinct) {
   constexpr uint32_t CS = 1u << HTB_LOG;
   __shared__ uint32_t tk[CS];
   __shared__ uint32_t tc[CS];
-  bool bad = false;
   for (size_t ci = blockIdx.x; ci < nchunks; ci += gridDim.x) {
     const uint4 ch = chunk[ci];
     const uint32_t u = ch.w;
@@ -89,47 +114,30 @@ __global__ void __launch_bounds__(HTB_B) ht_scratch_kernel(const uint64_t *off, 
         }
         s = (s + 1u) & (CS - 1u);
       }
-      if (!done) bad |= !cnt_add(gk, gc, glg, c, 1u);
+      if (!done) scratch_add(gk, gc, glg, c, 1u, distinct + h);
     }
     __syncthreads();
     for (uint32_t s = threadIdx.x; s < CS; s += HTB_B)
-      if (tk[s] != EMPTY) bad |= !cnt_add(gk, gc, glg, tk[s], tc[s]);
-    __syncthreads();
-  }
-  if (bad) atomicOr(&ctr->err, ERR_TABLE_FULL);
-}
-
-// Build step 2: distinct communities of each hub (a block per hub).
-__global__ void ht_count_kernel(size_t hubs, const uint64_t *soff, const uint8_t *slg, const uint32_t *skey,
-                                uint32_t *n) {
-  __shared__ uint32_t total;
-  for (size_t h = blockIdx.x; h < hubs; h += gridDim.x) {
-    if (threadIdx.x == 0) total = 0;
-    __syncthreads();
-    const uint64_t o = soff[h];
-    const uint32_t cap = 1u << slg[h];
-    uint32_t c = 0;
-    for (uint32_t s = threadIdx.x; s < cap; s += blockDim.x) c += skey[o + s] != EMPTY;
-#pragma unroll
-    for (int x = 16; x > 0; x >>= 1) c += __shfl_xor_sync(0xffffffffu, c, x);
-    if ((threadIdx.x & 31) == 0 && c) atomicAdd(&total, c);
-    __syncthreads();
-    if (threadIdx.x == 0) n[h] = total;
+      if (tk[s] != EMPTY) scratch_add(gk, gc, glg, tk[s], tc[s], distinct + h);
     __syncthreads();
   }
 }
 
-// Build step 3: each hub's scratch entries into its table (a block per hub;
-// the table has at least four times the entries in slots). Hubs marked bad
-// (too many communities for the largest table) are skipped.
+// Build step 2: the scratch entries into the hubs' tables (at least four times
+// the entries in slots), HTF_SLOTS scratch slots a block. Hubs marked bad (too
+// many communities for the largest table) are skipped. (R-MAT scale 24: 0.27
+// ms; a block per hub over scratch tables of any size took 2.4.)
+constexpr uint32_t HTF_SLOTS = 8192;
 __global__ void ht_fill_kernel(size_t hubs, const uint64_t *soff, const uint8_t *slg, const uint32_t *skey,
                                const uint32_t *scnt, HubTabView t) {
-  for (size_t h = blockIdx.x; h < hubs; h += gridDim.x) {
+  constexpr uint32_t PIECES = (4u * HT_MAX_KEYS + HTF_SLOTS - 1) / HTF_SLOTS;
+  for (size_t i = blockIdx.x; i < hubs * PIECES; i += gridDim.x) {
+    const size_t h = i / PIECES;
+    const uint32_t s0 = uint32_t(i % PIECES) * HTF_SLOTS, s1 = min(s0 + HTF_SLOTS, 1u << slg[h]);
     if (t.bad[h]) continue;
     const uint64_t o = soff[h];
-    const uint32_t cap = 1u << slg[h];
     uint32_t *k = t.key + t.off[h], *c = t.cnt + t.off[h];
-    for (uint32_t s = threadIdx.x; s < cap; s += blockDim.x) {
+    for (uint32_t s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
       const uint32_t x = skey[o + s];
       if (x != EMPTY && !cnt_add(k, c, t.lg[h], x, scnt[o + s])) ht_mark_bad(t, uint32_t(h));
     }
@@ -203,25 +211,18 @@ void launch_ht_slots(const uint32_t *hubs, size_t n, uint32_t *slot, cudaStream_
 }
 
 void launch_ht_scratch(const Level &lv, const uint32_t *q, const uint32_t *slot, const uint64_t *soff,
-                       const uint8_t *slg, uint32_t *skey, uint32_t *scnt, Counters *ctr, cudaStream_t s) {
+                       const uint8_t *slg, uint32_t *skey, uint32_t *scnt, uint32_t *distinct, cudaStream_t s) {
   const size_t n = lv.hub.chunks;
   if (!n) return;
   ht_scratch_kernel<<<blocks_for(n, size_t(1) << 16), HTB_B, 0, s>>>(lv.off, lv.key, lv.hub.chunk, n, q, slot, soff,
-                                                                    slg, skey, scnt, ctr);
-  LVG_CHECK_LAUNCH();
-}
-
-void launch_ht_count(size_t hubs, const uint64_t *soff, const uint8_t *slg, const uint32_t *skey, uint32_t *n,
-                     cudaStream_t s) {
-  if (!hubs) return;
-  ht_count_kernel<<<blocks_for(hubs, size_t(1) << 16), 256, 0, s>>>(hubs, soff, slg, skey, n);
+                                                                    slg, skey, scnt, distinct);
   LVG_CHECK_LAUNCH();
 }
 
 void launch_ht_fill(size_t hubs, const uint64_t *soff, const uint8_t *slg, const uint32_t *skey,
                     const uint32_t *scnt, const HubTabView &t, cudaStream_t s) {
   if (!hubs) return;
-  ht_fill_kernel<<<blocks_for(hubs, size_t(1) << 16), 256, 0, s>>>(hubs, soff, slg, skey, scnt, t);
+  ht_fill_kernel<<<blocks_for(hubs * 8, size_t(1) << 16), 256, 0, s>>>(hubs, soff, slg, skey, scnt, t);
   LVG_CHECK_LAUNCH();
 }
 

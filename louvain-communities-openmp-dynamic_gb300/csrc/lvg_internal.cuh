@@ -655,14 +655,14 @@ void launch_relayout_rows(const uint64_t *old_off, const uint32_t *deg, const ui
 void launch_move_hubs(bool sync, const MoveArgs &a, cudaStream_t s, cudaStream_t s_tab = nullptr);
 // Resident hub tables. Building (from membership q, for the hubs of plan P of
 // the uploaded level): each chunk of a hub's edges counts its communities in
-// shared memory and adds them to the hub's scratch table (2^slg[h] >= 2 deg
-// slots at soff[h]); ht_count gives each hub's distinct communities; ht_fill
-// copies each scratch table into the hub's table of the final layout.
+// shared memory and adds them to the hub's scratch table (2^slg[h] slots at
+// soff[h], zeroed, as is distinct), which leaves each hub's distinct
+// communities in distinct[h] (some number above HT_MAX_KEYS if there are more);
+// ht_fill copies each scratch table into the hub's table of the final layout.
+constexpr uint32_t HT_MAX_KEYS = 16384;
 void launch_ht_slots(const uint32_t *hubs, size_t n, uint32_t *slot, cudaStream_t s);
 void launch_ht_scratch(const Level &lv, const uint32_t *q, const uint32_t *slot, const uint64_t *soff,
-                       const uint8_t *slg, uint32_t *skey, uint32_t *scnt, Counters *ctr, cudaStream_t s);
-void launch_ht_count(size_t hubs, const uint64_t *soff, const uint8_t *slg, const uint32_t *skey, uint32_t *n,
-                     cudaStream_t s);
+                       const uint8_t *slg, uint32_t *skey, uint32_t *scnt, uint32_t *distinct, cudaStream_t s);
 void launch_ht_fill(size_t hubs, const uint64_t *soff, const uint8_t *slg, const uint32_t *skey,
                     const uint32_t *scnt, const HubTabView &t, cudaStream_t s);
 // Deterministic mode: the table updates of a colour class's decided moves
