@@ -716,9 +716,11 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   Workspace &W = *g->ws;
   cudaStream_t s = g->stream;
   if (g->profiling || !g->tuning.level_graphs || L <= 0) return false;
-  // resident hub tables are kept by the launch-by-launch kernels; a frontier
-  // run of one class starts from lists of its few marked vertices there
-  if (W.ht_now.key || listed) return false;
+  // asynchronous runs keep resident hub tables by the launch-by-launch kernels
+  // (deterministic ones here: the two phases of a 1e-4 |E| batch and its
+  // inverse on R-MAT scale 24 take 5.7 ms, by launches 12.5); a frontier run of
+  // one class starts from lists of its few marked vertices there
+  if ((W.ht_now.key && !(sync && lv.unit)) || listed) return false;
   const HubPlan &P = lv.hub;
   // Asynchronous runs from a prior on a level with hubs keep the launches: in
   // which order a class's degree bins see each other's moves differs there,
@@ -748,15 +750,17 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
       W.hub_done.ensure(P.hubs);
       LVG_CUDA(cudaMemsetAsync(W.hub_done.p, 0, W.hub_done.n * 4, s));
     }
-    W.hub_move.ensure(P.hubs);
+    W.hub_move.ensure(2 * P.hubs);
     a.hub_vertex = P.hub_vertex; a.hub_first = P.hub_first; a.hub_parts = P.hub_parts; a.seg_off = P.seg_off;
     a.chunk = P.chunk; a.chunk_part = P.chunk_part; a.merge = P.merge;
     a.chunk_cnt = W.chunk_cnt.p; a.part_key = W.part_key.p; a.part_val = reinterpret_cast<uint32_t *>(W.part_val.p);
     a.segs = W.hub_segs.p; a.hub_kd = W.hub_kd.p; a.hub_best = W.hub_best.p;
-    a.hub_done = W.hub_done.p; a.hub_move = W.hub_move.p;
+    a.hub_done = W.hub_done.p; a.hub_move = W.hub_move.p; a.hub_from = W.hub_move.p + P.hubs;
+    a.ht = W.ht_now;
     for (int k = 0; k <= lv.colors; ++k) {
       a.chunk_begin[k] = uint32_t(P.chunk_begin[k]);
       a.merge_begin[k] = uint32_t(P.merge_begin[k]);
+      a.hub_begin[k] = uint32_t(P.hub_begin[k]);
     }
   }
   if (uc) {

@@ -351,7 +351,8 @@ struct PhaseArgs {
   uint32_t *chunk_cnt, *part_key, *part_val, *segs;
   float *hub_kd;                // [span]
   unsigned long long *hub_best; // [hubs] zero between uses, as hub_done
-  uint32_t *hub_done, *hub_move;
+  uint32_t *hub_done, *hub_move, *hub_from;
+  HubTabView ht;      // resident hub tables (deterministic mode, unit weights); key nullptr without
   // graph unions (nullptr for one graph), as MoveArgs
   const uint32_t *gid;
   const float *gkr;
@@ -363,7 +364,8 @@ struct PhaseArgs {
   const double *gM;
   int itcap;          // iterations of a graph of the union
   uint32_t start[MAX_BUCKETS + 1];  // Level::bin_start
-  uint32_t chunk_begin[MAX_COLORS + 1], merge_begin[MAX_COLORS + 1];  // hub chunks and merge tasks of a class
+  // hub chunks, merge tasks and hubs of a class
+  uint32_t chunk_begin[MAX_COLORS + 1], merge_begin[MAX_COLORS + 1], hub_begin[MAX_COLORS + 1];
 };
 // Hub chunks (lvg_tuning::hub_chunk) up to this many edges fit the phase
 // kernel's table and leave room for the partitions' counters.

@@ -52,6 +52,7 @@ constexpr int PW = PB / 32;               // warps per block
 constexpr uint32_t LOG_BLOCK = 14;        // shared slots of a block's vertex (log2)
 constexpr uint32_t TABLE_WORDS = 2u << LOG_BLOCK;  // keys and values
 constexpr uint32_t LIST_CAP = 1920;       // listed vertices a block keeps in shared memory
+constexpr uint32_t TODO = 256;            // hub chunks a block looks through at a time
 constexpr uint32_t MERGE_FULL = 8192;     // partial entries of a hub that one block merges at once
 // One wait of the grid barrier gives up after this many polls (seconds; a
 // class takes microseconds), flags ERR_BARRIER and ends the kernel.
@@ -89,6 +90,7 @@ struct Shared {
   uint32_t nmv, nbig;          // moves of the class; those with long rows
   uint32_t hubmv;              // hubs moved by the block's merges
   uint32_t over, bad, stop;
+  uint32_t ntodo, todo[TODO];  // hub chunks that have work
   uint32_t any;                // some block moved a vertex before the last barrier that counts moves
   unsigned long long sum;      // the iteration's gain sum, or the union's graphs still moving
 };
@@ -268,8 +270,11 @@ __device__ __forceinline__ void phase_control(const PhaseArgs &a, uint32_t i, ui
   else atomicAdd(&a.ctl->gactive[slot], 1ull);
 }
 
-// Mark the neighbours row[0..m) of u (thread t of n), four in flight.
-__device__ __forceinline__ void mark_row(const PhaseArgs &a, uint32_t u, uint64_t o, uint32_t m, uint32_t t, uint32_t n) {
+// Mark the neighbours row[0..m) of u (thread t of n), four in flight; with
+// resident hub tables (tabs), u's move from community d to c into the tables
+// of those that are hubs.
+__device__ __forceinline__ void mark_row(const PhaseArgs &a, uint32_t u, uint64_t o, uint32_t m, uint32_t t, uint32_t n,
+                                         bool tabs = false, uint32_t d = 0, uint32_t c = 0) {
   for (uint32_t j = t; j < m; j += 4 * n) {
     uint32_t v[4];
 #pragma unroll
@@ -277,6 +282,13 @@ __device__ __forceinline__ void mark_row(const PhaseArgs &a, uint32_t u, uint64_
 #pragma unroll
     for (int k = 0; k < 4; ++k)
       if (v[k] != u) a.vaff[v[k]] = 1;
+    if (tabs) {
+      uint32_t h[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) h[k] = v[k] != u ? a.ht.slot[v[k]] : NO_HUB;
+      for (int k = 0; k < 4; ++k)
+        if (h[k] != NO_HUB) ht_move(a.ht, v[k], d, c, a.ctr);
+    }
   }
 }
 
@@ -423,15 +435,34 @@ __device__ __forceinline__ Sum<MODE> scan_row(const PhaseArgs &a, Shared &S, uin
   return kd;
 }
 
+// The group's best of its threads' moves (gain bg, community bc): the largest
+// gain (positive, so its bits order as the floats), then the lowest id.
+__device__ __forceinline__ void group_best(Shared &S, float bg, uint32_t n, uint32_t id, int w0, uint32_t &gb,
+                                           uint32_t &bc) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  gb = __reduce_max_sync(0xffffffffu, __float_as_uint(bg));
+  bc = __reduce_min_sync(0xffffffffu, __float_as_uint(bg) == gb ? bc : EMPTY);
+  if (n > 32) {
+    if (lane == 0) { S.redg[wid] = gb; S.redc[wid] = bc; }
+    group_sync(id, n);
+    gb = 0;
+    bc = EMPTY;
+    for (uint32_t k = 0; k < (n >> 5); ++k) {
+      const uint32_t og = S.redg[w0 + k], oc = S.redc[w0 + k];
+      if (og > gb || (og == gb && oc < bc)) { gb = og; bc = oc; }
+    }
+  } else {
+    __syncwarp();
+  }
+}
+
 // The best move of u over the communities of a table (kd: the weight to its
-// own community), by the n threads of a group whose first warp is w0: the
-// largest gain (positive, so its bits order as the floats), then the lowest
-// id. Four slots of a thread in flight: their communities' totals are gathers.
+// own community), by the n threads of a group whose first warp is w0. Four
+// slots of a thread in flight: their communities' totals are gathers.
 template <bool SYNC, int MODE>
 __device__ __forceinline__ void best_of_table(const PhaseArgs &a, Shared &S, const uint32_t *keys, const uint32_t *vals,
                                               uint32_t slots, uint32_t t, uint32_t n, uint32_t id, int w0, float kd,
                                               double wu, double td, float kr, uint32_t &gb, uint32_t &bc) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const float wuf = __double2float_rn(wu);
   float bg = 0.f;
   bc = EMPTY;
@@ -451,22 +482,8 @@ __device__ __forceinline__ void best_of_table(const PhaseArgs &a, Shared &S, con
       if (g > 0.f && better(g, c[k], bg, bc)) { bg = g; bc = c[k]; }
     }
   }
-  gb = __reduce_max_sync(0xffffffffu, __float_as_uint(bg));
-  bc = __reduce_min_sync(0xffffffffu, __float_as_uint(bg) == gb ? bc : EMPTY);
-  if (n > 32) {
-    if (lane == 0) { S.redg[wid] = gb; S.redc[wid] = bc; }
-    group_sync(id, n);
-    gb = 0;
-    bc = EMPTY;
-    for (uint32_t k = 0; k < (n >> 5); ++k) {
-      const uint32_t og = S.redg[w0 + k], oc = S.redc[w0 + k];
-      if (og > gb || (og == gb && oc < bc)) { gb = og; bc = oc; }
-    }
-  } else {
-    __syncwarp();
-  }
+  group_best(S, bg, n, id, w0, gb, bc);
 }
-
 // One vertex by the n threads (1, 4, 8 or 32 warps, thread t) of a group, with
 // a table of twice its degree (at most 2^lgmax slots).
 template <bool SYNC, int MODE>
@@ -504,12 +521,86 @@ __device__ __forceinline__ void group_vertex(const PhaseArgs &a, Shared &S, uint
   }
 }
 
+// Hub h of the plan by the n threads of a group from its resident table, which
+// describes the state of the class's start: the community it goes to into
+// hub_move (EMPTY: it stays, or is not active) and the one it leaves into
+// hub_from. A hub whose table is bad is left to its chunks. 256 threads a hub:
+// a table has 64 to 65536 slots, and a class a hub or two for each block; what
+// it costs is the chain of loads, not the slots. The tables are brought up to
+// date where the movers' neighbours are marked (mark_row), which looks at those
+// rows anyway; as a kernel of its own per class it took 156 us, reading every
+// vertex's decision.
+__device__ __forceinline__ bool table_good(const PhaseArgs &a, uint32_t u) {
+  const uint32_t h = a.ht.key ? a.ht.slot[u] : NO_HUB;
+  return h != NO_HUB && !a.ht.bad[h];
+}
+
+__device__ __forceinline__ void table_hub(const PhaseArgs &a, Shared &S, uint32_t h, uint32_t t, uint32_t n,
+                                          uint32_t id, unsigned long long &fix, unsigned long long &slots) {
+  const int w0 = int(threadIdx.x >> 5) - int(t >> 5);
+  const uint32_t u = a.hub_vertex[h], ti = a.ht.slot[u];
+  if (ti == NO_HUB || a.ht.bad[ti]) return;
+  if (!a.vaff[u] || (a.fa && !a.fa[u])) {
+    if (t == 0) a.hub_move[h] = EMPTY;
+    return;
+  }
+  const uint64_t o = a.ht.off[ti];
+  const int lg = a.ht.lg[ti];
+  const uint32_t m = 1u << lg, d = a.vcom[u];
+  const uint32_t *keys = a.ht.key + o, *cnt = a.ht.cnt + o;
+  const double wu = a.vtot[u], td = a.ctot[d];
+  const float wuf = __double2float_rn(wu);
+  float kd = 0.f;
+  for (uint32_t s = hash_hi(d, lg), p = 0; p < m; ++p, s = (s + 1u) & (m - 1u)) {
+    const uint32_t c = keys[s];
+    if (c == d) kd = float(cnt[s]);
+    if (c == d || c == EMPTY) break;
+  }
+  float bg = 0.f;
+  uint32_t bc = EMPTY, gb;
+  constexpr int U = 4;
+  for (uint32_t s = t; s < m; s += U * n) {
+    uint32_t c[U], k[U];
+    double tc[U];
+#pragma unroll
+    for (int x = 0; x < U; ++x) c[x] = s + x * n < m ? keys[s + x * n] : EMPTY;
+#pragma unroll
+    for (int x = 0; x < U; ++x) {
+      if (c[x] == d) c[x] = EMPTY;
+      k[x] = c[x] != EMPTY ? cnt[s + x * n] : 0u;
+      tc[x] = c[x] != EMPTY ? a.ctot[c[x]] : 0.0;
+    }
+#pragma unroll
+    for (int x = 0; x < U; ++x) {
+      if (!k[x]) continue;
+      const float g = gain_of(float(k[x]), kd, wu, wuf, tc[x], td, a.kr);
+      if (g > 0.f && better(g, c[x], bg, bc)) { bg = g; bc = c[x]; }
+    }
+  }
+  group_best(S, bg, n, id, w0, gb, bc);
+  if (t == 0) {
+    const bool moved = bc != EMPTY && bc != 0u;  // (community 0 is never a target)
+    if (bc != EMPTY) fix += gain_to_fix(__uint_as_float(gb));
+    a.hub_move[h] = moved ? bc : EMPTY;
+    a.hub_from[h] = d;
+    a.vaff[u] = 0;
+    atomicAdd(&S.cnt[NUM_BINS - 1], 1u);
+    if (moved) atomicAdd(&S.hubmv, 1u);
+    slots += m;
+  }
+  group_sync(id, n);  // (the group's sums are read until here)
+}
+
 // ---- hubs (degree above 8192), in two steps with a grid barrier between.
 // Step 1, a block per chunk of a hub's edges: the chunk's communities are
 // counted in the block's table and written out as (community, weight) pairs,
 // grouped by the hub's `parts` hash partitions of the communities (segs: the
 // groups' bounds), so that step 2 splits a hub of many communities over
 // blocks. chunk_cnt is EMPTY for a hub that is not active.
+__device__ __forceinline__ bool hub_active(const PhaseArgs &a, uint32_t u) {
+  return a.vaff[u] && (!a.fa || a.fa[u]) && (!a.gact || a.gact[a.gid[u]]) && !table_good(a, u);
+}
+
 template <bool SYNC, int MODE>
 __device__ __forceinline__ void hub_chunk(const PhaseArgs &a, Shared &S, uint32_t ci, uint32_t *table) {
   using V = Sum<MODE>;
@@ -517,7 +608,7 @@ __device__ __forceinline__ void hub_chunk(const PhaseArgs &a, Shared &S, uint32_
   const uint4 ch = a.chunk[ci];
   const uint32_t u = ch.w, h = ch.x;
   if (threadIdx.x == 0) {
-    S.over = a.vaff[u] && (!a.fa || a.fa[u]) && (!a.gact || a.gact[a.gid[u]]);
+    S.over = hub_active(a, u);
     S.next = 0;
   }
   __syncthreads();
@@ -602,6 +693,7 @@ __device__ __forceinline__ void hub_merge(const PhaseArgs &a, Shared &S, uint2 t
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const uint32_t h = task.x, r = task.y, R = a.hub_parts[h];
   const uint32_t u = a.hub_vertex[h];
+  if (table_good(a, u)) return;  // (decided from its table; block-uniform)
   const uint32_t c0 = a.hub_first[h], nc = a.hub_first[h + 1] - c0;
   if (threadIdx.x == 0) { S.next = 0; S.over = 0; }
   __syncthreads();
@@ -693,7 +785,9 @@ __device__ __forceinline__ void hub_merge(const PhaseArgs &a, Shared &S, uint2 t
       S.edges[NUM_BINS - 1] += a.deg[u];
       if (moved) {
         S.hubmv += 1;
-        if constexpr (!SYNC) {
+        if constexpr (SYNC) {
+          a.hub_from[h] = d;
+        } else {
           atomicAdd(&a.ctot[d], -wu);
           atomicAdd(&a.ctot[bc], wu);
           a.vcom[u] = bc;
@@ -739,7 +833,8 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
   uint32_t nbar = 0;  // barriers so far
   double el = 0.0;
   unsigned long long fix = 0;  // the thread's share of the iteration's gain sum
-  unsigned long long sum = 0;
+  unsigned long long sum = 0, slots = 0;
+  const bool tabs = SYNC && MODE == UNIT && a.ht.key;  // the hubs are decided from resident tables
   uint32_t l = 0;
   while (l < uint32_t(a.L)) {
     // what ends an iteration: its gain sum, or the graphs of the union still moving
@@ -778,10 +873,43 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
       __syncthreads();
       // ---- 2. decide them
       const uint32_t ch0 = a.chunk_begin[k], nch = a.chunk_begin[k + 1] - ch0;
-      for (uint32_t t = G - 1 - bid; t < nch; t += G) {  // (from the last block: the first ones have the heaviest lists)
-        hub_chunk<SYNC, MODE>(a, S, ch0 + t, table);
-        __syncthreads();
+      // the block's chunks of the class that pred holds for, to work(); 256 are
+      // asked at once: most are of hubs with nothing to do, and one after the
+      // other each would cost the latency of two loads. (From the last block:
+      // the first ones have the heaviest lists.)
+      auto each_chunk = [&](auto pred, auto work) {
+        for (uint32_t t0 = G - 1 - bid; t0 < nch; t0 += TODO * G) {
+          if (tid == 0) S.ntodo = 0;
+          __syncthreads();
+          const uint32_t t = t0 + tid * G;
+          if (tid < TODO && t < nch && pred(t)) S.todo[atomicAdd(&S.ntodo, 1u)] = t;
+          __syncthreads();
+          const uint32_t n = S.ntodo;
+          for (uint32_t i = 0; i < n; ++i) {
+            work(S.todo[i]);
+            __syncthreads();
+          }
+          __syncthreads();
+        }
+      };
+      bool scan = nch != 0;  // some hub of the class is counted from its edges
+      if constexpr (SYNC && MODE == UNIT) {
+        if (tabs && nch) {
+          scan = ld_relaxed(a.ht.nbad) != 0;  // (raised between decisions only: the same for every block)
+          const uint32_t g = wid >> 3, h1 = a.hub_begin[k + 1];
+          for (uint32_t h = a.hub_begin[k] + (G - 1 - bid) * 4 + g; h < h1; h += G * 4)
+            table_hub(a, S, h, tid & 255u, 256, 9 + g, fix, slots);
+          __syncthreads();
+        }
       }
+      if (scan)
+        each_chunk(
+            [&](uint32_t t) {
+              const bool act = hub_active(a, a.chunk[ch0 + t].w);
+              if (!act) a.chunk_cnt[ch0 + t] = EMPTY;
+              return act;
+            },
+            [&](uint32_t t) { hub_chunk<SYNC, MODE>(a, S, ch0 + t, table); });
       auto blocks = [&] {  // degree above 512: the whole block, then eight warps each
         const uint32_t c10 = S.cnt[10], c9 = S.cnt[9];
         for (uint32_t i = 0; i < c10; ++i) {
@@ -844,7 +972,7 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
         blocks();
       }
       __syncthreads();
-      if (nch) {  // (the same for every block)
+      if (scan) {  // (the same for every block)
         if (tid == 0) S.next = 0;
         if (!grid_barrier(a, S, nbar++, 0, nullptr)) return;
         const uint32_t m0 = a.merge_begin[k], m1 = a.merge_begin[k + 1];
@@ -876,45 +1004,59 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
       if constexpr (SYNC) {
         if (any) {
           // eight lanes per move; rows above 256 entries by 256 threads
-          uint32_t *big = table;
+          uint32_t *big = table;  // (vertex, its old and new community)
+          constexpr uint32_t BIG_CAP = TABLE_WORDS / 3;
           const uint32_t sl = tid & 7u;
           for (uint32_t i = tid >> 3; i < nmv; i += PB / 8) {
             const uint2 m = mv[i];
             const uint64_t o = a.off[m.x];
             const uint32_t dg = a.deg[m.x];
+            uint32_t d = 0, late = 0;
             if (sl == 0) {
-              const uint32_t d = a.vcom[m.x];
+              d = a.vcom[m.x];
               const double wu = a.vtot[m.x];
               atomicAdd(&a.ctot[d], -wu);
               atomicAdd(&a.ctot[m.y], wu);
               a.vcom[m.x] = m.y;
-              if (dg > 256) big[atomicAdd(&S.nbig, 1u)] = m.x;
+              if (dg > 256) {
+                const uint32_t j = atomicAdd(&S.nbig, 1u);
+                if (j < BIG_CAP) {
+                  big[3 * j] = m.x;
+                  big[3 * j + 1] = d;
+                  big[3 * j + 2] = m.y;
+                  late = 1;
+                }
+              }
             }
-            if (dg <= 256) mark_row(a, m.x, o, dg, sl, 8);
+            d = __shfl_sync(0xffu << (lane & 24u), d, 0, 8);
+            if (!__shfl_sync(0xffu << (lane & 24u), late, 0, 8)) mark_row(a, m.x, o, dg, sl, 8, tabs, d, m.y);
           }
           __syncthreads();
-          const uint32_t nbig = S.nbig;
-          for (uint32_t i = wid >> 3; i < nbig; i += PW / 8) mark_row(a, big[i], a.off[big[i]], a.deg[big[i]], tid & 255u, 256);
-          for (uint32_t t = G - 1 - bid; t < nch; t += G) {  // the moved hubs' chunks
-            const uint4 ch = a.chunk[ch0 + t];
-            const uint32_t c = a.hub_move[ch.x], u = ch.w;
-            if (c == EMPTY) continue;
-            if (ch.y == 0 && tid == 0) {
-              const uint32_t d = a.vcom[u];
-              const double wu = a.vtot[u];
-              atomicAdd(&a.ctot[d], -wu);
-              atomicAdd(&a.ctot[c], wu);
-              a.vcom[u] = c;
-            }
-            mark_row(a, u, a.off[u] + ch.y, ch.z - ch.y, tid, PB);
+          const uint32_t nbig = min(S.nbig, BIG_CAP);
+          for (uint32_t i = wid >> 3; i < nbig; i += PW / 8) {
+            const uint32_t u = big[3 * i];
+            mark_row(a, u, a.off[u], a.deg[u], tid & 255u, 256, tabs, big[3 * i + 1], big[3 * i + 2]);
           }
+          each_chunk([&](uint32_t t) { return a.hub_move[a.chunk[ch0 + t].x] != EMPTY; },  // the moved hubs' chunks
+                     [&](uint32_t t) {
+                       const uint4 ch = a.chunk[ch0 + t];
+                       const uint32_t c = a.hub_move[ch.x], d = a.hub_from[ch.x], u = ch.w;
+                       if (ch.y == 0 && tid == 0) {
+                         const double wu = a.vtot[u];
+                         atomicAdd(&a.ctot[d], -wu);
+                         atomicAdd(&a.ctot[c], wu);
+                         a.vcom[u] = c;
+                       }
+                       mark_row(a, u, a.off[u] + ch.y, ch.z - ch.y, tid, PB, tabs, d, c);
+                     });
         }
       } else {
         // the moved hubs' neighbours, by the blocks of their chunks
-        for (uint32_t t = G - 1 - bid; t < nch; t += G) {
-          const uint4 ch = a.chunk[ch0 + t];
-          if (a.hub_move[ch.x] != EMPTY) mark_row(a, ch.w, a.off[ch.w] + ch.y, ch.z - ch.y, tid, PB);
-        }
+        each_chunk([&](uint32_t t) { return a.hub_move[a.chunk[ch0 + t].x] != EMPTY; },
+                   [&](uint32_t t) {
+                     const uint4 ch = a.chunk[ch0 + t];
+                     mark_row(a, ch.w, a.off[ch.w] + ch.y, ch.z - ch.y, tid, PB);
+                   });
       }
       if (last && a.gfix)  // graph unions: each graph's own stop test
         for (uint32_t i = bid * PB + tid; i < a.graphs; i += G * PB) phase_control(a, i, l % 3);
@@ -948,6 +1090,7 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
     atomicAdd(&a.ctr->bin_edges[tid], S.se[tid]);
     atomicAdd(&a.ctr->edges, S.se[tid]);
   }
+  if (SYNC && MODE == UNIT && slots) atomicAdd(&a.ctr->ht_slots, slots);
   if (tid == 0) {
     if (S.moves) atomicAdd(&a.ctr->moves, S.moves);
     if (S.bad) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
