@@ -1833,10 +1833,10 @@ PlanCounts plan_device(lvg_graph *g, const uint32_t *ds, const uint32_t *dd, con
   };
   one(ds, dd, dw, nd, g->u_ds.p, g->u_dd.p, g->u_dw.p, g->u_cnt.p + 0);
   one(is, id, iw, ni, g->u_is.p, g->u_id.p, g->u_iw.p, g->u_cnt.p + 1);
-  g->u_touch.ensure(S + 1); g->u_tpos.ensure(S + 1); g->u_tscan.ensure(scan_scratch_elems(S + 1));
+  g->u_touch.ensure(2 * n); g->u_tpos.ensure(2 * n + 1); g->u_tscan.ensure(scan_scratch_elems(2 * n + 1));
   g->u_rows.ensure(std::min(S, nd + ni));
   launch_plan_rows(g->u_ds.p, g->u_cnt.p + 0, g->u_is.p, g->u_cnt.p + 1, n, g->u_touch.p, g->u_tpos.p,
-                   g->u_tscan.p, S, g->u_rows.p, g->upd.p, g->u_cnt.p + 2, s);
+                   g->u_tscan.p, g->u_rows.p, g->upd.p, g->u_cnt.p + 2, s);
   LVG_CUDA(cudaMemcpyAsync(g->hcnt.p, g->u_cnt.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   LVG_CUDA(cudaMemcpyAsync(g->hupd.p + UPD_MAXG, g->upd.p + UPD_MAXG, sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
   LVG_CUDA(cudaStreamSynchronize(s));

@@ -617,8 +617,8 @@ void launch_first_flags(const uint64_t *key, size_t n, uint32_t *flag, cudaStrea
 void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t *flag, const uint32_t *pos,
                         size_t n, int b, const float *w, uint32_t *os, uint32_t *od, float *ow, cudaStream_t s);
 void launch_plan_rows(const uint32_t *ds, const uint32_t *nd, const uint32_t *is, const uint32_t *ni, size_t cap,
-                      uint32_t *touched, uint32_t *tpos, uint32_t *scan, size_t span, UpdRow *rows,
-                      unsigned long long *upd, uint32_t *nrows, cudaStream_t s);
+                      uint32_t *flag, uint32_t *pos, uint32_t *scan, UpdRow *rows, unsigned long long *upd,
+                      uint32_t *nrows, cudaStream_t s);
 
 // ---------------------------------------------------------------- generators (lvg_gen.cu)
 // Stable radix sorts of 64-bit keys over bits [0, end_bit) (cub); the result

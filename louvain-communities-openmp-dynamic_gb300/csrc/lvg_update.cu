@@ -145,61 +145,180 @@ __device__ __forceinline__ uint32_t row_of(const uint64_t *start, uint32_t nrows
   return lo;
 }
 
-// Step 2, one thread per source item (old entries from f0, then insertions)
-// of all touched rows: the item's place in the rewritten row, into scratch.
-// An old entry at i goes to i - (kept deletions before it) + (kept
-// insertions before it); a kept insertion j to j's kept rank + (old entries
-// before it) - (kept deletions before it).
+// The rows of a stretch [x0, x1) of a flat range, for a converged warp: r0 and
+// r1, the rows of its ends, found by 32 probes at a time (a search of 17 steps
+// per item was most of the time of the passes below), and the starts of the
+// 32 rows from r0 on, one a lane.
+struct WarpRows {
+  uint32_t r0, r1;
+  uint64_t st;
+  __device__ __forceinline__ WarpRows(const uint64_t *start, uint32_t nrows, uint64_t x0, uint64_t x1) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t lo = 0, hi = nrows;  // start[lo] <= x0 < start[hi]
+    while (hi - lo > 1) {
+      const uint32_t step = (hi - lo + 31u) >> 5, at = lo + lane * step;
+      const uint32_t n = __popc(__ballot_sync(0xffffffffu, at < hi && start[at] <= x0));  // (a prefix; at least lane 0)
+      lo += (n - 1) * step;
+      hi = min(hi, lo + step);
+    }
+    r0 = lo;
+    st = r0 + lane < nrows ? start[r0 + lane] : ~0ull;
+    const uint32_t n = __popc(__ballot_sync(0xffffffffu, st < x1));
+    r1 = n < 32 ? r0 + n - 1 : r0 + 31 + row_of(start + r0 + 31, nrows - r0 - 31, x1 - 1);
+  }
+  // The row of item x (of this stretch), by all lanes.
+  __device__ __forceinline__ uint32_t find(const uint64_t *start, uint64_t x) const {
+    if (r1 == r0) return r0;
+    if (r1 - r0 >= 32) return r0 + row_of(start + r0, r1 - r0 + 1, x);
+    uint32_t at = 0;
+#pragma unroll
+    for (uint32_t step = 16; step > 0; step >>= 1)
+      if (__shfl_sync(0xffffffffu, st, at + step) <= x) at += step;
+    return r0 + at;
+  }
+};
+
+// Items a warp takes at once: enough stretches for every warp of the device,
+// at most 1024 items (the ends' searches and a row's plan are paid once).
+uint32_t items_per_warp(uint64_t total) {
+  uint32_t per = 32;
+  while (per < 1024 && total / (2 * per) >= 16384) per *= 2;
+  return per;
+}
+
+// Step 2, over the source items (old entries from f0, then insertions) of all
+// touched rows: the item's place in the rewritten row, into scratch. An old
+// entry at i goes to i - (kept deletions before it) + (kept insertions before
+// it); a kept insertion j to j's kept rank + (old entries before it) - (kept
+// deletions before it). Where a stretch of old entries lies between two
+// neighbouring batch entries of its row, it is copied by a constant shift: the
+// bulk of the items are those of a few long rows. (A 1e-4 |E| batch on R-MAT
+// scale 24: 269 us, 446 with a search of the rows and the row's lists per
+// item.)
 __global__ void merge_items_kernel(const uint64_t *off, const uint32_t *deg, const uint32_t *key, const float *w,
                                    const UpdRow *rows, uint32_t nrows, const uint32_t *dd, const uint32_t *id,
                                    const float *iw, size_t nd_all, const uint32_t *pre, const uint32_t *keep,
-                                   const RowPlan *plan, const uint64_t *src, uint64_t total, const uint64_t *spos,
-                                   uint32_t *skey, float *sw) {
-  for (uint64_t x = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < total;
-       x += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t r = row_of(src, nrows, x);
-    const UpdRow R = rows[r];
-    const RowPlan P = plan[r];
-    const uint64_t o = off[R.u];
-    const uint32_t n = deg[R.u];
-    const uint32_t *row = key + o;
-    const uint32_t *dl = dd + R.d0, nd = R.d1 - R.d0;
-    const uint32_t *il = id + R.i0, ni = R.i1 - R.i0;
-    const uint32_t *dpre = pre + R.d0, *ipre = pre + nd_all + R.i0;
-    const uint32_t j = uint32_t(x - src[r]);
-    const uint64_t base = spos[r];
-    if (j < n - P.f0) {
-      const uint32_t i = P.f0 + j;
-      const uint32_t k = row[i];
-      const uint32_t a = count_less(dl, nd, k);
-      if (a < nd && dl[a] == k) continue;  // deleted (present, so kept)
-      const uint32_t b = count_less(il, ni, k);
-      const uint32_t at = i - (a < nd ? dpre[a] : P.dcarry) + (b < ni ? ipre[b] : P.icarry) - P.f0;
-      skey[base + at] = k;
-      sw[base + at] = w[o + i];
-    } else {
-      const uint32_t jj = j - (n - P.f0);
-      if (!keep[nd_all + R.i0 + jj]) continue;  // already present: tidied away
-      const uint32_t k = il[jj];
-      const uint32_t a = count_less(dl, nd, k);
-      const uint32_t at = ipre[jj] + count_less(row, n, k) - (a < nd ? dpre[a] : P.dcarry) - P.f0;
-      skey[base + at] = k;
-      sw[base + at] = iw[R.i0 + jj];
+                                   const RowPlan *plan, const uint64_t *src, uint64_t total, uint32_t per,
+                                   const uint64_t *spos, uint32_t *skey, float *sw) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t warps = uint64_t(gridDim.x) * blockDim.x / 32;
+  for (uint64_t x0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * per; x0 < total; x0 += warps * per) {
+    const uint64_t x1 = min(x0 + per, total);
+    const WarpRows W(src, nrows, x0, x1);
+    if (W.r0 == W.r1) {
+      const uint32_t r = W.r0;
+      const UpdRow R = rows[r];
+      const RowPlan P = plan[r];
+      const uint64_t o = off[R.u];
+      const uint32_t n = deg[R.u], i0 = P.f0 + uint32_t(x0 - src[r]), i1 = P.f0 + uint32_t(x1 - src[r]);
+      if (i1 <= n) {  // old entries only
+        const uint32_t *dl = dd + R.d0, nd = R.d1 - R.d0;
+        const uint32_t *il = id + R.i0, ni = R.i1 - R.i0;
+        // lanes 0-3: the batch entries before the stretch's ends
+        const uint32_t k = key[o + (lane & 1u ? i1 - 1 : i0)];
+        const uint32_t c = lane & 2u ? count_less(il, ni, k) : count_less(dl, nd, k);
+        const uint32_t a0 = __shfl_sync(0xffffffffu, c, 0), a1 = __shfl_sync(0xffffffffu, c, 1);
+        const uint32_t b0 = __shfl_sync(0xffffffffu, c, 2), b1 = __shfl_sync(0xffffffffu, c, 3);
+        const uint32_t last = __shfl_sync(0xffffffffu, k, 1);
+        const bool shift = a0 == a1 && b0 == b1 && !(a1 < nd && dl[a1] == last);
+        const uint32_t *dpre = pre + R.d0, *ipre = pre + nd_all + R.i0;
+        const uint64_t base = spos[r] - P.f0;
+        const uint32_t by = (b0 < ni ? ipre[b0] : P.icarry) - (a0 < nd ? dpre[a0] : P.dcarry);
+        for (uint32_t i = i0 + lane; i < i1; i += 128) {
+          uint32_t kk[4];
+          float ww[4];
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            if (i + 32 * q < i1) { kk[q] = key[o + i + 32 * q]; ww[q] = w[o + i + 32 * q]; }
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const uint32_t ii = i + 32 * q;
+            if (ii >= i1) continue;
+            uint32_t at = ii + by;
+            if (!shift) {
+              const uint32_t aa = a0 + count_less(dl + a0, a1 - a0, kk[q]);
+              if (aa < nd && dl[aa] == kk[q]) continue;  // deleted (present, so kept)
+              const uint32_t bb = b0 + count_less(il + b0, b1 - b0, kk[q]);
+              at = ii - (aa < nd ? dpre[aa] : P.dcarry) + (bb < ni ? ipre[bb] : P.icarry);
+            }
+            skey[base + at] = kk[q];
+            sw[base + at] = ww[q];
+          }
+        }
+        continue;
+      }
+    }
+    for (uint64_t x = x0 + lane; x - lane < x1; x += 32) {  // any rows, any items
+      const uint32_t r = W.find(src, min(x, x1 - 1));
+      if (x >= x1) continue;
+      const UpdRow R = rows[r];
+      const RowPlan P = plan[r];
+      const uint64_t o = off[R.u];
+      const uint32_t n = deg[R.u];
+      const uint32_t *row = key + o;
+      const uint32_t *dl = dd + R.d0, nd = R.d1 - R.d0;
+      const uint32_t *il = id + R.i0, ni = R.i1 - R.i0;
+      const uint32_t *dpre = pre + R.d0, *ipre = pre + nd_all + R.i0;
+      const uint32_t j = uint32_t(x - src[r]);
+      const uint64_t base = spos[r];
+      if (j < n - P.f0) {
+        const uint32_t i = P.f0 + j;
+        const uint32_t k = row[i];
+        const uint32_t a = count_less(dl, nd, k);
+        if (a < nd && dl[a] == k) continue;  // deleted (present, so kept)
+        const uint32_t b = count_less(il, ni, k);
+        const uint32_t at = i - (a < nd ? dpre[a] : P.dcarry) + (b < ni ? ipre[b] : P.icarry) - P.f0;
+        skey[base + at] = k;
+        sw[base + at] = w[o + i];
+      } else {
+        const uint32_t jj = j - (n - P.f0);
+        if (!keep[nd_all + R.i0 + jj]) continue;  // already present: tidied away
+        const uint32_t k = il[jj];
+        const uint32_t a = count_less(dl, nd, k);
+        const uint32_t at = ipre[jj] + count_less(row, n, k) - (a < nd ? dpre[a] : P.dcarry) - P.f0;
+        skey[base + at] = k;
+        sw[base + at] = iw[R.i0 + jj];
+      }
     }
   }
 }
 
-// Step 3, one thread per rewritten entry: scratch -> the row's place (in
-// place from f0, or the row's new stretch in the pool at pool + gpos[r]).
+// Step 3, over the rewritten entries: scratch -> the row's place (in place
+// from f0, or the row's new stretch in the pool at pool + gpos[r]). (The same
+// batch: 232 us, 417 with a search per entry.)
 __global__ void copy_items_kernel(const uint64_t *off, const UpdRow *rows, uint32_t nrows, const RowPlan *plan,
-                                  const uint64_t *spos, uint64_t total, const uint64_t *grow, const uint64_t *gpos,
-                                  uint64_t pool, const uint32_t *skey, const float *sw, uint32_t *key, float *w) {
-  for (uint64_t x = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; x < total;
-       x += uint64_t(gridDim.x) * blockDim.x) {
-    const uint32_t r = row_of(spos, nrows, x);
-    const uint64_t dst = (grow[r] ? pool + gpos[r] : off[rows[r].u]) + plan[r].f0 + (x - spos[r]);
-    key[dst] = skey[x];
-    w[dst] = sw[x];
+                                  const uint64_t *spos, uint64_t total, uint32_t per, const uint64_t *grow,
+                                  const uint64_t *gpos, uint64_t pool, const uint32_t *skey, const float *sw,
+                                  uint32_t *key, float *w) {
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint64_t warps = uint64_t(gridDim.x) * blockDim.x / 32;
+  auto place = [&](uint32_t r) {  // of entry 0 of the flat range, were it the row's
+    return (grow[r] ? pool + gpos[r] : off[rows[r].u]) + plan[r].f0 - spos[r];
+  };
+  for (uint64_t x0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32 * per; x0 < total; x0 += warps * per) {
+    const uint64_t x1 = min(x0 + per, total);
+    const WarpRows W(spos, nrows, x0, x1);
+    if (W.r0 == W.r1) {
+      const uint64_t to = place(W.r0);
+      for (uint64_t x = x0 + lane; x < x1; x += 128) {
+        uint32_t kk[4];
+        float ww[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (x + 32 * q < x1) { kk[q] = skey[x + 32 * q]; ww[q] = sw[x + 32 * q]; }
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (x + 32 * q < x1) { key[to + x + 32 * q] = kk[q]; w[to + x + 32 * q] = ww[q]; }
+      }
+    } else {
+      for (uint64_t x = x0 + lane; x - lane < x1; x += 32) {
+        const uint32_t r = W.find(spos, min(x, x1 - 1));
+        if (x >= x1) continue;
+        const uint64_t dst = place(r) + x;
+        key[dst] = skey[x];
+        w[dst] = sw[x];
+      }
+    }
   }
 }
 
@@ -230,14 +349,20 @@ __global__ void finish_rows_kernel(uint64_t *off, uint32_t *deg, uint32_t *cap, 
   }
 }
 
-// Present vertices, counted into *dst.
+// Present vertices, counted into *dst, sixteen flags per load (ex is a device
+// allocation, so aligned; a byte per load took 30 us on R-MAT scale 24).
 __global__ void count_present_kernel(const uint8_t *ex, size_t n, unsigned long long *dst) {
-  unsigned long long c = 0;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x)
-    c += ex[i] != 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(dst, c);
+  unsigned int c = 0;
+  const size_t n16 = n / 16, t = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const uint4 *e16 = reinterpret_cast<const uint4 *>(ex);
+  auto some = [](uint32_t v) { return __popc(__vcmpne4(v, 0u)) / 8; };
+  for (size_t i = t; i < n16; i += size_t(gridDim.x) * blockDim.x) {
+    const uint4 v = e16[i];
+    c += some(v.x) + some(v.y) + some(v.z) + some(v.w);
+  }
+  if (t < n % 16) c += ex[16 * n16 + t] != 0;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(dst, (unsigned long long)c);
 }
 
 // Spread a compact CSR into the gapped layout (one warp per row; gaps zero).
@@ -305,17 +430,6 @@ __global__ void unpack_keys_kernel(const uint64_t *key, const uint32_t *val, con
   }
 }
 
-// touched[u] = 1 for every source of the (deduplicated) lists; their lengths
-// are read from the device (*nd, *ni).
-__global__ void touch_kernel(const uint32_t *ds, const uint32_t *nd, const uint32_t *is, const uint32_t *ni,
-                             size_t cap, uint32_t *touched) {
-  const uint32_t a = *nd, c = *ni;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < cap; i += size_t(gridDim.x) * blockDim.x) {
-    if (i < a) touched[ds[i]] = 1;
-    if (i < c) touched[is[i]] = 1;
-  }
-}
-
 __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t n, uint32_t x) {
   uint32_t lo = 0, hi = n;
   while (lo < hi) {
@@ -325,21 +439,45 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t 
   return lo;
 }
 
-// One UpdRow per touched vertex, in id order; the longest insertion run into
-// upd[UPD_MAXG].
-__global__ void plan_rows_kernel(const uint32_t *touched, const uint32_t *tpos, size_t span, const uint32_t *ds,
-                                 const uint32_t *nd, const uint32_t *is, const uint32_t *ni, UpdRow *rows,
-                                 unsigned long long *upd) {
+// The touched vertices are the sources of the two sorted lists (their lengths
+// are read from the device: *nd, *ni; room for cap entries each): flag[i] = 1
+// for the first deletion of a source, flag[cap + j] = 1 for the first
+// insertion of a source without deletions.
+__global__ void row_flags_kernel(const uint32_t *ds, const uint32_t *nd, const uint32_t *is, const uint32_t *ni,
+                                 size_t cap, uint32_t *flag) {
   const uint32_t a = *nd, c = *ni;
-  for (size_t u = size_t(blockIdx.x) * blockDim.x + threadIdx.x; u < span; u += size_t(gridDim.x) * blockDim.x) {
-    if (!touched[u]) continue;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < cap; i += size_t(gridDim.x) * blockDim.x) {
+    flag[i] = i < a && (i == 0 || ds[i] != ds[i - 1]);
+    bool f = i < c && (i == 0 || is[i] != is[i - 1]);
+    if (f) {
+      const uint32_t p = lower_bound_u32(ds, a, is[i]);
+      f = !(p < a && ds[p] == is[i]);
+    }
+    flag[cap + i] = f;
+  }
+}
+
+// One UpdRow per touched vertex, in id order (pos: the flags' exclusive prefix;
+// a row's place is its rank in its own list plus the other list's flagged
+// sources below it); the longest insertion run into upd[UPD_MAXG]. (A pass over
+// all vertices for the batch's few sources took 0.25 ms with its scan on R-MAT
+// scale 24.)
+__global__ void plan_rows_kernel(const uint32_t *flag, const uint32_t *pos, size_t cap, const uint32_t *ds,
+                                 const uint32_t *nd, const uint32_t *is, const uint32_t *ni, UpdRow *rows,
+                                 unsigned long long *upd, uint32_t *nrows) {
+  const uint32_t a = *nd, c = *ni;
+  const uint32_t deletions = pos[cap], total = pos[2 * cap];  // flagged
+  if (blockIdx.x == 0 && threadIdx.x == 0) *nrows = total;
+  for (size_t t = size_t(blockIdx.x) * blockDim.x + threadIdx.x; t < 2 * cap; t += size_t(gridDim.x) * blockDim.x) {
+    if (!flag[t]) continue;
+    const bool del = t < cap;
     UpdRow R;
-    R.u = uint32_t(u);
-    R.d0 = lower_bound_u32(ds, a, R.u);
-    R.d1 = lower_bound_u32(ds, a, R.u + 1);
-    R.i0 = lower_bound_u32(is, c, R.u);
+    R.u = del ? ds[t] : is[t - cap];
+    R.d0 = del ? uint32_t(t) : lower_bound_u32(ds, a, R.u);
+    R.d1 = del ? lower_bound_u32(ds, a, R.u + 1) : R.d0;
+    R.i0 = del ? lower_bound_u32(is, c, R.u) : uint32_t(t - cap);
     R.i1 = lower_bound_u32(is, c, R.u + 1);
-    rows[tpos[u]] = R;
+    rows[del ? pos[t] + (pos[cap + R.i0] - deletions) : pos[t] - deletions + pos[R.d0]] = R;
     if (R.i1 > R.i0) atomicMax(&upd[UPD_MAXG], (unsigned long long)(R.i1 - R.i0));
   }
 }
@@ -407,8 +545,9 @@ void launch_merge_items(const uint64_t *off, const uint32_t *deg, const uint32_t
                         const uint64_t *src, uint64_t total, const uint64_t *spos, uint32_t *skey, float *sw,
                         cudaStream_t s) {
   if (!total) return;
-  merge_items_kernel<<<grid_for(total, 256), 256, 0, s>>>(off, deg, key, w, rows, uint32_t(nrows), dd, id, iw, nd_all,
-                                                          pre, keep, plan, src, total, spos, skey, sw);
+  const uint32_t per = items_per_warp(total);
+  merge_items_kernel<<<grid_for((total + per - 1) / per * 32, 256), 256, 0, s>>>(
+      off, deg, key, w, rows, uint32_t(nrows), dd, id, iw, nd_all, pre, keep, plan, src, total, per, spos, skey, sw);
   LVG_CHECK_LAUNCH();
 }
 
@@ -417,8 +556,9 @@ void launch_copy_items(const uint64_t *off, const UpdRow *rows, size_t nrows, co
                        uint64_t pool, const uint32_t *skey, const float *sw, uint32_t *key, float *w,
                        cudaStream_t s) {
   if (!total) return;
-  copy_items_kernel<<<grid_for(total, 256), 256, 0, s>>>(off, rows, uint32_t(nrows), plan, spos, total, grow, gpos,
-                                                         pool, skey, sw, key, w);
+  const uint32_t per = items_per_warp(total);
+  copy_items_kernel<<<grid_for((total + per - 1) / per * 32, 256), 256, 0, s>>>(
+      off, rows, uint32_t(nrows), plan, spos, total, per, grow, gpos, pool, skey, sw, key, w);
   LVG_CHECK_LAUNCH();
 }
 
@@ -433,7 +573,7 @@ void launch_finish_rows(uint64_t *off, uint32_t *deg, uint32_t *cap, uint32_t *k
 
 void launch_count_present(const uint8_t *ex, size_t span, unsigned long long *upd, cudaStream_t s) {
   if (!span) return;
-  count_present_kernel<<<grid_for(span, 256), 256, 0, s>>>(ex, span, &upd[UPD_ORDER]);
+  count_present_kernel<<<grid_for(span / 16, 256), 256, 0, s>>>(ex, span, &upd[UPD_ORDER]);
   LVG_CHECK_LAUNCH();
 }
 
@@ -466,15 +606,13 @@ void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t
 }
 
 void launch_plan_rows(const uint32_t *ds, const uint32_t *nd, const uint32_t *is, const uint32_t *ni, size_t cap,
-                      uint32_t *touched, uint32_t *tpos, uint32_t *scan, size_t span, UpdRow *rows,
-                      unsigned long long *upd, uint32_t *nrows, cudaStream_t s) {
-  LVG_CUDA(cudaMemsetAsync(touched, 0, span * sizeof(uint32_t), s));
-  if (cap) {
-    touch_kernel<<<grid_for(cap, 256), 256, 0, s>>>(ds, nd, is, ni, cap, touched);
-    LVG_CHECK_LAUNCH();
-  }
-  exclusive_scan_u32(touched, tpos, span, nrows, scan, s);
-  plan_rows_kernel<<<grid_for(span, 256), 256, 0, s>>>(touched, tpos, span, ds, nd, is, ni, rows, upd);
+                      uint32_t *flag, uint32_t *pos, uint32_t *scan, UpdRow *rows, unsigned long long *upd,
+                      uint32_t *nrows, cudaStream_t s) {
+  if (!cap) return;
+  row_flags_kernel<<<grid_for(cap, 256), 256, 0, s>>>(ds, nd, is, ni, cap, flag);
+  LVG_CHECK_LAUNCH();
+  exclusive_scan_u32(flag, pos, 2 * cap, pos + 2 * cap, scan, s);
+  plan_rows_kernel<<<grid_for(2 * cap, 256), 256, 0, s>>>(flag, pos, cap, ds, nd, is, ni, rows, upd, nrows);
   LVG_CHECK_LAUNCH();
 }
 
