@@ -769,7 +769,9 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   }
   for (int i = 0; i <= lv.colors * NUM_BINS; ++i) a.start[i] = uint32_t(lv.bin_start[i]);
   launch_fill_bytes(W.phase_ctl.p, 0, sizeof(PhaseCtl), s);
-  launch_phase(sync, lv.unit, lv.whole && g->total_weight < 2147483648.0, grid, a, s);
+  // (a dynamic run's totals begin with the caller's, which can be any numbers)
+  const bool small = g->total_weight < 2147483648.0;
+  launch_phase(sync, lv.unit, lv.whole && small, !from_prior && small, grid, a, s);
   ++g->stats.move_launches;
   ++g->stats.level_graphs;
   LVG_CUDA(cudaMemcpyAsync(g->hctr.p, g->ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));

@@ -375,7 +375,7 @@ constexpr uint64_t PHASE_MAX_DEGREE = 8192ull * 16384ull;  // partitions the cou
 // device cannot launch cooperatively).
 uint32_t phase_grid(const Level &lv);
 uint32_t phase_list_cap(const Level &lv, uint32_t grid);
-void launch_phase(bool sync, bool unit, bool whole, uint32_t grid, const PhaseArgs &a, cudaStream_t s);
+void launch_phase(bool sync, bool unit, bool whole, bool totals, uint32_t grid, const PhaseArgs &a, cudaStream_t s);
 bool phase_lists_fit(uint32_t cap);  // the lists stay in shared memory
 
 // Arguments of the aggregation kernels (inc/louvain.hxx:897-912, 987-992).

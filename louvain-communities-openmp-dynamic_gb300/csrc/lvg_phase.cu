@@ -60,20 +60,50 @@ constexpr uint32_t BARRIER_POLLS = 1u << 24;
 
 // The level's weights: any FP32, all 1, or whole numbers whose total is below 2^31.
 enum Weights { FLOATS, UNIT, WHOLE };
+// With UNIT or WHOLE: the vertices' and communities' totals are known to be
+// whole numbers below 2^31 too (static runs: sums of such weights), so gains
+// are computed from their integers. The SM issues an FP64 instruction of a warp
+// in 16 cycles, and a gain takes three of them (two additions and the rounding
+// to FP32): with tables a quarter full that was two thirds of a large vertex's
+// time (16.6 of 26 us above degree 2048, 5.7 of 12.8 at 257-512). The sum wu +
+// tc - td is exact either way and rounded once, so the gains are the same bits.
+constexpr int TOTALS = 4;
 template <int MODE>
-using Sum = typename std::conditional<MODE == FLOATS, float, uint32_t>::type;
+using Tot = typename std::conditional<(MODE & TOTALS) != 0, uint32_t, double>::type;
+// A whole number below 2^32 out of its FP64 bits (an FP64-to-integer
+// conversion would be as slow as the additions).
+__device__ __forceinline__ uint32_t whole_of(double x) {
+  const uint32_t hi = uint32_t(__double2hiint(x)), lo = uint32_t(__double2loint(x));
+  const uint32_t top = __funnelshift_l(lo, hi, 11) | 0x80000000u;  // the mantissa's first 32 bits
+  return __funnelshift_rc(top, 0u, 1054u - (hi >> 20));            // (0: shifted out)
+}
+template <int MODE>
+__device__ __forceinline__ Tot<MODE> total(double x) {
+  if constexpr ((MODE & TOTALS) != 0) return whole_of(x);
+  else return x;
+}
+__device__ __forceinline__ float rounded(double x) { return __double2float_rn(x); }
+__device__ __forceinline__ float rounded(uint32_t x) { return __uint2float_rn(x); }
+// gain_of() of whole totals, beside the one of FP64 totals.
+using lvg::gain_of;
+__device__ __forceinline__ float gain_of(float kc, float kd, uint32_t wu, float wuf, uint32_t tc, uint32_t td, float kr) {
+  const float c = __int2float_rn(int(wu + tc - td));
+  return __fsub_rn(__fsub_rn(kc, kd), __fmul_rn(__fmul_rn(wuf, c), kr));
+}
+template <int MODE>
+using Sum = typename std::conditional<(MODE & 3) == FLOATS, float, uint32_t>::type;
 __device__ __forceinline__ uint32_t bits(float x) { return __float_as_uint(x); }
 __device__ __forceinline__ uint32_t bits(uint32_t x) { return x; }
 template <int MODE>
 __device__ __forceinline__ Sum<MODE> of_bits(uint32_t x) {
-  if constexpr (MODE == FLOATS) return __uint_as_float(x);
+  if constexpr ((MODE & 3) == FLOATS) return __uint_as_float(x);
   else return x;
 }
 // Weight of edge i.
 template <int MODE>
 __device__ __forceinline__ Sum<MODE> weight(const PhaseArgs &a, uint64_t i) {
-  if constexpr (MODE == FLOATS) return __ldcs(a.w + i);
-  else if constexpr (MODE == WHOLE) return __float2uint_rn(__ldcs(a.w + i));
+  if constexpr ((MODE & 3) == FLOATS) return __ldcs(a.w + i);
+  else if constexpr ((MODE & 3) == WHOLE) return __float2uint_rn(__ldcs(a.w + i));
   else return 1u;
 }
 
@@ -294,12 +324,12 @@ __device__ __forceinline__ void mark_row(const PhaseArgs &a, uint32_t u, uint64_
 
 // One thread: vertex u of community d leaves for c.
 template <bool SYNC>
-__device__ __forceinline__ void commit(const PhaseArgs &a, Shared &S, uint2 *mv, uint32_t u, uint32_t d, uint32_t c,
-                                       double wu) {
+__device__ __forceinline__ void commit(const PhaseArgs &a, Shared &S, uint2 *mv, uint32_t u, uint32_t d, uint32_t c) {
   const uint32_t i = atomicAdd(&S.nmv, 1u);
   if constexpr (SYNC) {
     mv[i] = make_uint2(u, c);
   } else {
+    const double wu = a.vtot[u];
     atomicAdd(&a.ctot[d], -wu);
     atomicAdd(&a.ctot[c], wu);
     a.vcom[u] = c;
@@ -322,7 +352,7 @@ __device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uin
   const uint32_t tl = lane & (T - 1);
   const unsigned tmask = (T == 32 ? 0xffffffffu : ((1u << T) - 1u) << (lane & ~(T - 1)));
   uint32_t u[N], dg[N], d[N], v[N], c[N];
-  double wu[N], td[N];
+  Tot<MODE> wu[N], td[N];
   V w[N];
 #pragma unroll
   for (int r = 0; r < N; ++r) {
@@ -333,14 +363,14 @@ __device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uin
   for (int r = 0; r < N; ++r) {
     dg[r] = 0;
     d[r] = EMPTY;
-    wu[r] = 0.0;
+    wu[r] = 0;
     v[r] = u[r];
     w[r] = 0;
     if (u[r] != EMPTY) {
       const uint64_t o = a.off[u[r]];
       dg[r] = a.deg[u[r]];
       d[r] = a.vcom[u[r]];
-      wu[r] = a.vtot[u[r]];
+      wu[r] = total<MODE>(a.vtot[u[r]]);
       if (tl < dg[r]) {
         v[r] = __ldcs(a.key + o + tl);
         w[r] = weight<MODE>(a, o + tl);
@@ -350,10 +380,10 @@ __device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uin
 #pragma unroll
   for (int r = 0; r < N; ++r) {
     c[r] = v[r] != u[r] ? live<SYNC>(a.vcom + v[r]) : EMPTY;
-    td[r] = u[r] != EMPTY ? live<SYNC>(a.ctot + d[r]) : 0.0;
+    td[r] = total<MODE>(u[r] != EMPTY ? live<SYNC>(a.ctot + d[r]) : 0.0);
   }
   V kc[N], kd[N];
-  double tc[N];
+  Tot<MODE> tc[N];
   unsigned lead = 0;
 #pragma unroll
   for (int r = 0; r < N; ++r) {
@@ -365,8 +395,8 @@ __device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uin
     const unsigned grp = __match_any_sync(0xffffffffu, c[r]) & tmask;
     const bool is = c[r] != EMPTY && (grp & ((1u << lane) - 1u)) == 0u;
     lead |= unsigned(is) << r;
-    tc[r] = is ? live<SYNC>(a.ctot + c[r]) : 0.0;
-    if constexpr (MODE == UNIT) {
+    tc[r] = total<MODE>(is ? live<SYNC>(a.ctot + c[r]) : 0.0);
+    if constexpr ((MODE & 3) == UNIT) {
       kc[r] = __popc(grp);
       kd[r] = __popc(__ballot_sync(0xffffffffu, kd[r] != 0u) & tmask);
     } else {
@@ -380,7 +410,7 @@ __device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uin
     float bg = 0.f;
     uint32_t bc = EMPTY;
     if ((lead >> r) & 1u) {
-      const float g = gain_of(float(kc[r]), float(kd[r]), wu[r], __double2float_rn(wu[r]), tc[r], td[r], G.kr);
+      const float g = gain_of(float(kc[r]), float(kd[r]), wu[r], rounded(wu[r]), tc[r], td[r], G.kr);
       if (g > 0.f) { bg = g; bc = c[r]; }
     }
     for (uint32_t sh = T >> 1; sh; sh >>= 1) {
@@ -391,7 +421,7 @@ __device__ __forceinline__ void tile_vertices(const PhaseArgs &a, Shared &S, uin
     const bool moved = bc != EMPTY && bc != G.zero;
     if (u[r] != EMPTY && tl == 0) {
       if (bc != EMPTY) add_gain(a, fix, G, bg);
-      if (moved) commit<SYNC>(a, S, mv, u[r], d[r], bc, wu[r]);
+      if (moved) commit<SYNC>(a, S, mv, u[r], d[r], bc);
       atomicAdd(&S.edges[bin], dg[r]);
     }
     if constexpr (!SYNC) {
@@ -427,8 +457,8 @@ __device__ __forceinline__ Sum<MODE> scan_row(const PhaseArgs &a, Shared &S, uin
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       if (c[k] == d) { kd += w[k]; c[k] = EMPTY; }
-      if constexpr (MODE == FLOATS) fine &= add_warp(keys, vals, lg, c[k], w[k], lane);
-      else if (c[k] != EMPTY) fine &= add<V>(keys, vals, lg, c[k], MODE == UNIT ? 1u : w[k]);
+      if constexpr ((MODE & 3) == FLOATS) fine &= add_warp(keys, vals, lg, c[k], w[k], lane);
+      else if (c[k] != EMPTY) fine &= add<V>(keys, vals, lg, c[k], (MODE & 3) == UNIT ? 1u : w[k]);
     }
   }
   if (!fine) S.bad = 1;  // (a table has twice as many slots as neighbours)
@@ -462,18 +492,18 @@ __device__ __forceinline__ void group_best(Shared &S, float bg, uint32_t n, uint
 template <bool SYNC, int MODE>
 __device__ __forceinline__ void best_of_table(const PhaseArgs &a, Shared &S, const uint32_t *keys, const uint32_t *vals,
                                               uint32_t slots, uint32_t t, uint32_t n, uint32_t id, int w0, float kd,
-                                              double wu, double td, float kr, uint32_t &gb, uint32_t &bc) {
-  const float wuf = __double2float_rn(wu);
+                                              Tot<MODE> wu, Tot<MODE> td, float kr, uint32_t &gb, uint32_t &bc) {
+  const float wuf = rounded(wu);
   float bg = 0.f;
   bc = EMPTY;
   constexpr int U = 4;
   for (uint32_t s = t; s < slots; s += U * n) {
     uint32_t c[U];
-    double tc[U];
+    Tot<MODE> tc[U];
 #pragma unroll
     for (int k = 0; k < U; ++k) c[k] = s + k * n < slots ? keys[s + k * n] : EMPTY;
 #pragma unroll
-    for (int k = 0; k < U; ++k) tc[k] = c[k] != EMPTY ? live<SYNC>(a.ctot + c[k]) : 0.0;
+    for (int k = 0; k < U; ++k) tc[k] = total<MODE>(c[k] != EMPTY ? live<SYNC>(a.ctot + c[k]) : 0.0);
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       if (c[k] == EMPTY) continue;
@@ -496,7 +526,7 @@ __device__ __forceinline__ void group_vertex(const PhaseArgs &a, Shared &S, uint
   const uint64_t o = a.off[u];
   const uint32_t dg = a.deg[u];
   const uint32_t d = a.vcom[u];
-  const double wu = a.vtot[u], td = live<SYNC>(a.ctot + d);
+  const Tot<MODE> wu = total<MODE>(a.vtot[u]), td = total<MODE>(live<SYNC>(a.ctot + d));
   const Of G(a, u);
   const uint32_t lg = min(lgmax, uint32_t(ceil_log2(2ull * dg)));
   uint32_t *keys = table, *vals = table + (1u << lg);
@@ -512,7 +542,7 @@ __device__ __forceinline__ void group_vertex(const PhaseArgs &a, Shared &S, uint
   const bool moved = bc != EMPTY && bc != G.zero;
   if (t == 0) {
     if (bc != EMPTY) add_gain(a, fix, G, __uint_as_float(gb));
-    if (moved) commit<SYNC>(a, S, mv, u, d, bc, wu);
+    if (moved) commit<SYNC>(a, S, mv, u, d, bc);
     atomicAdd(&S.edges[bin], dg);
   }
   if constexpr (!SYNC) {
@@ -725,7 +755,7 @@ __device__ __forceinline__ void hub_merge(const PhaseArgs &a, Shared &S, uint2 t
   uint32_t *keys = table, *vals = table + slots;
   for (uint32_t s = threadIdx.x; s < slots; s += PB) { keys[s] = EMPTY; vals[s] = 0u; }
   const uint32_t d = a.vcom[u];
-  const double wu = a.vtot[u], td = live<SYNC>(a.ctot + d);
+  const Tot<MODE> wu = total<MODE>(a.vtot[u]), td = total<MODE>(live<SYNC>(a.ctot + d));
   const V kd = of_bits<MODE>(__float_as_uint(a.hub_kd[u]));
   const Of G(a, u);
   __syncthreads();
@@ -788,8 +818,9 @@ __device__ __forceinline__ void hub_merge(const PhaseArgs &a, Shared &S, uint2 t
         if constexpr (SYNC) {
           a.hub_from[h] = d;
         } else {
-          atomicAdd(&a.ctot[d], -wu);
-          atomicAdd(&a.ctot[bc], wu);
+          const double x = a.vtot[u];
+          atomicAdd(&a.ctot[d], -x);
+          atomicAdd(&a.ctot[bc], x);
           a.vcom[u] = bc;
         }
       }
@@ -1151,15 +1182,17 @@ uint32_t phase_list_cap(const Level &lv, uint32_t grid) {
   return uint32_t(cap);
 }
 
-void launch_phase(bool sync, bool unit, bool whole, uint32_t grid, const PhaseArgs &a, cudaStream_t s) {
+void launch_phase(bool sync, bool unit, bool whole, bool totals, uint32_t grid, const PhaseArgs &a, cudaStream_t s) {
+  const int mode = unit ? UNIT : whole ? WHOLE : FLOATS;
+  const bool t = totals && mode != FLOATS;
   if (sync) {
-    if (unit) launch<true, UNIT>(grid, a, s);
-    else if (whole) launch<true, WHOLE>(grid, a, s);
-    else launch<true, FLOATS>(grid, a, s);
+    if (mode == FLOATS) launch<true, FLOATS>(grid, a, s);
+    else if (mode == UNIT) t ? launch<true, UNIT | TOTALS>(grid, a, s) : launch<true, UNIT>(grid, a, s);
+    else t ? launch<true, WHOLE | TOTALS>(grid, a, s) : launch<true, WHOLE>(grid, a, s);
   } else {
-    if (unit) launch<false, UNIT>(grid, a, s);
-    else if (whole) launch<false, WHOLE>(grid, a, s);
-    else launch<false, FLOATS>(grid, a, s);
+    if (mode == FLOATS) launch<false, FLOATS>(grid, a, s);
+    else if (mode == UNIT) t ? launch<false, UNIT | TOTALS>(grid, a, s) : launch<false, UNIT>(grid, a, s);
+    else t ? launch<false, WHOLE | TOTALS>(grid, a, s) : launch<false, WHOLE>(grid, a, s);
   }
 }
 

@@ -72,3 +72,26 @@ def test_every_degree_group_matches_cpu_replay(cuda, orc, lvg, edges, weights, c
     assert np.array_equal(r.membership, s.membership) and np.array_equal(r.communityWeight, s.communityWeight)
     for k in ("move_vertices", "move_edges", "moves", "move_bin_vertices", "move_bin_edges"):
         assert st[k] == H.stats()[k], k
+
+
+@pytest.mark.parametrize("scale", [1, 2])
+def test_totals_around_2_31(cuda, lvg, scale):
+    """Whole weights whose total lies below 2^31 (gains from integer totals) and
+    above (FP64), with community totals beyond FP32's 2^24: the launch-by-launch
+    path's FP64 totals, bit for bit. One pass: its FP32 sums per vertex and
+    community stay below 2^24, exact in any order."""
+    x = lvg.planted_partition(4096, 256, 256, 0.5, 3)
+    u = np.repeat(np.arange(x.span), np.diff(x.offsets).astype(np.int64))
+    x.weights[:] = scale * (1500 + (np.minimum(u, x.keys) * 7919 + np.maximum(u, x.keys) * 104729) % 1000)
+    total = x.weights.astype(np.float64).sum()
+    assert 2 ** 30 < total / scale < 2 ** 31 and (total >= 2 ** 31) == (scale == 2)
+    out = []
+    for graphs in (0, 1):
+        g = cuda.Graph(x)
+        cuda.set_tuning(g, level_graphs=graphs)
+        r = cuda.louvain_static(g, cuda.LouvainOptions(deterministic=True, maxPasses=1))
+        assert (g.stats()["level_graphs"] > 0) == bool(graphs)
+        out.append(r)
+    assert out[1].communityWeight.max() > 2 ** 24
+    for f in ("membership", "vertexWeight", "communityWeight"):
+        assert np.array_equal(getattr(out[0], f), getattr(out[1], f))
