@@ -526,7 +526,6 @@ int lvg_graph_trim(lvg_graph *g, int level) {
     g->u_tmp.release();
     g->u_rows.release();
     g->u_plan.release();
-    g->u_wdelta.release();
     // the host calls' hub-table caches (rebuilt by the next call that needs them)
     auto drop = [](lvg::HubTables &t) {
       t.off.release(); t.lg.release(); t.bad.release(); t.key.release(); t.cnt.release(); t.nbad.release();

@@ -1814,6 +1814,23 @@ PlanCounts plan_device(lvg_graph *g, const uint32_t *ds, const uint32_t *dd, con
   cudaStream_t s = g->stream;
   const size_t S = g->base.span, n = std::max(nd, ni);
   const int b = id_bits(S);
+  if (nd + ni > 0 && n <= PLAN_SMALL && b <= PLAN_SMALL_ID) {  // in one block
+    g->u_ds.ensure(nd); g->u_dd.ensure(nd); g->u_dw.ensure(nd);
+    g->u_is.ensure(ni); g->u_id.ensure(ni); g->u_iw.ensure(ni);
+    g->u_rows.ensure(std::min(S, nd + ni));
+    g->u_cnt.ensure(4);
+    g->hcnt.ensure(4);
+    launch_plan_small(ds, dd, dw, nd, is, id, iw, ni, g->u_ds.p, g->u_dd.p, g->u_dw.p, g->u_is.p, g->u_id.p,
+                      g->u_iw.p, g->u_rows.p, g->u_cnt.p, s);
+    LVG_CUDA(cudaMemcpyAsync(g->hcnt.p, g->u_cnt.p, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    LVG_CUDA(cudaStreamSynchronize(s));
+    PlanCounts c;
+    c.nd = g->hcnt.p[0];
+    c.ni = g->hcnt.p[1];
+    c.nrows = g->hcnt.p[2];
+    c.max_group = g->hcnt.p[3];
+    return c;
+  }
   g->u_k0.ensure(n); g->u_k1.ensure(n); g->u_v0.ensure(n); g->u_v1.ensure(n);
   g->u_flag.ensure(n + 1); g->u_pos.ensure(n + 1); g->u_pscan.ensure(scan_scratch_elems(n + 1));
   g->u_ds.ensure(nd); g->u_dd.ensure(nd); g->u_dw.ensure(nd);
@@ -1888,8 +1905,9 @@ void relayout(lvg_graph *g, size_t need) {
 
 // Tidy and apply a planned batch (plan_device's lists and rows). The kept
 // flags of the tidied batch are left in g->u_keep (deletions, then
-// insertions).
-void apply_plan(lvg_graph *g, const PlanCounts &pc) {
+// insertions); `tidied` (if given) is called when they are on their way, to
+// enqueue work behind them before the host waits for the new degree bins.
+void apply_plan(lvg_graph *g, const PlanCounts &pc, const std::function<void()> &tidied) {
   const UpdRow *rows = g->u_rows.p;
   const size_t nrows = pc.nrows, nd = pc.nd, ni = pc.ni;
   const uint32_t *dd = g->u_dd.p, *id = g->u_id.p;
@@ -1904,34 +1922,35 @@ void apply_plan(lvg_graph *g, const PlanCounts &pc) {
   g->u_len.ensure(nrows); g->u_src.ensure(nrows); g->u_grow.ensure(nrows);
   g->u_spos.ensure(nrows + 1); g->u_srcpos.ensure(nrows + 1); g->u_gpos.ensure(nrows + 1);
   g->u_scan.ensure(scan_scratch_elems(nrows + 1));
-  g->u_wdelta.ensure(1);
   uint8_t *ex = b.ex ? g->ex.p : nullptr;
   uint64_t T = 0, SRC = 0, GROW = 0;
   for (int attempt = 0;; ++attempt) {
     LVG_CUDA(cudaMemsetAsync(g->upd.p, 0, UPD_SLOTS * sizeof(uint64_t), s));
-    LVG_CUDA(cudaMemsetAsync(g->u_wdelta.p, 0, sizeof(double), s));
     launch_row_plan(g->off.p, g->deg.p, g->cap.p, g->key.p, g->w.p, rows, nrows, dd, id, iw, nd, g->u_pre.p,
-                    g->u_keep.p, g->u_plan.p, g->u_len.p, g->u_src.p, g->u_grow.p, ex, g->upd.p, g->u_wdelta.p, s);
-    exclusive_scan_u64(g->u_len.p, g->u_spos.p, nrows, g->u_spos.p + nrows, g->u_scan.p, s);
-    exclusive_scan_u64(g->u_src.p, g->u_srcpos.p, nrows, g->u_srcpos.p + nrows, g->u_scan.p, s);
-    exclusive_scan_u64(g->u_grow.p, g->u_gpos.p, nrows, g->u_gpos.p + nrows, g->u_scan.p, s);
+                    g->u_keep.p, g->u_plan.p, g->u_len.p, g->u_src.p, g->u_grow.p, ex, g->upd.p,
+                    reinterpret_cast<double *>(g->upd.p + UPD_WEIGHT), s);
+    if (nrows <= ROWS_SMALL) {
+      launch_row_scans_small(g->u_len.p, g->u_src.p, g->u_grow.p, nrows, g->u_spos.p, g->u_srcpos.p, g->u_gpos.p,
+                             g->upd.p, s);
+    } else {
+      auto sum = [&](int i) { return reinterpret_cast<uint64_t *>(g->upd.p + i); };
+      exclusive_scan_u64(g->u_len.p, g->u_spos.p, nrows, sum(UPD_ENTRIES), g->u_scan.p, s);
+      exclusive_scan_u64(g->u_src.p, g->u_srcpos.p, nrows, sum(UPD_SOURCE), g->u_scan.p, s);
+      exclusive_scan_u64(g->u_grow.p, g->u_gpos.p, nrows, sum(UPD_GROW), g->u_scan.p, s);
+    }
     unsigned long long *h = g->hupd.p;
     LVG_CUDA(cudaMemcpyAsync(h, g->upd.p, UPD_SLOTS * sizeof(uint64_t), cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaMemcpyAsync(h + 3, g->u_spos.p + nrows, 8, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaMemcpyAsync(h + 4, g->u_srcpos.p + nrows, 8, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaMemcpyAsync(h + 5, g->u_gpos.p + nrows, 8, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaMemcpyAsync(h + 6, g->u_wdelta.p, 8, cudaMemcpyDeviceToHost, s));
     LVG_CUDA(cudaStreamSynchronize(s));
-    T = h[3];
-    SRC = h[4];
-    GROW = h[5];
+    T = h[UPD_ENTRIES];
+    SRC = h[UPD_SOURCE];
+    GROW = h[UPD_GROW];
     if (g->slots - g->pool_cursor >= GROW) break;
     if (attempt) throw Error(LVG_ECUDA, "batch apply: the re-laid-out pool is too small (internal sizing error)");
     relayout(g, GROW);  // fresh capacities: plan again
   }
   const long long edge_delta = (long long)g->hupd.p[UPD_EDGES];
   double wdelta;
-  std::memcpy(&wdelta, &g->hupd.p[6], sizeof(double));
+  std::memcpy(&wdelta, &g->hupd.p[UPD_WEIGHT], sizeof(double));
   g->u_skey.ensure(T);
   g->u_sw.ensure(T);
   const uint64_t pool = g->pool_cursor;
@@ -1943,7 +1962,8 @@ void apply_plan(lvg_graph *g, const PlanCounts &pc) {
                      g->u_gpos.p, pool, s);
   g->pool_cursor += GROW;
   static_assert(offsetof(Counters, nonwhole) == offsetof(Counters, nonunit) + sizeof(unsigned long long), "");
-  if (b.whole && ni) {  // an insertion of another weight ends the unit-weight (whole-weight) fast path
+  const bool whole = b.whole;
+  if (whole && ni) {  // an insertion of another weight ends the unit-weight (whole-weight) fast path
     LVG_CUDA(cudaMemsetAsync(&g->ctr.p->nonunit, 0, 2 * sizeof(unsigned long long), s));
     launch_count_nonunit(iw, ni, g->ctr.p, s);
     LVG_CUDA(cudaMemcpyAsync(&g->hctr.p->nonunit, &g->ctr.p->nonunit, 2 * sizeof(unsigned long long),
@@ -1953,13 +1973,8 @@ void apply_plan(lvg_graph *g, const PlanCounts &pc) {
     launch_count_present(ex, b.span, g->upd.p, s);
     LVG_CUDA(cudaMemcpyAsync(g->hupd.p + UPD_ORDER, g->upd.p + UPD_ORDER, 8, cudaMemcpyDeviceToHost, s));
   }
-  LVG_CUDA(cudaStreamSynchronize(s));
-  if (b.whole && ni) {
-    b.unit = b.unit && !g->hctr.p->nonunit;
-    b.whole = !g->hctr.p->nonwhole;
-  }
+  if (tidied) tidied();
   b.edges = size_t((long long)b.edges + edge_delta);
-  if (ex) b.order = g->hupd.p[UPD_ORDER];
   g->total_weight += wdelta;
   // degrees changed: new bins and hub plan; the captured iteration is stale
   drop_graphs(g);
@@ -1969,6 +1984,11 @@ void apply_plan(lvg_graph *g, const PlanCounts &pc) {
   // and allocated again) on every apply
   if (b.edges > g->ws->X) g->ws->allocate(b.span, b.edges + b.edges / 16, s);
   compute_bins(g, b, g->deg.p, g->bins.p, g->ws->binscratch.p, b.colors);  // synchronises
+  if (whole && ni) {
+    b.unit = b.unit && !g->hctr.p->nonunit;
+    b.whole = !g->hctr.p->nonwhole;
+  }
+  if (ex) b.order = g->hupd.p[UPD_ORDER];
   build_hub_plan(g, b, g->hubplan);
 }
 
@@ -1984,21 +2004,27 @@ PlanCounts tidy_apply(lvg_graph *g, const uint32_t *ds, const uint32_t *dd, cons
   if (nd > 0x7FFFFFFFull || ni > 0x7FFFFFFFull) throw Error(LVG_EINVAL, "batch apply: more than 2^31-1 entries");
   cudaStream_t s = g->stream;
   PlanCounts pc = plan_device(g, ds, dd, dw, nd, is, id, iw, ni);
-  apply_plan(g, pc);
   const size_t n = pc.nd + pc.ni;
   PlanCounts out;
   out.max_group = pc.max_group;
-  if (n && pc.nrows) {
+  apply_plan(g, pc, [&] {
+    g->hcnt.ensure(4);
+    if (n <= ROWS_SMALL) {
+      launch_tidy_small(g->u_ds.p, g->u_dd.p, g->u_dw.p, pc.nd, g->u_is.p, g->u_id.p, g->u_iw.p, pc.ni, g->u_keep.p,
+                        tds, tdd, tdw, tis, tid, tiw, g->u_cnt.p, s);
+      LVG_CUDA(cudaMemcpyAsync(g->hcnt.p, g->u_cnt.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      return;
+    }
     g->u_pos.ensure(n + 1);
     g->u_pscan.ensure(scan_scratch_elems(n + 1));
     exclusive_scan_u32(g->u_keep.p, g->u_pos.p, n, g->u_pos.p + n, g->u_pscan.p, s);
     launch_tidy_compact(g->u_ds.p, g->u_dd.p, g->u_dw.p, pc.nd, g->u_keep.p, g->u_pos.p, nullptr, tds, tdd, tdw, s);
     launch_tidy_compact(g->u_is.p, g->u_id.p, g->u_iw.p, pc.ni, g->u_keep.p + pc.nd, g->u_pos.p + pc.nd,
                         g->u_pos.p + pc.nd, tis, tid, tiw, s);
-    g->hcnt.ensure(4);
     LVG_CUDA(cudaMemcpyAsync(g->hcnt.p, g->u_pos.p + pc.nd, 4, cudaMemcpyDeviceToHost, s));
     LVG_CUDA(cudaMemcpyAsync(g->hcnt.p + 1, g->u_pos.p + n, 4, cudaMemcpyDeviceToHost, s));
-    LVG_CUDA(cudaStreamSynchronize(s));
+  });
+  if (pc.nrows) {  // (apply_plan has waited)
     out.nd = g->hcnt.p[0];
     out.ni = g->hcnt.p[1] - g->hcnt.p[0];
   }

@@ -313,7 +313,6 @@ struct lvg_graph {
   DBuf<UpdRow> u_rows;
   DBuf<uint64_t> u_len, u_src, u_grow, u_spos, u_srcpos, u_gpos, u_scan, u_k0, u_k1;
   DBuf<RowPlan> u_plan;
-  DBuf<double> u_wdelta;
   DBuf<uint32_t> u_skey, u_pre, u_keep, u_pos, u_pscan, u_v0, u_v1, u_flag, u_touch, u_tpos, u_tscan;
   DBuf<uint32_t> u_cnt;
   DBuf<uint32_t> u_ds, u_dd, u_is, u_id;

@@ -578,7 +578,11 @@ __host__ __device__ inline uint32_t row_capacity(uint32_t d) { return d + (d >> 
 constexpr int UPD_EDGES = 0;  // change of the edge count (two's complement)
 constexpr int UPD_ORDER = 1;  // present vertices after the batch
 constexpr int UPD_MAXG = 2;   // longest run of insertions sharing a source
-constexpr int UPD_SLOTS = 3;
+constexpr int UPD_ENTRIES = 3;  // entries of the touched rows to rewrite
+constexpr int UPD_SOURCE = 4;   // source items of the touched rows
+constexpr int UPD_GROW = 5;     // pool entries the touched rows take
+constexpr int UPD_WEIGHT = 6;   // change of the total weight (FP64)
+constexpr int UPD_SLOTS = 7;
 void launch_row_caps(const uint64_t *coff, size_t n, uint32_t *deg, uint32_t *cap, uint64_t *cap64, cudaStream_t s);
 void launch_spread_rows(const uint64_t *coff, const uint32_t *ckey, const float *cw, size_t n, const uint64_t *off,
                         const uint32_t *cap, uint32_t *key, float *w, cudaStream_t s);
@@ -619,6 +623,24 @@ void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t
 void launch_plan_rows(const uint32_t *ds, const uint32_t *nd, const uint32_t *is, const uint32_t *ni, size_t cap,
                       uint32_t *flag, uint32_t *pos, uint32_t *scan, UpdRow *rows, unsigned long long *upd,
                       uint32_t *nrows, cudaStream_t s);
+
+// The steps of a small batch in one block each (a batch of a few hundred
+// entries is launch after launch of a few microseconds otherwise): the whole
+// plan of up to PLAN_SMALL deletions and insertions whose ids fit PLAN_SMALL_ID
+// bits; the three scans of up to ROWS_SMALL touched rows, with their sums in
+// upd[UPD_ENTRIES..UPD_GROW]; the tidied lists of up to ROWS_SMALL entries.
+constexpr size_t PLAN_SMALL = 2048, ROWS_SMALL = 4096;
+constexpr int PLAN_SMALL_ID = 26;
+void launch_plan_small(const uint32_t *ds, const uint32_t *dd, const float *dw, size_t nd, const uint32_t *is,
+                       const uint32_t *id, const float *iw, size_t ni, uint32_t *ods, uint32_t *odd, float *odw,
+                       uint32_t *ois, uint32_t *oid, float *oiw, UpdRow *rows, uint32_t *cnt, cudaStream_t s);
+void launch_row_scans_small(const uint64_t *len, const uint64_t *src, const uint64_t *grow, size_t nrows,
+                            uint64_t *spos, uint64_t *srcpos, uint64_t *gpos, unsigned long long *upd,
+                            cudaStream_t s);
+void launch_tidy_small(const uint32_t *ds, const uint32_t *dd, const float *dw, size_t nd, const uint32_t *is,
+                       const uint32_t *id, const float *iw, size_t ni, const uint32_t *keep, uint32_t *tds,
+                       uint32_t *tdd, float *tdw, uint32_t *tis, uint32_t *tid, float *tiw, uint32_t *cnt,
+                       cudaStream_t s);
 
 // ---------------------------------------------------------------- generators (lvg_gen.cu)
 // Stable radix sorts of 64-bit keys over bits [0, end_bit) (cub); the result

@@ -497,6 +497,212 @@ __global__ void tidy_compact_kernel(const uint32_t *src, const uint32_t *dst, co
   }
 }
 
+// ---- the steps of a small batch, one block each
+
+constexpr int SB = 1024;  // threads
+constexpr int SI = 4;     // consecutive items a thread holds
+static_assert(SB * SI == 2 * PLAN_SMALL && SB * SI == ROWS_SMALL, "");
+
+// Exclusive prefix of x over the block's threads; the sum into *total. (All
+// threads; `part` holds 33 values and is free again after the call's barrier.)
+template <class T>
+__device__ __forceinline__ T block_prefix(T x, T *part, T *total) {
+  const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5;
+  T inc = x;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const T y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= uint32_t(o)) inc += y;
+  }
+  if (lane == 31) part[wid] = inc;
+  __syncthreads();
+  if (wid == 0) {
+    T p = part[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const T y = __shfl_up_sync(0xffffffffu, p, o);
+      if (lane >= uint32_t(o)) p += y;
+    }
+    part[lane] = p;
+  }
+  __syncthreads();
+  const T before = wid ? part[wid - 1] : T(0);
+  *total = part[31];
+  __syncthreads();
+  return before + inc - x;
+}
+
+// Both lists packed as (list, source, target, index) keys and sorted at once in
+// shared memory (a bitonic network), the first of each equal (list, source,
+// target) kept in batch order, and a row per source: what the passes above do
+// for large batches in thirteen launches (22 us for 1280 entries against 60 and
+// the gaps between them; with the two kernels below, half the host's waits and
+// fewer copies an applied and answered batch of 640 edges on a 1M-vertex graph
+// takes 367 us instead of 443). A list above PLAN_SMALL would leave the chip
+// idle behind one block for longer than the passes take. cnt: kept deletions and insertions,
+// rows, the longest insertion run.
+__global__ void __launch_bounds__(SB) plan_small_kernel(const uint32_t *ds, const uint32_t *dd, const float *dw,
+                                                        uint32_t nd, const uint32_t *is, const uint32_t *id,
+                                                        const float *iw, uint32_t ni, uint32_t n2, uint32_t *ods,
+                                                        uint32_t *odd, float *odw, uint32_t *ois, uint32_t *oid,
+                                                        float *oiw, UpdRow *rows, uint32_t *cnt) {
+  constexpr int IB = 11, KB = PLAN_SMALL_ID;  // bits of an index and of an id
+  static_assert((1u << IB) == PLAN_SMALL && 1 + 2 * KB + IB <= 64, "");
+  __shared__ __align__(16) unsigned long long key[SB * SI];
+  __shared__ uint32_t part[33];
+  __shared__ uint32_t run;
+  const uint32_t tid = threadIdx.x, n = nd + ni;
+  for (uint32_t e = tid; e < n2; e += SB) {
+    unsigned long long k = ~0ull;
+    if (e < nd) k = ((unsigned long long)ds[e] << KB | dd[e]) << IB | e;
+    else if (e < n) k = 1ull << (2 * KB + IB) | ((unsigned long long)is[e - nd] << KB | id[e - nd]) << IB | (e - nd);
+    key[e] = k;
+  }
+  if (tid == 0) run = 0;
+  __syncthreads();
+  for (uint32_t size = 2; size <= n2; size <<= 1)
+    for (uint32_t step = size >> 1; step > 0; step >>= 1) {
+      for (uint32_t t = tid; t < n2 / 2; t += SB) {
+        const uint32_t i = (t & ~(step - 1)) * 2 + (t & (step - 1)), j = i + step;
+        const unsigned long long a = key[i], b = key[j];
+        if ((a > b) == ((i & size) == 0)) { key[i] = b; key[j] = a; }
+      }
+      // (a warp's 32 pairs of a step up to 32 lie in its own 64 keys)
+      if (step > 32 || (step == 1 && size > 32)) __syncthreads();
+      else __syncwarp();
+    }
+  __syncthreads();
+  // the first of each run, four consecutive keys a thread
+  unsigned long long k[SI];
+  uint32_t first = 0, tot;
+#pragma unroll
+  for (int x = 0; x < SI; ++x) {
+    const uint32_t e = tid * SI + x;
+    k[x] = e < n ? key[e] : ~0ull;
+    if (e < n && (e == 0 || key[e - 1] >> IB != k[x] >> IB)) first |= 1u << x;
+  }
+  uint32_t at = block_prefix<uint32_t>(uint32_t(__popc(first)), part, &tot);  // (and key[] is read)
+  // kept deletions: those of list 0 (sorted first)
+  uint32_t dels = 0;
+#pragma unroll
+  for (int x = 0; x < SI; ++x) dels += (first >> x & 1u) && k[x] >> (2 * KB + IB) == 0;
+  uint32_t a;
+  block_prefix<uint32_t>(dels, part, &a);
+  uint32_t *src = reinterpret_cast<uint32_t *>(key), *pos = src + SB * SI;  // kept sources; the rows before each
+#pragma unroll
+  for (int x = 0; x < SI; ++x) {
+    if (!(first >> x & 1u)) continue;
+    const uint32_t u = uint32_t(k[x] >> (KB + IB)) & ((1u << KB) - 1u), v = uint32_t(k[x] >> IB) & ((1u << KB) - 1u);
+    const uint32_t i = uint32_t(k[x]) & ((1u << IB) - 1u);
+    src[at] = u;
+    if (at < a) { ods[at] = u; odd[at] = v; odw[at] = dw[i]; }
+    else { ois[at - a] = u; oid[at - a] = v; oiw[at - a] = iw[i]; }
+    ++at;
+  }
+  __syncthreads();
+  const uint32_t c = tot - a;
+  const uint32_t *us = src + a;  // the insertions' sources
+  uint32_t head = 0;
+#pragma unroll
+  for (int x = 0; x < SI; ++x) {
+    const uint32_t e = tid * SI + x;
+    if (e >= tot) continue;
+    bool h = e == 0 || e == a || src[e] != src[e - 1];
+    if (h && e >= a) {
+      const uint32_t p = lower_bound_u32(src, a, src[e]);
+      h = !(p < a && src[p] == src[e]);
+    }
+    if (h) head |= 1u << x;
+  }
+  uint32_t nrows;
+  uint32_t before = block_prefix<uint32_t>(uint32_t(__popc(head)), part, &nrows);
+  uint32_t b = before;
+#pragma unroll
+  for (int x = 0; x < SI; ++x) {
+    const uint32_t e = tid * SI + x;
+    if (e < tot) pos[e] = b;
+    b += head >> x & 1u;
+  }
+  __syncthreads();
+  const uint32_t drows = a < tot ? pos[a] : nrows;  // rows of sources with deletions
+#pragma unroll
+  for (int x = 0; x < SI; ++x) {
+    if (!(head >> x & 1u)) continue;
+    const uint32_t e = tid * SI + x;
+    const bool del = e < a;
+    UpdRow R;
+    R.u = src[e];
+    R.d0 = del ? e : lower_bound_u32(src, a, R.u);
+    R.d1 = del ? lower_bound_u32(src, a, R.u + 1) : R.d0;
+    R.i0 = del ? lower_bound_u32(us, c, R.u) : e - a;
+    R.i1 = lower_bound_u32(us, c, R.u + 1);
+    const uint32_t o = del ? R.i0 + a : R.d0;  // the other list's rows below
+    const uint32_t p = o < tot ? pos[o] : nrows;
+    rows[del ? pos[e] + (p - drows) : pos[e] - drows + p] = R;
+    if (R.i1 > R.i0) atomicMax(&run, R.i1 - R.i0);
+  }
+  __syncthreads();
+  if (tid == 0) { cnt[0] = a; cnt[1] = c; cnt[2] = nrows; cnt[3] = run; }
+}
+
+// The exclusive prefixes of the rows' rewritten entries, source items and pool
+// entries, and their sums.
+__global__ void __launch_bounds__(SB) row_scans_small_kernel(const uint64_t *len, const uint64_t *src,
+                                                             const uint64_t *grow, uint32_t nrows, uint64_t *spos,
+                                                             uint64_t *srcpos, uint64_t *gpos,
+                                                             unsigned long long *upd) {
+  __shared__ unsigned long long part[33];
+  const uint64_t *in[3] = {len, src, grow};
+  uint64_t *out[3] = {spos, srcpos, gpos};
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    unsigned long long x[SI], sum = 0, total;
+#pragma unroll
+    for (int i = 0; i < SI; ++i) {
+      const uint32_t e = threadIdx.x * SI + i;
+      x[i] = e < nrows ? in[q][e] : 0ull;
+      sum += x[i];
+    }
+    unsigned long long at = block_prefix<unsigned long long>(sum, part, &total);
+#pragma unroll
+    for (int i = 0; i < SI; ++i) {
+      const uint32_t e = threadIdx.x * SI + i;
+      if (e < nrows) out[q][e] = at;
+      at += x[i];
+    }
+    if (threadIdx.x == 0) upd[UPD_ENTRIES + q] = total;
+  }
+}
+
+// The kept entries of both lists, in order; cnt: kept deletions, kept entries.
+__global__ void __launch_bounds__(SB) tidy_small_kernel(const uint32_t *ds, const uint32_t *dd, const float *dw,
+                                                        uint32_t nd, const uint32_t *is, const uint32_t *id,
+                                                        const float *iw, uint32_t ni, const uint32_t *keep,
+                                                        uint32_t *tds, uint32_t *tdd, float *tdw, uint32_t *tis,
+                                                        uint32_t *tid, float *tiw, uint32_t *cnt) {
+  __shared__ uint32_t part[33];
+  uint32_t kept = 0, dels = 0, total, a;
+#pragma unroll
+  for (int i = 0; i < SI; ++i) {
+    const uint32_t e = threadIdx.x * SI + i;
+    if (e < nd + ni && keep[e]) {
+      kept |= 1u << i;
+      dels += e < nd;
+    }
+  }
+  uint32_t at = block_prefix<uint32_t>(uint32_t(__popc(kept)), part, &total);
+  block_prefix<uint32_t>(dels, part, &a);
+#pragma unroll
+  for (int i = 0; i < SI; ++i) {
+    if (!(kept >> i & 1u)) continue;
+    const uint32_t e = threadIdx.x * SI + i;
+    if (e < nd) { tds[at] = ds[e]; tdd[at] = dd[e]; tdw[at] = dw[e]; }
+    else { tis[at - a] = is[e - nd]; tid[at - a] = id[e - nd]; tiw[at - a] = iw[e - nd]; }
+    ++at;
+  }
+  if (threadIdx.x == 0) { cnt[0] = a; cnt[1] = total; }
+}
+
 // Copy every row into a new gapped layout (one warp per row; gaps zero).
 __global__ void relayout_kernel(const uint64_t *old_off, const uint32_t *deg, const uint32_t *old_key,
                                 const float *old_w, size_t n, const uint64_t *off, const uint32_t *cap,
@@ -613,6 +819,32 @@ void launch_plan_rows(const uint32_t *ds, const uint32_t *nd, const uint32_t *is
   LVG_CHECK_LAUNCH();
   exclusive_scan_u32(flag, pos, 2 * cap, pos + 2 * cap, scan, s);
   plan_rows_kernel<<<grid_for(2 * cap, 256), 256, 0, s>>>(flag, pos, cap, ds, nd, is, ni, rows, upd, nrows);
+  LVG_CHECK_LAUNCH();
+}
+
+void launch_plan_small(const uint32_t *ds, const uint32_t *dd, const float *dw, size_t nd, const uint32_t *is,
+                       const uint32_t *id, const float *iw, size_t ni, uint32_t *ods, uint32_t *odd, float *odw,
+                       uint32_t *ois, uint32_t *oid, float *oiw, UpdRow *rows, uint32_t *cnt, cudaStream_t s) {
+  uint32_t n2 = 64;
+  while (n2 < nd + ni) n2 *= 2;
+  plan_small_kernel<<<1, SB, 0, s>>>(ds, dd, dw, uint32_t(nd), is, id, iw, uint32_t(ni), n2, ods, odd, odw, ois, oid,
+                                     oiw, rows, cnt);
+  LVG_CHECK_LAUNCH();
+}
+
+void launch_row_scans_small(const uint64_t *len, const uint64_t *src, const uint64_t *grow, size_t nrows,
+                            uint64_t *spos, uint64_t *srcpos, uint64_t *gpos, unsigned long long *upd,
+                            cudaStream_t s) {
+  row_scans_small_kernel<<<1, SB, 0, s>>>(len, src, grow, uint32_t(nrows), spos, srcpos, gpos, upd);
+  LVG_CHECK_LAUNCH();
+}
+
+void launch_tidy_small(const uint32_t *ds, const uint32_t *dd, const float *dw, size_t nd, const uint32_t *is,
+                       const uint32_t *id, const float *iw, size_t ni, const uint32_t *keep, uint32_t *tds,
+                       uint32_t *tdd, float *tdw, uint32_t *tis, uint32_t *tid, float *tiw, uint32_t *cnt,
+                       cudaStream_t s) {
+  tidy_small_kernel<<<1, SB, 0, s>>>(ds, dd, dw, uint32_t(nd), is, id, iw, uint32_t(ni), keep, tds, tdd, tdw, tis, tid,
+                                     tiw, cnt);
   LVG_CHECK_LAUNCH();
 }
 
