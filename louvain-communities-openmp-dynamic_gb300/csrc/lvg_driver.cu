@@ -1336,11 +1336,11 @@ void run(lvg_graph *g, int method, const DBatch &b, StateRef prior, StateRef out
   info.iterations = l;
   info.passes = p;
   info.t /= rep; info.tm /= rep; info.ti /= rep; info.tp /= rep; info.tl /= rep; info.ta /= rep;
-  g->stats.move_vertices = g->hctr.p->vertices;
-  g->stats.move_edges = g->hctr.p->edges;
   g->stats.moves = g->hctr.p->moves;
   g->stats.aggregate_edges = g->hctr.p->agg_edges;
   for (int b = 0; b < NUM_BINS; ++b) {
+    g->stats.move_vertices += g->hctr.p->bin_vertices[b];
+    g->stats.move_edges += g->hctr.p->bin_edges[b];
     g->stats.move_bin_vertices[b] = g->hctr.p->bin_vertices[b];
     g->stats.move_bin_edges[b] = g->hctr.p->bin_edges[b];
     g->stats.move_bin_overflow[b] = g->hctr.p->bin_over[b];
@@ -1489,11 +1489,11 @@ void run_union(lvg_graph *g, const lvg_options &o, RunInfo &info) {
   LVG_CUDA(cudaMemcpyAsync(U.hctl.p, U.ctl.p, n * sizeof(GraphCtl), cudaMemcpyDeviceToHost, s));
   read_counters(g);
   info.t /= rep; info.tm /= rep; info.ti /= rep; info.tp /= rep; info.tl /= rep; info.ta /= rep;
-  g->stats.move_vertices = g->hctr.p->vertices;
-  g->stats.move_edges = g->hctr.p->edges;
   g->stats.moves = g->hctr.p->moves;
   g->stats.aggregate_edges = g->hctr.p->agg_edges;
   for (int b = 0; b < NUM_BINS; ++b) {
+    g->stats.move_vertices += g->hctr.p->bin_vertices[b];
+    g->stats.move_edges += g->hctr.p->bin_edges[b];
     g->stats.move_bin_vertices[b] = g->hctr.p->bin_vertices[b];
     g->stats.move_bin_edges[b] = g->hctr.p->bin_edges[b];
     g->stats.move_bin_overflow[b] = g->hctr.p->bin_over[b];

@@ -158,8 +158,6 @@ struct Level {
 // Device counters block (one allocation; mirrored in pinned host memory).
 struct Counters {
   unsigned long long el_fix;     // Σ best gains, 2^-16 fixed point
-  unsigned long long vertices;   // processed vertices
-  unsigned long long edges;      // scanned edges
   unsigned long long moves;      // moved vertices
   unsigned long long agg_edges;  // edges read by aggregation
   unsigned long long affected;   // residual affected flags

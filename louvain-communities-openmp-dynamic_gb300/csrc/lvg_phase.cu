@@ -1117,9 +1117,7 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
   }
   if (tid < NUM_BINS && S.sv[tid]) {
     atomicAdd(&a.ctr->bin_vertices[tid], S.sv[tid]);
-    atomicAdd(&a.ctr->vertices, S.sv[tid]);
     atomicAdd(&a.ctr->bin_edges[tid], S.se[tid]);
-    atomicAdd(&a.ctr->edges, S.se[tid]);
   }
   if (SYNC && MODE == UNIT && slots) atomicAdd(&a.ctr->ht_slots, slots);
   if (tid == 0) {
