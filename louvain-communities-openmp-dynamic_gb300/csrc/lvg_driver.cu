@@ -718,7 +718,7 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   if (g->profiling || !g->tuning.level_graphs || L <= 0) return false;
   // asynchronous runs keep resident hub tables by the launch-by-launch kernels
   // (deterministic ones here: the two phases of a 1e-4 |E| batch and its
-  // inverse on R-MAT scale 24 take 5.7 ms, by launches 12.5); a frontier run of
+  // inverse on R-MAT scale 24 take 3.7 ms, by launches 12.5); a frontier run of
   // one class starts from lists of its few marked vertices there
   if ((W.ht_now.key && !(sync && lv.unit)) || listed) return false;
   const HubPlan &P = lv.hub;
@@ -768,10 +768,29 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
     a.graphs = uint32_t(uc->n); a.gctl = uc->ctl; a.gM = uc->M; a.itcap = uc->L;
   }
   for (int i = 0; i <= lv.colors * NUM_BINS; ++i) a.start[i] = uint32_t(lv.bin_start[i]);
-  launch_fill_bytes(W.phase_ctl.p, 0, sizeof(PhaseCtl), s);
   // (a dynamic run's totals begin with the caller's, which can be any numbers)
-  const bool small = g->total_weight < 2147483648.0;
-  launch_phase(sync, lv.unit, lv.whole && small, !from_prior && small, grid, a, s);
+  const bool small = g->total_weight < 2147483648.0, totals = !from_prior && small && (lv.unit || lv.whole);
+  if (sync && !totals) {
+    size_t pieces = 0, n10 = 0, n9 = 0;
+    for (int k = 0; k < lv.colors; ++k) {
+      const size_t c10 = lv.bucket_size(k, 10), c9 = lv.bucket_size(k, 9);
+      pieces = std::max(pieces, 8 * c10 + 2 * c9);  // (of 1024 edges, up to degrees 8192 and 2048)
+      n10 = std::max(n10, c10);
+      n9 = std::max(n9, c9);
+    }
+    if (pieces) {
+      W.phase_big.ensure(pieces);
+      a.big = W.phase_big.p;
+    }
+    // with several vertices above degree 512 for each block, the blocks share them
+    if (n10 * 4 + n9 >= size_t(16) * grid) {
+      W.phase_heavy.ensure(n10 + n9);
+      a.heavy = W.phase_heavy.p;
+      a.heavy9 = uint32_t(n10);
+    }
+  }
+  launch_fill_bytes(W.phase_ctl.p, 0, sizeof(PhaseCtl), s);
+  launch_phase(sync, lv.unit, lv.whole && small, totals, grid, a, s);
   ++g->stats.move_launches;
   ++g->stats.level_graphs;
   LVG_CUDA(cudaMemcpyAsync(g->hctr.p, g->ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));

@@ -62,6 +62,8 @@ struct Workspace {
   // the phase kernel's shared words, and its blocks' lists when they are too
   // long for shared memory
   DBuf<PhaseCtl> phase_ctl;
+  DBuf<uint4> phase_big;         // phase kernel: the large movers of a class
+  DBuf<uint32_t> phase_heavy;    // and the large vertices its blocks share
   DBuf<uint2> phase_mv;
   DBuf<uint32_t> phase_list, hub_segs, hub_done, hub_move;
   // resident hub tables: build scratch, and the tables the first pass of the

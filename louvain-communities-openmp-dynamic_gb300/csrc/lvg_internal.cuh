@@ -213,38 +213,43 @@ __device__ __forceinline__ void ht_mark_bad(const HubTabView &t, uint32_t h) {
   t.bad[h] = 1;
 }
 
-// Hub v's table after a neighbour moved from community `from` to `to` (a no-op
-// when v is not a hub or its table is marked bad). `from` is present: it is
-// the neighbour's community, counted when the table was built or when the
-// neighbour moved in. A table without room for `to` is marked bad.
-__device__ __forceinline__ void ht_move(const HubTabView &t, uint32_t v, uint32_t from, uint32_t to, Counters *ctr) {
-  const uint32_t h = t.slot[v];
-  if (h == NO_HUB || t.bad[h]) return;
+// Hub h's table (a no-op when it is marked bad) after a neighbour moved from
+// community `from` to `to`. `from` is present: it is the neighbour's community,
+// counted when the table was built or when the neighbour moved in. A table
+// without room for `to` is marked bad. The first slots of both are fetched
+// together: what this costs is the chain of loads.
+__device__ __forceinline__ void ht_move_at(const HubTabView &t, uint32_t h, uint32_t from, uint32_t to, Counters *ctr) {
   const uint64_t o = t.off[h];
   const int lg = t.lg[h];
+  if (t.bad[h]) return;
   const uint32_t mask = (1u << lg) - 1u;
   bool found = false, placed = false;
-  uint32_t s = hash_hi(from, lg);
+  uint32_t s = hash_hi(from, lg), s2 = hash_hi(to, lg);
+  uint32_t k = ld_relaxed(t.key + o + s), k2 = ld_relaxed(t.key + o + s2);
   for (uint32_t p = 0; p <= mask; ++p) {
-    const uint32_t k = ld_relaxed(t.key + o + s);
     if (k == from) { atomicSub(t.cnt + o + s, 1u); found = true; break; }
     if (k == EMPTY) break;
     s = (s + 1u) & mask;
+    k = ld_relaxed(t.key + o + s);
   }
-  s = hash_hi(to, lg);
   for (uint32_t p = 0; p <= mask; ++p) {
-    uint32_t k = ld_relaxed(t.key + o + s);
-    if (k == EMPTY) {
-      k = atomicCAS(t.key + o + s, EMPTY, to);
-      if (k == EMPTY) k = to;
+    if (k2 == EMPTY) {
+      k2 = atomicCAS(t.key + o + s2, EMPTY, to);
+      if (k2 == EMPTY) k2 = to;
     }
-    if (k == to) { atomicAdd(t.cnt + o + s, 1u); placed = true; break; }
-    s = (s + 1u) & mask;
+    if (k2 == to) { atomicAdd(t.cnt + o + s2, 1u); placed = true; break; }
+    s2 = (s2 + 1u) & mask;
+    k2 = ld_relaxed(t.key + o + s2);
   }
   if (!found || !placed) {
     ht_mark_bad(t, h);
     atomicAdd(&ctr->ht_over, 1ull);
   }
+}
+// The same for neighbour v, when it is a hub.
+__device__ __forceinline__ void ht_move(const HubTabView &t, uint32_t v, uint32_t from, uint32_t to, Counters *ctr) {
+  const uint32_t h = t.slot[v];
+  if (h != NO_HUB) ht_move_at(t, h, from, to, ctr);
 }
 
 // Per-graph control of a graph-union run (lvg_static_union), on the device:
@@ -318,6 +323,9 @@ struct PhaseCtl {
   unsigned long long fix[3];      // an iteration's gain sum
   unsigned long long gactive[3];  // graph unions: graphs still moving
   unsigned long long aborted;     // a block gave a wait up
+  // deterministic mode, turns over class steps: row pieces of large movers,
+  // listed vertices of degree bins 10 and 9, and the shared queue's next unit
+  uint32_t pieces[3], heavy[3][2], queue[3];
 };
 
 // Arguments of the phase kernel: a level's whole local-moving phase.
@@ -350,6 +358,9 @@ struct PhaseArgs {
   float *hub_kd;                // [span]
   unsigned long long *hub_best; // [hubs] zero between uses, as hub_done
   uint32_t *hub_done, *hub_move, *hub_from;
+  uint4 *big;         // deterministic mode: (vertex, its old and new community, piece) of large movers
+  uint32_t *heavy;    // the vertices of bins 10 and 9 (from heavy9 on) of a class that blocks share, or nullptr
+  uint32_t heavy9;
   HubTabView ht;      // resident hub tables (deterministic mode, unit weights); key nullptr without
   // graph unions (nullptr for one graph), as MoveArgs
   const uint32_t *gid;

@@ -52,6 +52,7 @@ constexpr int PW = PB / 32;               // warps per block
 constexpr uint32_t LOG_BLOCK = 14;        // shared slots of a block's vertex (log2)
 constexpr uint32_t TABLE_WORDS = 2u << LOG_BLOCK;  // keys and values
 constexpr uint32_t LIST_CAP = 1920;       // listed vertices a block keeps in shared memory
+constexpr uint32_t PIECE = 1024;          // edges of a large mover's row marked at once
 constexpr uint32_t TODO = 256;            // hub chunks a block looks through at a time
 constexpr uint32_t MERGE_FULL = 8192;     // partial entries of a hub that one block merges at once
 // One wait of the grid barrier gives up after this many polls (seconds; a
@@ -107,6 +108,17 @@ __device__ __forceinline__ Sum<MODE> weight(const PhaseArgs &a, uint64_t i) {
   else return 1u;
 }
 
+// Deterministic runs that are not static ones of whole weights: a few marked
+// vertices a class, most of the work in large ones. Their blocks share the
+// vertices of degree bins 9 and 10 of a class through one list and the rows of
+// large movers in pieces; dealt out beforehand, the unluckiest block of a class
+// took 1.6 times the average to decide and 4 times to mark. (Two runs of a 1e-4
+// |E| batch on R-MAT scale 24: 5.7 -> 3.7 ms.) Static runs keep their own
+// shares: every block has many vertices, and the shared words cost small levels
+// 2-5 %.
+template <bool SYNC, int MODE>
+constexpr bool SHARES = SYNC && (MODE & TOTALS) == 0;
+
 struct Shared {
   uint32_t off[MAX_BUCKETS];   // [class][bin]: the block's first list slot of the bin
   uint32_t pos[MAX_BUCKETS];   // [class][bin]: the bin's first position dealt to the block
@@ -121,6 +133,8 @@ struct Shared {
   uint32_t hubmv;              // hubs moved by the block's merges
   uint32_t over, bad, stop;
   uint32_t ntodo, todo[TODO];  // hub chunks that have work
+  uint32_t turn;               // of the class step: the words of PhaseCtl's triples
+  uint32_t unit[2];            // the block's units of the shared queue
   uint32_t any;                // some block moved a vertex before the last barrier that counts moves
   unsigned long long sum;      // the iteration's gain sum, or the union's graphs still moving
 };
@@ -317,10 +331,50 @@ __device__ __forceinline__ void mark_row(const PhaseArgs &a, uint32_t u, uint64_
 #pragma unroll
       for (int k = 0; k < 4; ++k) h[k] = v[k] != u ? a.ht.slot[v[k]] : NO_HUB;
       for (int k = 0; k < 4; ++k)
-        if (h[k] != NO_HUB) ht_move(a.ht, v[k], d, c, a.ctr);
+        if (h[k] != NO_HUB) ht_move_at(a.ht, h[k], d, c, a.ctr);
     }
   }
 }
+// The same by whole warps (thread t of n, both multiples of 32 for lane 0): the
+// hubs among a warp's 128 neighbours are dealt to its lanes, since the
+// neighbours of a large vertex are often hubs and a lane with four of them
+// would update their tables one after the other.
+__device__ __forceinline__ void mark_row_warp(const PhaseArgs &a, uint32_t u, uint64_t o, uint32_t m, uint32_t t,
+                                              uint32_t n, bool tabs, uint32_t d, uint32_t c) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t j = t; j - lane < m; j += 4 * n) {
+    uint32_t v[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = j + k * n < m ? __ldcs(a.key + o + j + k * n) : u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (v[k] != u) a.vaff[v[k]] = 1;
+    if (tabs) {
+      uint32_t h[4], has[4], hits = 0;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) h[k] = v[k] != u ? a.ht.slot[v[k]] : NO_HUB;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        has[k] = __ballot_sync(0xffffffffu, h[k] != NO_HUB);
+        hits += __popc(has[k]);
+      }
+      for (uint32_t i = lane; i - lane < hits; i += 32) {
+        uint32_t mine = NO_HUB, before = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const uint32_t cnt = __popc(has[k]);
+          const bool in = i >= before && i < before + cnt;
+          const uint32_t x = __shfl_sync(0xffffffffu, h[k], in ? __fns(has[k], 0, int(i - before) + 1) : lane);
+          if (in) mine = x;
+          before += cnt;
+        }
+        if (mine != NO_HUB) ht_move_at(a.ht, mine, d, c, a.ctr);
+        __syncwarp();
+      }
+    }
+  }
+}
+
 
 // One thread: vertex u of community d leaves for c.
 template <bool SYNC>
@@ -542,7 +596,15 @@ __device__ __forceinline__ void group_vertex(const PhaseArgs &a, Shared &S, uint
   const bool moved = bc != EMPTY && bc != G.zero;
   if (t == 0) {
     if (bc != EMPTY) add_gain(a, fix, G, __uint_as_float(gb));
-    if (moved) commit<SYNC>(a, S, mv, u, d, bc);
+    if (moved) {
+      if (SHARES<SYNC, MODE> && bin >= 9) {  // its row is marked in pieces, by whichever blocks
+        const uint32_t n = (dg + PIECE - 1) / PIECE, at = atomicAdd(&a.ctl->pieces[S.turn], n);
+        for (uint32_t p = 0; p < n; ++p) a.big[at + p] = make_uint4(u, d, bc, p);
+        atomicAdd(&S.hubmv, 1u);
+      } else {
+        commit<SYNC>(a, S, mv, u, d, bc);
+      }
+    }
     atomicAdd(&S.edges[bin], dg);
   }
   if constexpr (!SYNC) {
@@ -866,13 +928,17 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
   unsigned long long fix = 0;  // the thread's share of the iteration's gain sum
   unsigned long long sum = 0, slots = 0;
   const bool tabs = SYNC && MODE == UNIT && a.ht.key;  // the hubs are decided from resident tables
-  uint32_t l = 0;
+  constexpr bool SHARE = SHARES<SYNC, MODE>;
+  uint32_t l = 0, step = 0;
   while (l < uint32_t(a.L)) {
     // what ends an iteration: its gain sum, or the graphs of the union still moving
     const unsigned long long *total = a.gfix ? &a.ctl->gactive[l % 3] : &a.ctl->fix[l % 3];
     for (int k = 0; k < K; ++k) {
       const bool last = k == K - 1;
       // ---- 1. the block's active vertices of the class, per bin
+      const uint32_t turn = SHARE ? step++ % 3 : 0u;
+      const bool shared = SHARE && a.heavy;  // bins 9 and 10 through a list of all blocks
+      if (SHARE && tid == 0) S.turn = turn;
       const uint32_t tot = S.tot[k];
       const uint32_t *off = S.off + k * NUM_BINS;
       for (uint32_t t0 = tid - lane; t0 < tot; t0 += PB) {
@@ -899,7 +965,13 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
         const int leader = __ffs(grp) - 1;
         if (b >= 0 && int(lane) == leader) rank = atomicAdd(&S.cnt[b], uint32_t(__popc(grp)));
         rank = __shfl_sync(0xffffffffu, rank, leader);
-        if (b >= 0) list[off[b] + rank + __popc(grp & ((1u << lane) - 1u))] = u;
+        if (shared) {
+          uint32_t at = 0;
+          if (b >= 9 && int(lane) == leader) at = atomicAdd(&a.ctl->heavy[turn][10 - b], uint32_t(__popc(grp)));
+          at = __shfl_sync(0xffffffffu, at, leader);
+          if (b >= 9) a.heavy[(b == 9 ? a.heavy9 : 0u) + at + __popc(grp & ((1u << lane) - 1u))] = u;
+        }
+        if (b >= 0 && !(shared && b >= 9)) list[off[b] + rank + __popc(grp & ((1u << lane) - 1u))] = u;
       }
       __syncthreads();
       // ---- 2. decide them
@@ -987,7 +1059,7 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
         }
       };
       if constexpr (SYNC) {  // the order changes nothing but the time: long work first
-        blocks();
+        if (!shared) blocks();
         fours();
         units();
       } else {
@@ -1003,18 +1075,43 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
         blocks();
       }
       __syncthreads();
-      if (scan) {  // (the same for every block)
+      if (scan || shared) {  // (the same for every block)
         if (tid == 0) S.next = 0;
         if (!grid_barrier(a, S, nbar++, 0, nullptr)) return;
+      }
+      if (scan) {
         const uint32_t m0 = a.merge_begin[k], m1 = a.merge_begin[k + 1];
         for (uint32_t t = m0 + bid; t < m1; t += G) {
           hub_merge<SYNC, MODE>(a, S, a.merge[t], table, fix);
           __syncthreads();
         }
       }
+      if (shared) {
+        // the class's listed vertices of bin 10, one to a block at a time, and
+        // of bin 9, four (the next unit is fetched while one is decided)
+        const uint32_t n10 = __ldcg(&a.ctl->heavy[turn][0]), n9 = __ldcg(&a.ctl->heavy[turn][1]);
+        const uint32_t nu = n10 + (n9 + 3) / 4, g = wid >> 3;
+        uint32_t x = bid;
+        for (uint32_t r = 0; x < nu; ++r) {
+          if (tid == 0) S.unit[r & 1] = G + atomicAdd(&a.ctl->queue[turn], 1u);
+          if (x < n10) {
+            group_vertex<SYNC, MODE>(a, S, mv, __ldcg(a.heavy + x), tid, PB, 0, table, LOG_BLOCK, 10, fix);
+          } else if ((x - n10) * 4 + g < n9) {
+            group_vertex<SYNC, MODE>(a, S, mv, __ldcg(a.heavy + a.heavy9 + (x - n10) * 4 + g), tid & 255u, 256, 9 + g,
+                                     table + g * 8192u, 12, 9, fix);
+          }
+          __syncthreads();
+          x = S.unit[r & 1];
+        }
+        __syncthreads();
+      }
       const uint32_t nmv = S.nmv, moves = nmv + S.hubmv;
       if (tid == 0) {
         S.next = 0;
+        if (SHARE && a.big && bid == 0) {  // (last used two steps ago)
+          const uint32_t t = (turn + 1) % 3;
+          a.ctl->pieces[t] = 0; a.ctl->heavy[t][0] = 0; a.ctl->heavy[t][1] = 0; a.ctl->queue[t] = 0;
+        }
         S.moves += moves;
         if (last && bid == 0) { a.ctl->fix[(l + 1) % 3] = 0; a.ctl->gactive[(l + 1) % 3] = 0; }
       }
@@ -1034,9 +1131,18 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
       // ---- 3. commit the decisions, mark the movers' neighbours
       if constexpr (SYNC) {
         if (any) {
-          // eight lanes per move; rows above 256 entries by 256 threads
+          // Eight lanes per move, longer rows by 256 threads; where the blocks
+          // share, by a warp, and those of degree bins 9 and 10 in pieces. With
+          // few moves a row is long above 32 entries there: eight lanes take
+          // eight rounds for one of 256, each with up to four hub tables to
+          // update one after the other, and the block that had one kept the
+          // others waiting (40 us a class of a 1e-4 |E| batch on R-MAT scale
+          // 24).
           uint32_t *big = table;  // (vertex, its old and new community)
           constexpr uint32_t BIG_CAP = TABLE_WORDS / 3;
+          const uint32_t wide = SHARE && nmv <= 8 * PW ? 32u : 256u;
+          const bool cut = SHARE && a.big && a.start[k * NUM_BINS + NUM_BINS - 1] > a.start[k * NUM_BINS + 9];
+          const uint32_t np = cut ? __ldcg(&a.ctl->pieces[turn]) : 0u;
           const uint32_t sl = tid & 7u;
           for (uint32_t i = tid >> 3; i < nmv; i += PB / 8) {
             const uint2 m = mv[i];
@@ -1049,7 +1155,7 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
               atomicAdd(&a.ctot[d], -wu);
               atomicAdd(&a.ctot[m.y], wu);
               a.vcom[m.x] = m.y;
-              if (dg > 256) {
+              if (dg > wide) {
                 const uint32_t j = atomicAdd(&S.nbig, 1u);
                 if (j < BIG_CAP) {
                   big[3 * j] = m.x;
@@ -1064,9 +1170,23 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
           }
           __syncthreads();
           const uint32_t nbig = min(S.nbig, BIG_CAP);
-          for (uint32_t i = wid >> 3; i < nbig; i += PW / 8) {
+          for (uint32_t i = SHARE ? wid : wid >> 3; i < nbig; i += SHARE ? PW : PW / 8) {
             const uint32_t u = big[3 * i];
-            mark_row(a, u, a.off[u], a.deg[u], tid & 255u, 256, tabs, big[3 * i + 1], big[3 * i + 2]);
+            if constexpr (SHARE) mark_row_warp(a, u, a.off[u], a.deg[u], lane, 32, tabs, big[3 * i + 1], big[3 * i + 2]);
+            else mark_row(a, u, a.off[u], a.deg[u], tid & 255u, 256);
+          }
+          if constexpr (SHARE) {  // the pieces of the class's large movers, 256 threads each
+            for (uint32_t i = bid * 4 + (wid >> 3); i < np; i += G * 4) {
+              const uint4 e = __ldcg(a.big + i);
+              const uint32_t dg = a.deg[e.x], p = e.w * PIECE;
+              if (p == 0 && (tid & 255u) == 0) {
+                const double wu = a.vtot[e.x];
+                atomicAdd(&a.ctot[e.y], -wu);
+                atomicAdd(&a.ctot[e.z], wu);
+                a.vcom[e.x] = e.z;
+              }
+              mark_row_warp(a, e.x, a.off[e.x] + p, min(PIECE, dg - p), tid & 255u, 256, tabs, e.y, e.z);
+            }
           }
           each_chunk([&](uint32_t t) { return a.hub_move[a.chunk[ch0 + t].x] != EMPTY; },  // the moved hubs' chunks
                      [&](uint32_t t) {
@@ -1078,7 +1198,7 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
                          atomicAdd(&a.ctot[c], wu);
                          a.vcom[u] = c;
                        }
-                       mark_row(a, u, a.off[u] + ch.y, ch.z - ch.y, tid, PB, tabs, d, c);
+                       mark_row_warp(a, u, a.off[u] + ch.y, ch.z - ch.y, tid, PB, tabs, d, c);
                      });
         }
       } else {
