@@ -1119,7 +1119,10 @@ int lvg_autotune(lvg_graph *g, int method, const lvg_device_batch *b, const lvg_
     const lvg_tuning start = cur;
     for (int round = 0; round < 2; ++round) {
       if (colours) try_knob([](lvg_tuning &t, long v) { t.frontier_colors = int(v); }, {8, 4, 2, 1}, true);
-      try_knob([](lvg_tuning &t, long v) { t.hub_chunk = uint32_t(v); }, {2048, 4096, 8192, 16384}, false);
+      // (larger chunks would take the graph's static and deterministic runs off
+      // the phase kernel, whatever they give this workload: a static run of
+      // R-MAT scale 24 147 ms with 16384, 95 with 4096)
+      try_knob([](lvg_tuning &t, long v) { t.hub_chunk = uint32_t(v); }, {2048, 4096}, false);
       // concurrent bins and fused small bins together: each one's best value
       // depends on the other (R-MAT s24, DF at 1e-4 |E|, one class: 0.62 ms
       // with concurrent and unfused, 0.78 ms for the best of one at a time)
