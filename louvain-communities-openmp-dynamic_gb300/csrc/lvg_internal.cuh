@@ -624,11 +624,12 @@ void launch_tidy_compact(const uint32_t *src, const uint32_t *dst, const float *
 void launch_fresh_caps(const uint32_t *deg, size_t n, uint32_t *cap, uint64_t *cap64, cudaStream_t s);
 // The device-side plan of a batch: packed keys, stable sort, first of each
 // run, rows of the touched vertices.
-void launch_pack_keys(const uint32_t *src, const uint32_t *dst, size_t n, int b, uint64_t *key, uint32_t *val,
-                      cudaStream_t s);
+void launch_pack_keys(const uint32_t *ds, const uint32_t *dd, size_t nd, const uint32_t *is, const uint32_t *id,
+                      size_t ni, int b, uint64_t *key, uint32_t *val, cudaStream_t s);
 void launch_first_flags(const uint64_t *key, size_t n, uint32_t *flag, cudaStream_t s);
-void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t *flag, const uint32_t *pos,
-                        size_t n, int b, const float *w, uint32_t *os, uint32_t *od, float *ow, cudaStream_t s);
+void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t *flag, const uint32_t *pos, size_t nd,
+                        size_t ni, int b, const float *dw, const float *iw, uint32_t *ods, uint32_t *odd, float *odw,
+                        uint32_t *ois, uint32_t *oid, float *oiw, uint32_t *cd, uint32_t *ci, cudaStream_t s);
 void launch_plan_rows(const uint32_t *ds, const uint32_t *nd, const uint32_t *is, const uint32_t *ni, size_t cap,
                       uint32_t *flag, uint32_t *pos, uint32_t *scan, UpdRow *rows, unsigned long long *upd,
                       uint32_t *nrows, cudaStream_t s);

@@ -401,11 +401,13 @@ __global__ void fresh_caps_kernel(const uint32_t *deg, size_t n, uint32_t *cap, 
 
 // ---------------------------------------------------------------- plan
 
-// Batch entry i as a packed (src << b | dst) key, with its index.
-__global__ void pack_keys_kernel(const uint32_t *src, const uint32_t *dst, size_t n, int b, uint64_t *key,
-                                 uint32_t *val) {
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
-    key[i] = uint64_t(src[i]) << b | dst[i];
+// The entries of two lists as packed (list, src, dst) keys with their indices
+// (list: the bit above 2b, set for the second where both have entries).
+__global__ void pack_keys_kernel(const uint32_t *ds, const uint32_t *dd, size_t nd, const uint32_t *is,
+                                 const uint32_t *id, size_t ni, int b, uint64_t *key, uint32_t *val) {
+  const uint64_t second = nd ? uint64_t(1) << (2 * b & 63) : 0u;
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nd + ni; i += size_t(gridDim.x) * blockDim.x) {
+    key[i] = i < nd ? uint64_t(ds[i]) << b | dd[i] : second | uint64_t(is[i - nd]) << b | id[i - nd];
     val[i] = uint32_t(i);
   }
 }
@@ -417,16 +419,33 @@ __global__ void first_flags_kernel(const uint64_t *key, size_t n, uint32_t *flag
     flag[i] = i == 0 || key[i] != key[i - 1];
 }
 
+// The first of each run back into its list (the first list's keys are sorted
+// before the second's; pos: the flags' exclusive prefix, their sum at pos[nd +
+// ni]); the lists' lengths into *cd and *ci (where given).
 __global__ void unpack_keys_kernel(const uint64_t *key, const uint32_t *val, const uint32_t *flag,
-                                   const uint32_t *pos, size_t n, int b, const float *w, uint32_t *os, uint32_t *od,
-                                   float *ow) {
+                                   const uint32_t *pos, size_t nd, size_t ni, int b, const float *dw, const float *iw,
+                                   uint32_t *ods, uint32_t *odd, float *odw, uint32_t *ois, uint32_t *oid, float *oiw,
+                                   uint32_t *cd, uint32_t *ci) {
   const uint64_t mask = (uint64_t(1) << b) - 1;
-  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+  const uint32_t kept = pos[nd], all = pos[nd + ni];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (cd) *cd = kept;
+    if (ci) *ci = all - kept;
+  }
+  for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nd + ni; i += size_t(gridDim.x) * blockDim.x) {
     if (!flag[i]) continue;
-    const uint32_t o = pos[i];
-    os[o] = uint32_t(key[i] >> b);
-    od[o] = uint32_t(key[i] & mask);
-    ow[o] = w[val[i]];
+    const uint32_t u = uint32_t(key[i] >> b & mask), v = uint32_t(key[i] & mask);
+    if (i < nd) {
+      const uint32_t o = pos[i];
+      ods[o] = u;
+      odd[o] = v;
+      odw[o] = dw[val[i]];
+    } else {
+      const uint32_t o = pos[i] - kept;
+      ois[o] = u;
+      oid[o] = v;
+      oiw[o] = iw[val[i] - nd];
+    }
   }
 }
 
@@ -791,10 +810,10 @@ void launch_tidy_compact(const uint32_t *src, const uint32_t *dst, const float *
   LVG_CHECK_LAUNCH();
 }
 
-void launch_pack_keys(const uint32_t *src, const uint32_t *dst, size_t n, int b, uint64_t *key, uint32_t *val,
-                      cudaStream_t s) {
-  if (!n) return;
-  pack_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(src, dst, n, b, key, val);
+void launch_pack_keys(const uint32_t *ds, const uint32_t *dd, size_t nd, const uint32_t *is, const uint32_t *id,
+                      size_t ni, int b, uint64_t *key, uint32_t *val, cudaStream_t s) {
+  if (!(nd + ni)) return;
+  pack_keys_kernel<<<grid_for(nd + ni, 256), 256, 0, s>>>(ds, dd, nd, is, id, ni, b, key, val);
   LVG_CHECK_LAUNCH();
 }
 
@@ -804,10 +823,12 @@ void launch_first_flags(const uint64_t *key, size_t n, uint32_t *flag, cudaStrea
   LVG_CHECK_LAUNCH();
 }
 
-void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t *flag, const uint32_t *pos,
-                        size_t n, int b, const float *w, uint32_t *os, uint32_t *od, float *ow, cudaStream_t s) {
-  if (!n) return;
-  unpack_keys_kernel<<<grid_for(n, 256), 256, 0, s>>>(key, val, flag, pos, n, b, w, os, od, ow);
+void launch_unpack_keys(const uint64_t *key, const uint32_t *val, const uint32_t *flag, const uint32_t *pos, size_t nd,
+                        size_t ni, int b, const float *dw, const float *iw, uint32_t *ods, uint32_t *odd, float *odw,
+                        uint32_t *ois, uint32_t *oid, float *oiw, uint32_t *cd, uint32_t *ci, cudaStream_t s) {
+  if (!(nd + ni)) return;
+  unpack_keys_kernel<<<grid_for(nd + ni, 256), 256, 0, s>>>(key, val, flag, pos, nd, ni, b, dw, iw, ods, odd, odw, ois,
+                                                            oid, oiw, cd, ci);
   LVG_CHECK_LAUNCH();
 }
 
