@@ -17,9 +17,10 @@
 //   2. decides them: hubs (degree above 8192) chunk by chunk on many blocks,
 //      merged behind a further barrier; degree <= 32 by a tile of 4/8/16/32
 //      lanes that groups equal communities with warp matches and needs no
-//      table; degree 33-128 by a warp, 129-512 by four warps, 513-2048 by
-//      eight, above by the whole block, each with an open-addressing table of
-//      twice the degree in shared memory;
+//      table; degree 33-128 by a warp, 129-512 by four warps (by one where the
+//      weights' order counts, ORDERED), 513-2048 by eight, above by the whole
+//      block, each with an open-addressing table of twice the degree in shared
+//      memory;
 //   3. deterministic mode: waits until every block has decided, then commits
 //      its own decisions (community, totals) and marks the movers' neighbours.
 //      Asynchronous mode commits at once.
@@ -118,6 +119,18 @@ __device__ __forceinline__ Sum<MODE> weight(const PhaseArgs &a, uint64_t i) {
 // 2-5 %.
 template <bool SYNC, int MODE>
 constexpr bool SHARES = SYNC && (MODE & TOTALS) == 0;
+
+// Deterministic runs of any FP32 weights: the order of a sum is part of its
+// value, so up to degree 512 a vertex's weights are summed by one warp in one
+// order (equal communities of 32 neighbours in lane order, then the 32s in
+// turn), the same in every run and the one of the launch-by-launch kernels.
+// (Four warps adding to one table at degree 129-512 let two runs of one call
+// differ wherever two communities' weights are equal but for their order. First
+// pass of a planted partition with fractional weights, mean degree 48 / 100 /
+// 200 / 400: 2.08 / 2.43 / 1.44 / 2.58 ms, with four warps and no order 2.01 /
+// 2.07 / 1.50 / 2.08, launch by launch 4.88 / 4.25 / 2.13 / 2.86.)
+template <bool SYNC, int MODE>
+constexpr bool ORDERED = SYNC && (MODE & 3) == FLOATS;
 
 struct Shared {
   uint32_t off[MAX_BUCKETS];   // [class][bin]: the block's first list slot of the bin
@@ -260,6 +273,13 @@ __device__ __forceinline__ bool add_warp(uint32_t *keys, uint32_t *vals, uint32_
   }
   if (c != EMPTY) fine &= add<float>(keys, vals, lg, c, w);
   return fine;
+}
+// The same in one order: each community's weights summed in lane order and
+// added once (ORDERED).
+__device__ __forceinline__ bool add_ordered(uint32_t *keys, uint32_t *vals, uint32_t lg, uint32_t c, float w, int lane) {
+  const unsigned grp = __match_any_sync(0xffffffffu, c);
+  const float sum = match_sum<float>(grp, c != EMPTY, w, lane);
+  return c == EMPTY || (grp & ((1u << lane) - 1u)) != 0u || add<float>(keys, vals, lg, c, sum);
 }
 
 // A community or a total that other blocks change within the class: in
@@ -511,7 +531,9 @@ __device__ __forceinline__ Sum<MODE> scan_row(const PhaseArgs &a, Shared &S, uin
 #pragma unroll
     for (int k = 0; k < U; ++k) {
       if (c[k] == d) { kd += w[k]; c[k] = EMPTY; }
-      if constexpr ((MODE & 3) == FLOATS) fine &= add_warp(keys, vals, lg, c[k], w[k], lane);
+      if constexpr ((MODE & 3) == FLOATS)
+        fine &= ORDERED<SYNC, MODE> && n == 32 ? add_ordered(keys, vals, lg, c[k], w[k], lane)
+                                               : add_warp(keys, vals, lg, c[k], w[k], lane);
       else if (c[k] != EMPTY) fine &= add<V>(keys, vals, lg, c[k], (MODE & 3) == UNIT ? 1u : w[k]);
     }
   }
@@ -1028,6 +1050,16 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
       };
       auto fours = [&] {  // degree 129-512, tables in the first half of the area
         const uint32_t c8 = S.cnt[8], c7 = S.cnt[7];
+        if constexpr (ORDERED<SYNC, MODE>) {  // a warp each, tables in the whole area
+          if (wid < PW / 2)
+            for (uint32_t i = wid; i < c8; i += PW / 2)
+              group_vertex<SYNC, MODE>(a, S, mv, list[off[8] + i], lane, 32, 0, table + wid * 2048u, 10, 8, fix);
+          __syncthreads();
+          for (uint32_t i = wid; i < c7; i += PW)
+            group_vertex<SYNC, MODE>(a, S, mv, list[off[7] + i], lane, 32, 0, table + wid * 1024u, 9, 7, fix);
+          __syncthreads();
+          return;
+        }
         for (uint32_t i = wid >> 2; i < c8 + c7; i += PW / 4) {
           const int b = i < c8 ? 8 : 7;
           const uint32_t u = i < c8 ? list[off[8] + i] : list[off[7] + i - c8];
