@@ -41,7 +41,8 @@ extern "C" {
 #define LVG_OK        0
 #define LVG_EINVAL   (-22)   /* bad argument: id >= span, unsorted DS batch, size mismatch */
 #define LVG_ENOMEM   (-12)   /* device or host allocation failed */
-#define LVG_ETIMEOUT (-62)   /* a bounded device loop hit its cap (hash table overflow guard) */
+#define LVG_ETIMEOUT (-62)   /* a bounded device loop hit its cap (hash table overflow guard; a wait
+                                at a barrier given up, see lvg_set_barrier_polls) */
 #define LVG_ECUDA    (-1000) /* CUDA runtime error (no device, launch failure, ...), or a
                                  device-side invariant check (a worklist append outside
                                  its degree bin) */
@@ -427,8 +428,16 @@ typedef struct lvg_stats {
    * as one launch (lvg_tuning.level_graphs). */
   uint64_t level_graphs;
 } lvg_stats;
-/* Enable (1) or disable (0) per-launch event timing for calls on g. */
+/* Enable (1) or disable (0) per-launch event timing for calls on g. Calls then
+ * take the launch-by-launch path (as lvg_tuning.level_graphs = 0), whose launches
+ * have times of their own: the times are those kernels', and an asynchronous
+ * run's outcome is one of that path's. */
 int lvg_set_profiling(lvg_graph *g, int enable);
+/* The blocks of a local-moving phase wait for one another at barriers. Give a
+ * wait up after `polls` polls of its counter (about half a microsecond each; 0:
+ * the default, 2^24): the call then returns LVG_ETIMEOUT, its outputs are
+ * undefined, and the graph can be used as before. */
+int lvg_set_barrier_polls(lvg_graph *g, uint32_t polls);
 
 /* ---- Tuning (no reference counterpart). Launch-shape choices of a graph's
  * local-moving launches that leave Louvain's arithmetic unchanged, except

@@ -760,6 +760,12 @@ int lvg_set_profiling(lvg_graph *g, int enable) {
   return LVG_OK;
 }
 
+int lvg_set_barrier_polls(lvg_graph *g, uint32_t polls) {
+  if (!g) return lvg::fail(LVG_EINVAL, "null graph");
+  g->barrier_polls = polls;
+  return LVG_OK;
+}
+
 int lvg_get_stats(const lvg_graph *g, lvg_stats *out) {
   if (!g || !out) return lvg::fail(LVG_EINVAL, "null argument");
   *out = g->stats;

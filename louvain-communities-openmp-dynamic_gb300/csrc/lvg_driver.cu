@@ -707,6 +707,17 @@ void ensure_hub_buffers(lvg_graph *g, const Level &lv) {
   }
 }
 
+// What the merges of a phase leave zero for the next phase, zeroed: a phase
+// that ended half way (ERR_BARRIER) has partial sums and counts in it.
+void reset_hub_scratch(lvg_graph *g) {
+  Workspace &W = *g->ws;
+  cudaStream_t s = g->stream;
+  LVG_CUDA(cudaMemsetAsync(W.hub_kd.p, 0, W.hub_kd.n * sizeof(float), s));
+  if (W.hub_best.p) LVG_CUDA(cudaMemsetAsync(W.hub_best.p, 0, W.hub_best.n * 8, s));
+  if (W.hub_done.p) LVG_CUDA(cudaMemsetAsync(W.hub_done.p, 0, W.hub_done.n * 4, s));
+  if (W.hub_over.p) LVG_CUDA(cudaMemsetAsync(W.hub_over.p, 0, W.hub_over.n, s));
+}
+
 // Enqueue a level's whole local-moving phase as one launch of the phase
 // kernel (lvg_phase.cu) and the read-back of its counters. False, having
 // enqueued nothing, when the level takes the launch-by-launch path.
@@ -736,6 +747,7 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   W.phase_ctl.ensure(1);
   a.ctr = g->ctr.p; a.ctl = W.phase_ctl.p;
   a.kr = kr; a.colors = lv.colors; a.L = L; a.M = M; a.E = E;
+  a.polls = g->barrier_polls ? g->barrier_polls : PHASE_BARRIER_POLLS;
   a.cap = phase_list_cap(lv, grid);
   if (!phase_lists_fit(a.cap)) {
     W.phase_mv.ensure(size_t(grid) * a.cap);
@@ -838,7 +850,10 @@ int move_phase(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const 
       if (tail_done) *tail_done = true;
     }
     host_sync(g);
-    if (g->hctr.p->err) read_counters(g);  // raises the device error
+    if (g->hctr.p->err) {
+      reset_hub_scratch(g);
+      read_counters(g);  // raises the device error
+    }
     const int l = int(g->hctr.p->dev_iters);
     const double el = uc ? 0.0 : g->hctr.p->dev_el;  // graph unions: each graph's el is in its GraphCtl
     if (end) { end->l = l; end->el = el; }

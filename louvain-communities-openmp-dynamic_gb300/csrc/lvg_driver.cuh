@@ -362,6 +362,7 @@ struct lvg_graph {
       if (e) cudaEventDestroy(e);
   }
   bool profiling = false;
+  uint32_t barrier_polls = 0;  // lvg_set_barrier_polls
   lvg_stats stats = {};
   // batch buffers of the host-array entry points
   DBuf<uint32_t> b_ds, b_dd, b_is, b_id, b_seg;

@@ -345,6 +345,7 @@ struct PhaseArgs {
   float kr;
   int colors, L;
   double M, E;
+  uint32_t polls;     // after this many polls a wait of the grid barrier is given up (ERR_BARRIER)
   uint32_t cap;       // list slots of a block
   uint2 *gmv;         // [grid * cap] moves and lists of blocks that do not fit
   uint32_t *glist;    // shared memory
@@ -376,6 +377,9 @@ struct PhaseArgs {
   // hub chunks, merge tasks and hubs of a class
   uint32_t chunk_begin[MAX_COLORS + 1], merge_begin[MAX_COLORS + 1], hub_begin[MAX_COLORS + 1];
 };
+// Polls of a barrier wait unless the graph has its own limit: seconds, where a
+// class takes microseconds.
+constexpr uint32_t PHASE_BARRIER_POLLS = 1u << 24;
 // Hub chunks (lvg_tuning::hub_chunk) up to this many edges fit the phase
 // kernel's table and leave room for the partitions' counters.
 constexpr uint32_t PHASE_HUB_CHUNK = 4096;

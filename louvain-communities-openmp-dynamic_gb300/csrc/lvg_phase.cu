@@ -56,9 +56,6 @@ constexpr uint32_t LIST_CAP = 1920;       // listed vertices a block keeps in sh
 constexpr uint32_t PIECE = 1024;          // edges of a large mover's row marked at once
 constexpr uint32_t TODO = 256;            // hub chunks a block looks through at a time
 constexpr uint32_t MERGE_FULL = 8192;     // partial entries of a hub that one block merges at once
-// One wait of the grid barrier gives up after this many polls (seconds; a
-// class takes microseconds), flags ERR_BARRIER and ends the kernel.
-constexpr uint32_t BARRIER_POLLS = 1u << 24;
 
 // The level's weights: any FP32, all 1, or whole numbers whose total is below 2^31.
 enum Weights { FLOATS, UNIT, WHOLE };
@@ -163,8 +160,11 @@ __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long lon
 // the waiting poll also tells whether any block moved a vertex (S.any); three
 // words take turns, block 0 clearing the next one (whose last readers have all
 // arrived at the barrier before this one). `sum` (optional) is read behind the
-// barrier into S.sum. False when a wait was given up, here or in another
-// block: every thread of every block then returns.
+// barrier into S.sum. False when a wait was given up (PhaseArgs::polls), here
+// or in another block: every thread of the block then returns. The other
+// blocks get past this barrier at most (their next one never completes), so
+// every block ends, with the class's work in whatever state it was: the host
+// restores what a phase leaves zero for the next (reset_hub_scratch).
 __device__ __forceinline__ bool grid_barrier(const PhaseArgs &a, Shared &S, uint32_t n, uint32_t moves,
                                              const unsigned long long *sum) {
   __syncthreads();
@@ -180,7 +180,7 @@ __device__ __forceinline__ bool grid_barrier(const PhaseArgs &a, Shared &S, uint
       uint32_t polls = 0;
       while (uint32_t(v = ld_acquire(word)) < gridDim.x) {
         ++polls;
-        if (polls >= BARRIER_POLLS || ((polls & 255u) == 0 && ld_acquire(&a.ctl->aborted))) {
+        if (polls >= a.polls || ((polls & 255u) == 0 && ld_acquire(&a.ctl->aborted))) {
           atomicExch(&a.ctl->aborted, 1ull);
           atomicOr(&a.ctr->err, ERR_BARRIER);
           S.stop = 1;

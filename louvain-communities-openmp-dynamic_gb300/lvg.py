@@ -204,6 +204,7 @@ def load_library() -> C.CDLL:
     L.lvg_host_alloc.restype = vp
     L.lvg_host_free.argtypes = [vp]
     L.lvg_set_profiling.argtypes = [vp, i32]
+    L.lvg_set_barrier_polls.argtypes = [vp, C.c_uint32]
     L.lvg_tuning_default.argtypes = [C.POINTER(_Tuning)]
     L.lvg_tuning_default.restype = None
     L.lvg_graph_get_tuning.argtypes = [vp, C.POINTER(_Tuning)]
@@ -709,6 +710,10 @@ class Graph:
 
     def set_profiling(self, on: bool) -> None:
         _check(self._L.lvg_set_profiling(self.h, int(on)))
+
+    def set_barrier_polls(self, polls: int) -> None:
+        """Polls after which a wait at a phase's barrier is given up (0: the default)."""
+        _check(self._L.lvg_set_barrier_polls(self.h, polls))
 
     def device_bytes(self) -> int:
         """Device bytes held by the graph, its workspace and scratch (lvg_graph_device_bytes)."""
