@@ -1161,6 +1161,14 @@ void run(lvg_graph *g, int method, const DBatch &b, StateRef prior, StateRef out
   // resident hub tables: the dynamic methods on a unit-weight graph, between
   // two states (lvg_run_resident)
   const bool tabs0 = tprior && tout && uses_hub_tables(g, method);
+  // The result's tables follow its membership move by move: if the run ends by
+  // an error anywhere between, they are of no use.
+  struct DropOnError {
+    HubTables *t;
+    ~DropOnError() {
+      if (t) t->version = ~0ull;
+    }
+  } unfinished{tout};
   int l = 0, p = 0;
   for (int r = 0; r < rep; ++r) {
     g->events.reset();
@@ -1383,6 +1391,7 @@ void run(lvg_graph *g, int method, const DBatch &b, StateRef prior, StateRef out
   g->stats.hub_table_slots = g->hctr.p->ht_slots;
   g->stats.hub_table_overflow = g->hctr.p->ht_over;
   g->stats.kernel_launches = launch_counter() - launches0;
+  unfinished.t = nullptr;
 }
 
 // Static Louvain on a graph union: one run over all graphs, each graph

@@ -1,7 +1,7 @@
 """A phase whose barrier wait is given up (lvg_set_barrier_polls: here after one
 poll) ends with LVG_ETIMEOUT and leaves nothing behind: the next runs on the same
 graph and states equal those of fresh ones, bit for bit. The graph has hubs,
-whose partial sums and counts live from one phase to the next."""
+whose partial sums, counts and resident tables live from one phase to the next."""
 import numpy as np
 import pytest
 
@@ -58,3 +58,31 @@ def test_union_after_a_timeout(cuda, base):
     _times_out(cuda, U, lambda: cuda.louvain_static_union(U, o))
     for r, (m, ct) in zip(cuda.louvain_static_union(U, o), fresh):
         assert np.array_equal(r.membership, m) and np.array_equal(r.communityWeight, ct)
+
+
+def test_resident_tables_after_a_timeout(cuda, base):
+    """A frontier run in place: its state's tables were half brought up to date."""
+    x, prior = base
+    o = cuda.LouvainOptions(deterministic=True)
+    G = cuda.Graph(x)
+    db = cuda.DeviceBatch(G, cuda.random_batch(x, 3000, seed=5))
+    G.apply_batch(db)
+    st = cuda.State(G)
+    st.set(*prior)
+    cuda.run_resident(G, cuda.METHOD_FRONTIER, db, st, st, o)  # (with tables)
+    assert G.stats()["hub_tables_built"] == 1
+    more = cuda.DeviceBatch(G, cuda.random_batch(x, 4000, seed=6))
+    G.apply_batch(more)
+    _times_out(cuda, G, lambda: cuda.run_resident(G, cuda.METHOD_FRONTIER, more, st, st, o))
+    left = st.get()  # whatever the run left is a state: go on from it here and in a fresh graph
+    assert left[0].max() < G.span
+    batch = cuda.DeviceBatch(G, cuda.random_batch(x, 3000, seed=7))
+    G.apply_batch(batch)
+    cuda.run_resident(G, cuda.METHOD_FRONTIER, batch, st, st, o)
+    assert G.stats()["hub_tables_built"] == 1
+    F = cuda.Graph(G.download())
+    fs = cuda.State(F)
+    fs.set(*left)
+    cuda.run_resident(F, cuda.METHOD_FRONTIER, cuda.DeviceBatch(F, batch.download()), fs, fs, o)
+    for a, b in zip(st.get(), fs.get()):
+        assert np.array_equal(a, b)
