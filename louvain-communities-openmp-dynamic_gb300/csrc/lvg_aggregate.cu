@@ -591,16 +591,6 @@ __global__ void member_degrees_kernel(const uint32_t *cmem, const uint32_t *deg,
     dst[i] = deg[cmem[i]];
 }
 
-int sms() {  // SM count of the device, queried once (thread-safe static init)
-  static const int n = [] {
-    int dev = 0, c = 0;
-    LVG_CUDA(cudaGetDevice(&dev));
-    LVG_CUDA(cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev));
-    return c;
-  }();
-  return n;
-}
-
 template <class K>
 void set_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) LVG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
@@ -611,10 +601,10 @@ void launch_tile(const AggArgs &a, cudaStream_t s) {
   constexpr int TPB = TILE_BLOCK / T;
   const size_t smem = size_t(TPB) * C * 8;
   auto k = agg_tile_kernel<T, C>;
-  static bool configured = false;
-  if (!configured) { set_smem(k, smem); configured = true; }
+  static PerDevice<bool> configured;
+  configured.get([&] { set_smem(k, smem); return true; });
   size_t want = (a.count + TPB - 1) / TPB;
-  size_t cap = size_t(sms()) * (smem > 32 * 1024 ? 3 : 8);
+  size_t cap = size_t(device_sms()) * (smem > 32 * 1024 ? 3 : 8);
   unsigned grid = unsigned(want < cap ? want : cap);
   if (!grid) return;
   k<<<grid, TILE_BLOCK, smem, s>>>(a);
@@ -625,13 +615,14 @@ template <int MODE, int B, int LOGS>
 void launch_group(const AggArgs &a, cudaStream_t s) {
   const size_t smem = (size_t(1) << LOGS) * 8;
   auto k = agg_group_kernel<MODE, B, LOGS>;
-  // as many blocks as fit the device (queried once; thread-safe)
-  static const unsigned resident = [&] {
+  // as many blocks as fit the device
+  static PerDevice<unsigned> fit;
+  const unsigned resident = fit.get([&] {
     set_smem(k, smem);
     int per_sm = 0;
     LVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, B, smem));
-    return unsigned(per_sm > 0 ? per_sm : 1) * unsigned(sms());
-  }();
+    return unsigned(per_sm > 0 ? per_sm : 1) * unsigned(device_sms());
+  });
   const unsigned grid = a.count < resident ? a.count : resident;
   if (!grid) return;
   k<<<grid, B, smem, s>>>(a);
@@ -656,12 +647,12 @@ void launch_chunks(const AggArgs &a, const AggChunks &ch, size_t runs, size_t me
   const size_t smem1 = (size_t(1) << CHUNK_LOGS) * 8, smem2 = (size_t(1) << MERGE_LOGS) * 8;
   auto k1 = agg_chunk_kernel<MODE, AGG_CHUNK_B>;
   auto k2 = agg_merge_kernel<MODE, AGG_MERGE_B>;
-  static const bool configured = [&] {
+  static PerDevice<bool> configured;
+  configured.get([&] {
     set_smem(k1, smem1 + size_t(AGG_MAX_PARTS) * 4);
     set_smem(k2, smem2);
     return true;
-  }();
-  (void)configured;
+  });
   k1<<<unsigned(runs), AGG_CHUNK_B, smem1 + size_t(max_parts) * 4, s>>>(a, ch);  // (the partitions' counters behind)
   LVG_CHECK_LAUNCH();
   k2<<<unsigned(merges), AGG_MERGE_B, smem2, s>>>(a, ch);

@@ -739,7 +739,10 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   // R-MAT graph) than two runs of one order differ (0.2-0.7 %).
   if (P.hubs && from_prior && !sync) return false;
   if (P.hubs && (g->tuning.hub_chunk > PHASE_HUB_CHUNK || lv.bin_maxdeg[NUM_BINS - 1] > PHASE_MAX_DEGREE)) return false;
-  const uint32_t grid = phase_grid(lv);
+  // (a dynamic run's totals begin with the caller's, which can be any numbers)
+  const bool small = g->total_weight < 2147483648.0, whole = lv.whole && small;
+  const bool totals = !from_prior && small && (lv.unit || lv.whole);
+  const uint32_t grid = phase_grid(lv, sync, lv.unit, whole, totals);
   if (!grid) return false;
   PhaseArgs a{};
   a.off = lv.off; a.deg = lv.deg; a.key = lv.key; a.w = lv.w; a.bins = lv.bins;
@@ -780,8 +783,6 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
     a.graphs = uint32_t(uc->n); a.gctl = uc->ctl; a.gM = uc->M; a.itcap = uc->L;
   }
   for (int i = 0; i <= lv.colors * NUM_BINS; ++i) a.start[i] = uint32_t(lv.bin_start[i]);
-  // (a dynamic run's totals begin with the caller's, which can be any numbers)
-  const bool small = g->total_weight < 2147483648.0, totals = !from_prior && small && (lv.unit || lv.whole);
   if (sync && !totals) {
     size_t pieces = 0, n10 = 0, n9 = 0;
     for (int k = 0; k < lv.colors; ++k) {
@@ -802,7 +803,7 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
     }
   }
   launch_fill_bytes(W.phase_ctl.p, 0, sizeof(PhaseCtl), s);
-  launch_phase(sync, lv.unit, lv.whole && small, totals, grid, a, s);
+  launch_phase(sync, lv.unit, whole, totals, grid, a, s);
   ++g->stats.move_launches;
   ++g->stats.level_graphs;
   LVG_CUDA(cudaMemcpyAsync(g->hctr.p, g->ctr.p, sizeof(Counters), cudaMemcpyDeviceToHost, s));

@@ -1,6 +1,7 @@
 // lvg_internal.cuh — device data layout and kernel launchers shared by the
 // translation units of liblouvain_gb300.so.
 #pragma once
+#include <mutex>
 #include <utility>
 #include <vector>
 
@@ -57,6 +58,24 @@ struct DBuf {
     std::swap(p, o.p);
     std::swap(n, o.n);
     std::swap(acct, o.acct);
+  }
+};
+
+// A value of each device, made by the first call on it: a kernel's attributes
+// and the blocks that fit belong to a device, and handles of one process may
+// live on several (lvg_set_device).
+template <class T>
+struct PerDevice {
+  static constexpr int KEPT = 64;
+  std::once_flag made[KEPT];
+  T value[KEPT];
+  template <class Make>
+  T get(Make make) {
+    int dev = 0;
+    LVG_CUDA(cudaGetDevice(&dev));
+    if (dev >= KEPT) return make();
+    std::call_once(made[dev], [&] { value[dev] = make(); });
+    return value[dev];
   }
 };
 
@@ -385,8 +404,8 @@ constexpr uint32_t PHASE_BARRIER_POLLS = 1u << 24;
 constexpr uint32_t PHASE_HUB_CHUNK = 4096;
 constexpr uint64_t PHASE_MAX_DEGREE = 8192ull * 16384ull;  // partitions the counters hold
 // Blocks and list slots per block a level's phase kernel takes (0 blocks: the
-// device cannot launch cooperatively).
-uint32_t phase_grid(const Level &lv);
+// device cannot launch it cooperatively). The flags as launch_phase's.
+uint32_t phase_grid(const Level &lv, bool sync, bool unit, bool whole, bool totals);
 uint32_t phase_list_cap(const Level &lv, uint32_t grid);
 void launch_phase(bool sync, bool unit, bool whole, bool totals, uint32_t grid, const PhaseArgs &a, cudaStream_t s);
 bool phase_lists_fit(uint32_t cap);  // the lists stay in shared memory

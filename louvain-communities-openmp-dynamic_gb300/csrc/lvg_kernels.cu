@@ -8,16 +8,6 @@
 namespace lvg {
 namespace {
 
-int sms() {  // SM count of the device, queried once (thread-safe static init)
-  static const int n = [] {
-    int dev = 0, c = 0;
-    LVG_CUDA(cudaGetDevice(&dev));
-    LVG_CUDA(cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev));
-    return c;
-  }();
-  return n;
-}
-
 #define GRID_STRIDE(i, n) for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < (n); i += size_t(gridDim.x) * blockDim.x)
 
 __device__ __forceinline__ double warp_sum_d(double v) {
@@ -1111,7 +1101,7 @@ __global__ void sq_sum_kernel(const double *x, size_t n, double *dst) {
 
 int grid_for(size_t n, int block, int max_blocks_per_sm) {
   size_t want = (n + block - 1) / block;
-  size_t cap = size_t(sms()) * max_blocks_per_sm;
+  size_t cap = size_t(device_sms()) * max_blocks_per_sm;
   size_t g = want < cap ? want : cap;
   return int(g ? g : 1);
 }
@@ -1268,12 +1258,12 @@ void launch_ds_mark(const Level &g, const uint32_t *ds, const uint32_t *dd, size
     ds_expand_kernel<<<grid_for(g.span, 256), 256, 0, s>>>(g.ex, g.span, vcom, g.deg, neighbors, communities,
                                                             vertices, list, count);
     LVG_CHECK_LAUNCH();
-    ds_neighbors_kernel<<<unsigned(sms()) * 8, 256, 0, s>>>(g.off, g.deg, g.key, list, count, vertices);
+    ds_neighbors_kernel<<<unsigned(device_sms()) * 8, 256, 0, s>>>(g.off, g.deg, g.key, list, count, vertices);
     LVG_CHECK_LAUNCH();
     ds_big_chunks_kernel<<<grid_for(g.span, 256), 256, 0, s>>>(g.deg, list, count, g.span, chunks);
     LVG_CHECK_LAUNCH();
     exclusive_scan_u32(chunks, chunks, g.span, &ctr->ds_chunks, scan_scratch, s);
-    ds_neighbors_big_kernel<<<unsigned(sms()) * 8, 256, 0, s>>>(g.off, g.deg, g.key, list, count, g.span, chunks,
+    ds_neighbors_big_kernel<<<unsigned(device_sms()) * 8, 256, 0, s>>>(g.off, g.deg, g.key, list, count, g.span, chunks,
                                                                &ctr->ds_chunks, vertices);
     LVG_CHECK_LAUNCH();
   }
@@ -1289,7 +1279,7 @@ void launch_clear_isolated_multi(const IsolatedLists &L, uint8_t *vaff, const ui
   size_t most = 0, total = 0;
   for (int j = 0; j < L.k; ++j) { most = std::max(most, L.n[j]); total += L.n[j]; }
   if (!total) return;
-  const unsigned grid = unsigned(std::min<size_t>(size_t(L.k) * ((most + 255) / 256), size_t(sms()) * 8 * L.k));
+  const unsigned grid = unsigned(std::min<size_t>(size_t(L.k) * ((most + 255) / 256), size_t(device_sms()) * 8 * L.k));
   clear_isolated_multi_kernel<<<grid, 256, 0, s>>>(L, vaff, fa);
   LVG_CHECK_LAUNCH();
 }

@@ -1145,16 +1145,6 @@ __global__ void __launch_bounds__(B) hub_table_kernel(MoveArgs a) {
   if (threadIdx.x == 0 && slots) atomicAdd(&a.ctr->ht_slots, slots);
 }
 
-int num_sms() {  // SM count of the device, queried once (thread-safe static init)
-  static const int n = [] {
-    int dev = 0, c = 0;
-    LVG_CUDA(cudaGetDevice(&dev));
-    LVG_CUDA(cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev));
-    return c;
-  }();
-  return n;
-}
-
 template <class K>
 void set_smem(K kernel, size_t bytes) {
   if (bytes > 48 * 1024) LVG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes)));
@@ -1166,8 +1156,8 @@ void launch_small(const MoveArgs &a, SmallBins sb, cudaStream_t s) {
   constexpr size_t CMAX = size_t(TILE_BLOCK / (HI <= 1 ? 4 : HI == 2 ? 8 : HI == 3 ? 16 : 32)) *
                           (size_t(4) << HI) * 8;
   auto k = move_small_kernel<LO, HI, SYNC, UNIT, MINB>;
-  static bool configured = false;
-  if (!configured) { set_smem(k, CMAX); configured = true; }
+  static PerDevice<bool> configured;
+  configured.get([&] { set_smem(k, CMAX); return true; });
   const unsigned grid = sb.block_begin[HI - LO + 1];
   if (!grid) return;
   k<<<grid, TILE_BLOCK, CMAX, s>>>(a, sb);
@@ -1179,10 +1169,10 @@ void launch_tile(const MoveArgs &a, cudaStream_t s) {
   constexpr int TPB = TILE_BLOCK / T;
   const size_t smem = size_t(TPB) * C * 8;
   auto k = move_tile_kernel<T, C, SYNC, UNIT>;
-  static bool configured = false;
-  if (!configured) { set_smem(k, smem); configured = true; }
+  static PerDevice<bool> configured;
+  configured.get([&] { set_smem(k, smem); return true; });
   size_t want = (a.count + TPB - 1) / TPB;
-  size_t cap = size_t(num_sms()) * (smem > 32 * 1024 ? 3 : 8);
+  size_t cap = size_t(device_sms()) * (smem > 32 * 1024 ? 3 : 8);
   unsigned grid = unsigned(want < cap ? want : cap);
   if (!grid) return;
   k<<<grid, TILE_BLOCK, smem, s>>>(a);
@@ -1200,23 +1190,23 @@ constexpr int HUBM_B = 512, HUBM_LOGS = 13;     // hub merge
 constexpr int HUBS_B = 256;                     // hub spill
 constexpr int HUBT_B = 128;                     // resident hub tables
 
-// Resident blocks of a large-degree kernel on the whole device, queried once.
+// Resident blocks of a large-degree kernel on the whole device.
 template <class K>
 unsigned resident_blocks(K kernel, int block, size_t smem) {
   int per_sm = 0;
   LVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, block, smem));
-  return unsigned(std::max(1, per_sm)) * unsigned(num_sms());
+  return unsigned(std::max(1, per_sm)) * unsigned(device_sms());
 }
 
 template <int B, int LOGS, bool SYNC, bool UNIT>
 unsigned big_grid(size_t count, int cap_per_sm) {
   const size_t smem = (size_t(1) << LOGS) * 10;  // keys, values, claimed list
-  static const unsigned resident = [&] {
+  static PerDevice<unsigned> resident;
+  size_t r = resident.get([&] {
     set_smem(move_big_kernel<B, LOGS, SYNC, UNIT>, smem);
     return resident_blocks(move_big_kernel<B, LOGS, SYNC, UNIT>, B, smem);
-  }();
-  size_t r = resident;
-  if (cap_per_sm > 0) r = std::min(r, size_t(cap_per_sm) * size_t(num_sms()));
+  });
+  if (cap_per_sm > 0) r = std::min(r, size_t(cap_per_sm) * size_t(device_sms()));
   return unsigned(std::min<size_t>(count, r));
 }
 
@@ -1237,23 +1227,23 @@ void launch_hubs(const MoveArgs &a, cudaStream_t s, cudaStream_t s_tab) {
   if (!nh) return;
   auto k1 = hub_chunk_kernel<HUBC_B, HUBC_LOGS, UNIT>;
   auto k2 = hub_merge_kernel<HUBM_B, HUBM_LOGS, SYNC>;
-  static bool configured = false;
-  if (!configured) { set_smem(k1, smem1); set_smem(k2, smem2); configured = true; }
+  static PerDevice<bool> configured;
+  configured.get([&] { set_smem(k1, smem1); set_smem(k2, smem2); return true; });
   if (a.ht.key) {
-    hub_table_kernel<HUBT_B, SYNC><<<unsigned(std::min<size_t>(nh, size_t(num_sms()) * 8)), HUBT_B, 0,
+    hub_table_kernel<HUBT_B, SYNC><<<unsigned(std::min<size_t>(nh, size_t(device_sms()) * 8)), HUBT_B, 0,
                                      s_tab ? s_tab : s>>>(a);
     LVG_CHECK_LAUNCH();
   }
   // with resident tables the chunks only mark themselves empty (unless a
   // table went bad): a few blocks per SM loop over them
-  const size_t g1 = a.ht.key ? std::min<size_t>(nch, size_t(num_sms()) * 2) : nch;
+  const size_t g1 = a.ht.key ? std::min<size_t>(nch, size_t(device_sms()) * 2) : nch;
   k1<<<unsigned(g1), HUBC_B, smem1, s>>>(a);
   LVG_CHECK_LAUNCH();
   if (a.spill_keys) {
     hub_spill_kernel<HUBS_B><<<unsigned(nch), HUBS_B, 0, s>>>(a);
     LVG_CHECK_LAUNCH();
     const size_t slots = a.hub.class_slots[a.color];
-    const unsigned grid = unsigned(std::min<size_t>((slots + 255) / 256, size_t(num_sms()) * 8));
+    const unsigned grid = unsigned(std::min<size_t>((slots + 255) / 256, size_t(device_sms()) * 8));
     if (grid) {
       hub_argmax_kernel<<<grid, 256, 0, s>>>(a);
       LVG_CHECK_LAUNCH();
@@ -1261,7 +1251,7 @@ void launch_hubs(const MoveArgs &a, cudaStream_t s, cudaStream_t s_tab) {
   }
   // (with resident tables the merge has only the hubs of bad tables to do:
   // a block per SM, looping over the hubs)
-  const size_t g2 = a.ht.key ? std::min<size_t>(size_t(global_table_blocks(nh)), size_t(num_sms()))
+  const size_t g2 = a.ht.key ? std::min<size_t>(size_t(global_table_blocks(nh)), size_t(device_sms()))
                              : size_t(global_table_blocks(nh));
   k2<<<unsigned(g2), HUBM_B, smem2, s>>>(a);
   LVG_CHECK_LAUNCH();
@@ -1304,7 +1294,7 @@ int move_grid_blocks(int bin, bool sync, bool unit, size_t count, int big_cap) {
 }
 
 int global_table_blocks(size_t count) {
-  size_t cap = size_t(num_sms()) * 3;
+  size_t cap = size_t(device_sms()) * 3;
   return int(count < cap ? count : cap);
 }
 
@@ -1316,7 +1306,15 @@ void launch_move_hubs(bool sync, const MoveArgs &a, cudaStream_t s, cudaStream_t
   else launch_hubs<false, false>(a, s, s_tab);
 }
 
-int device_sms() { return num_sms(); }
+int device_sms() {
+  static PerDevice<int> sms;
+  return sms.get([] {
+    int dev = 0, c = 0;
+    LVG_CUDA(cudaGetDevice(&dev));
+    LVG_CUDA(cudaDeviceGetAttribute(&c, cudaDevAttrMultiProcessorCount, dev));
+    return c;
+  });
+}
 
 template <int MINB>
 void launch_small_1_6(bool sync, const MoveArgs &a, const SmallBins &sb, cudaStream_t s) {

@@ -1280,17 +1280,42 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
 
 constexpr size_t SMEM = (size_t(TABLE_WORDS) + 3 * LIST_CAP) * sizeof(uint32_t);
 
+// The device's blocks that can be resident at once, with the kernel's attribute
+// set (0: the device launches none cooperatively).
+template <bool SYNC, int MODE>
+uint32_t most_blocks() {
+  static PerDevice<uint32_t> most;
+  return most.get([] {
+    int dev = 0, coop = 0, per_sm = 0;
+    LVG_CUDA(cudaGetDevice(&dev));
+    LVG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return 0u;
+    auto k = phase_kernel<SYNC, MODE>;
+    LVG_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM)));
+    LVG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, PB, SMEM));
+    return uint32_t(per_sm) * uint32_t(device_sms());
+  });
+}
+
 template <bool SYNC, int MODE>
 void launch(uint32_t grid, const PhaseArgs &a, cudaStream_t s) {
-  static const bool configured = [] {  // (thread-safe, once)
-    LVG_CUDA(cudaFuncSetAttribute(phase_kernel<SYNC, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(SMEM)));
-    return true;
-  }();
-  (void)configured;
   void *args[] = {const_cast<PhaseArgs *>(&a)};
   LVG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void *>(phase_kernel<SYNC, MODE>), dim3(grid), dim3(PB), args,
                                        SMEM, s));
   ++launch_counter();
+}
+
+// f(SYNC, MODE) of the kernel that serves a phase.
+template <class F>
+void variant(bool sync, bool unit, bool whole, bool totals, F f) {
+  auto mode = [&](auto S) {
+    const bool t = totals && (unit || whole);
+    if (unit) t ? f(S, std::integral_constant<int, UNIT | TOTALS>()) : f(S, std::integral_constant<int, UNIT>());
+    else if (whole) t ? f(S, std::integral_constant<int, WHOLE | TOTALS>()) : f(S, std::integral_constant<int, WHOLE>());
+    else f(S, std::integral_constant<int, FLOATS>());
+  };
+  if (sync) mode(std::true_type());
+  else mode(std::false_type());
 }
 
 }  // namespace
@@ -1299,15 +1324,12 @@ bool phase_lists_fit(uint32_t cap) { return cap <= LIST_CAP; }
 
 // Enough blocks for the largest class's warps of work (a block's vertex
 // counts 32 of them, a tile-sized one its share of a warp) to be about one per
-// warp, at most one block per SM: fewer blocks make the barriers cheaper.
-uint32_t phase_grid(const Level &lv) {
-  static const bool coop = [] {
-    int dev = 0, c = 0;
-    LVG_CUDA(cudaGetDevice(&dev));
-    LVG_CUDA(cudaDeviceGetAttribute(&c, cudaDevAttrCooperativeLaunch, dev));
-    return c != 0;
-  }();
-  if (!coop) return 0;
+// warp, at most those that are resident at once: fewer blocks make the barriers
+// cheaper.
+uint32_t phase_grid(const Level &lv, bool sync, bool unit, bool whole, bool totals) {
+  uint32_t blocks = 0;
+  variant(sync, unit, whole, totals, [&](auto S, auto M) { blocks = most_blocks<S.value, M.value>(); });
+  if (!blocks) return 0;
   static const uint32_t share[NUM_BINS] = {0, 4, 8, 16, 32, 32, 32, 128, 128, 256, 1024, 1024};  // 1/32 warps
   uint64_t most = 0;
   for (int k = 0; k < lv.colors; ++k) {
@@ -1316,7 +1338,7 @@ uint32_t phase_grid(const Level &lv) {
     units += uint64_t(lv.hub.chunk_begin[k + 1] - lv.hub.chunk_begin[k]) * share[NUM_BINS - 1];  // (a block per chunk)
     most = std::max(most, units / 32);
   }
-  return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(uint64_t(device_sms()), (most + PW / 2 - 1) / (PW / 2))));
+  return uint32_t(std::max<uint64_t>(1, std::min<uint64_t>(blocks, (most + PW / 2 - 1) / (PW / 2))));
 }
 
 uint32_t phase_list_cap(const Level &lv, uint32_t grid) {
@@ -1333,17 +1355,7 @@ uint32_t phase_list_cap(const Level &lv, uint32_t grid) {
 }
 
 void launch_phase(bool sync, bool unit, bool whole, bool totals, uint32_t grid, const PhaseArgs &a, cudaStream_t s) {
-  const int mode = unit ? UNIT : whole ? WHOLE : FLOATS;
-  const bool t = totals && mode != FLOATS;
-  if (sync) {
-    if (mode == FLOATS) launch<true, FLOATS>(grid, a, s);
-    else if (mode == UNIT) t ? launch<true, UNIT | TOTALS>(grid, a, s) : launch<true, UNIT>(grid, a, s);
-    else t ? launch<true, WHOLE | TOTALS>(grid, a, s) : launch<true, WHOLE>(grid, a, s);
-  } else {
-    if (mode == FLOATS) launch<false, FLOATS>(grid, a, s);
-    else if (mode == UNIT) t ? launch<false, UNIT | TOTALS>(grid, a, s) : launch<false, UNIT>(grid, a, s);
-    else t ? launch<false, WHOLE | TOTALS>(grid, a, s) : launch<false, WHOLE>(grid, a, s);
-  }
+  variant(sync, unit, whole, totals, [&](auto S, auto M) { launch<S.value, M.value>(grid, a, s); });
 }
 
 }  // namespace lvg
