@@ -121,8 +121,9 @@ int lvg_graph_create(size_t span, const uint64_t *offsets, const uint32_t *keys,
 int lvg_graph_destroy(lvg_graph *g);
 /* Device bytes held by a graph: its gapped CSR, workspace and scratch. */
 size_t lvg_graph_device_bytes(const lvg_graph *g);
-/* Release scratch a graph keeps between calls: level 1 the global hash
- * tables and the batch-apply scratch, level 2 also the workspace. Later calls
+/* Release scratch a graph keeps between calls: level 1 the hash tables, the
+ * scratch of the local-moving phases, of the aggregation and of batch apply, and
+ * a union's pinned result staging; level 2 also the workspace. Later calls
  * allocate again what they need. */
 int lvg_graph_trim(lvg_graph *g, int level);
 /* G::span(), G::order(), G::size() (inc/Graph.hxx:59-80). */

@@ -513,8 +513,15 @@ int lvg_graph_trim(lvg_graph *g, int level) {
     if (g->ws) {
       lvg::Workspace &W = *g->ws;
       W.gkeys.release(); W.gvals.release();
-      W.part_key.release(); W.part_val.release(); W.chunk_cnt.release();
+      W.part_key.release(); W.part_val.release(); W.chunk_cnt.release(); W.hub_segs.release();
+      W.spill_keys.release(); W.spill_vals.release();
+      W.phase_big.release(); W.phase_heavy.release(); W.phase_mv.release(); W.phase_list.release();
+      W.ht_soff.release(); W.ht_slg.release(); W.ht_skey.release(); W.ht_scnt.release(); W.ht_n.release();
+      W.mpre.release(); W.agg_tdeg.release(); W.agg_plan.release();
+      W.agg_pairs.release(); W.agg_seg.release(); W.agg_lists.release();
     }
+    if (g->uni)
+      for (auto &b : g->uni->stage.buf) b.release();
     for (auto *d : {&g->u_k0, &g->u_k1, &g->u_len, &g->u_src, &g->u_grow, &g->u_spos, &g->u_srcpos, &g->u_gpos,
                     &g->u_scan})
       d->release();

@@ -86,13 +86,17 @@ struct HBuf {  // pinned host buffer, grows on demand
   HBuf() = default;
   HBuf(const HBuf &) = delete;
   HBuf &operator=(const HBuf &) = delete;
-  ~HBuf() { if (p) cudaFreeHost(p); }
+  ~HBuf() { release(); }
   void ensure(size_t k) {
     if (p && k <= n) return;
-    if (p) cudaFreeHost(p);
-    p = nullptr;
+    release();
     LVG_CUDA(cudaMallocHost(&p, (k ? k : 1) * sizeof(T)));
     n = k;
+  }
+  void release() {
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
   }
 };
 
