@@ -376,8 +376,11 @@ __global__ void __launch_bounds__(B) agg_group_kernel(AggArgs a) {
 // partition (parts: as many as leave about AGG_PART distinct communities each;
 // seg: the groups' bounds). A second kernel, a block per (community,
 // partition), sums a partition's pairs of all lists the same way and appends
-// them to the row. No table in global memory: its atomics (two per pair) took
-// longer than both kernels. Measured on an R-MAT scale-23 run against such
+// them to the community's merged row. The lists lie in the row's own place (a
+// list has at most as many pairs as its chunks edges, and the row has room for
+// them all), so a third kernel copies the merged row there: lists of their own
+// took 8 bytes per edge of these communities. No table in global memory: its
+// atomics (two per pair) took longer than both kernels. Measured on an R-MAT scale-23 run against such
 // tables: level 0 4.7 -> 2.9 ms, scale 18 2.4 -> 0.1 ms (too few chunks to hide
 // the atomics); a fixed eight lanes per list in the merge took 11 ms where a
 // community has two partitions.
@@ -484,7 +487,8 @@ __global__ void __launch_bounds__(B) agg_chunk_kernel(AggArgs a, AggChunks ch) {
       if (lane == 0) seg[R] = carry;
     }
     __syncthreads();
-    const uint64_t p0 = ch.part_off[j] + uint64_t(from) * AGG_CHUNK;
+    const uint64_t p0 = a.yoff[c] + uint64_t(from) * AGG_CHUNK;
+    uint32_t *yv = reinterpret_cast<uint32_t *>(a.yw);
     for (uint32_t s = threadIdx.x; s < CS; s += B) {
       const uint32_t x = keys[s];
       const uint32_t r = x != EMPTY ? part_of(x, R) : EMPTY;
@@ -493,7 +497,7 @@ __global__ void __launch_bounds__(B) agg_chunk_kernel(AggArgs a, AggChunks ch) {
       uint32_t at = 0;
       if (r != EMPTY && lane == leader) at = atomicAdd(&pc[r], uint32_t(__popc(grp)));
       at = __shfl_sync(0xffffffffu, at, leader) + __popc(grp & ((1u << lane) - 1u));
-      if (r != EMPTY) ch.pairs[p0 + at] = make_uint2(x, vals[s]);
+      if (r != EMPTY) { a.ykey[p0 + at] = x; yv[p0 + at] = vals[s]; }
     }
     __syncthreads();
     from = k + 1;
@@ -529,7 +533,7 @@ __global__ void __launch_bounds__(B) agg_merge_kernel(AggArgs a, AggChunks ch) {
   const uint32_t L = min(256u, max(8u, want ? 1u << (31 - __clz(want)) : 0u));
   const uint32_t sl = threadIdx.x & (L - 1u), step = B / L;
   const uint32_t *seg = ch.seg + ch.seg_off[j] + r;
-  const uint2 *p = ch.pairs + ch.part_off[j];
+  const uint32_t *pk = a.ykey + a.yoff[c], *pv = reinterpret_cast<const uint32_t *>(a.yw) + a.yoff[c];
   uint32_t k = threadIdx.x / L;
   uint32_t b = 0, e = 0, f = 0;
   if (k < nc) { b = seg[uint64_t(k) * (R + 1)]; e = seg[uint64_t(k) * (R + 1) + 1]; f = list_at[k]; }
@@ -540,18 +544,22 @@ __global__ void __launch_bounds__(B) agg_merge_kernel(AggArgs a, AggChunks ch) {
       ne = seg[uint64_t(k + step) * (R + 1) + 1];
       nf = list_at[k + step];
     }
-    const uint2 *g = p + uint64_t(f) * AGG_CHUNK;
+    const uint64_t g = uint64_t(f) * AGG_CHUNK;
     for (uint32_t q = b + sl; q < e; q += 4 * L) {  // four pairs of a lane in flight
-      uint2 x[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) x[u] = q + u * L < e ? __ldcs(g + q + u * L) : make_uint2(EMPTY, 0u);
+      uint32_t x[4], v[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
-        if (x[u].x == EMPTY) continue;
+        const bool in = q + u * L < e;
+        x[u] = in ? __ldcs(pk + g + q + u * L) : EMPTY;
+        v[u] = in ? __ldcs(pv + g + q + u * L) : 0u;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (x[u] == EMPTY) continue;
         Sum<MODE> w;
-        if constexpr (MODE == FLOATS) w = __uint_as_float(x[u].y);
-        else w = x[u].y;
-        ok &= sum_add(keys, vals, CS, hash_hi(x[u].x, MERGE_LOGS), x[u].x, w);
+        if constexpr (MODE == FLOATS) w = __uint_as_float(v[u]);
+        else w = v[u];
+        ok &= sum_add(keys, vals, CS, hash_hi(x[u], MERGE_LOGS), x[u], w);
       }
     }
     b = nb;
@@ -566,19 +574,31 @@ __global__ void __launch_bounds__(B) agg_merge_kernel(AggArgs a, AggChunks ch) {
   __syncthreads();
   if (threadIdx.x == 0) s_at = s_n ? atomicAdd(&a.ydeg[c], s_n) : 0u;  // the partition's place in the row
   __syncthreads();
-  const uint64_t y0 = a.yoff[c];
+  uint2 *out = ch.merged + ch.merged_off[j];
   for (uint32_t s = threadIdx.x; s < CS; s += B) {
     const uint32_t k = keys[s];
     const unsigned bal = __ballot_sync(0xffffffffu, k != EMPTY);
     uint32_t at = 0;
     if (lane == 0 && bal) at = atomicAdd(&s_at, uint32_t(__popc(bal)));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
-    if (k != EMPTY) {
-      a.ykey[y0 + at] = k;
-      a.yw[y0 + at] = value<MODE>(vals[s]);
-    }
+    if (k != EMPTY) out[at] = make_uint2(k, __float_as_uint(value<MODE>(vals[s])));
   }
   if (!ok) atomicOr(&a.ctr->err, ERR_TABLE_FULL);
+}
+
+// The merged rows to their places: a block per (community, partition) as
+// above, each a stretch of AGG_PART entries (and those that many partitions on).
+__global__ void __launch_bounds__(256) agg_place_kernel(AggArgs a, AggChunks ch) {
+  const uint2 task = ch.merge[blockIdx.x];
+  const uint32_t j = task.x, c = ch.comm[j], n = a.ydeg[c];
+  const uint64_t y0 = a.yoff[c];
+  const uint2 *in = ch.merged + ch.merged_off[j];
+  for (uint64_t b = uint64_t(task.y) * AGG_PART; b < n; b += uint64_t(ch.parts[j]) * AGG_PART)
+    for (uint64_t i = b + threadIdx.x; i < min(uint64_t(n), b + AGG_PART); i += 256) {
+      const uint2 x = __ldcs(in + i);
+      a.ykey[y0 + i] = x.x;
+      a.yw[y0 + i] = __uint_as_float(x.y);
+    }
 }
 
 __global__ void comm_tdeg_kernel(const uint32_t *list, size_t n, const uint64_t *yoff, uint64_t *out) {
@@ -656,6 +676,8 @@ void launch_chunks(const AggArgs &a, const AggChunks &ch, size_t runs, size_t me
   k1<<<unsigned(runs), AGG_CHUNK_B, smem1 + size_t(max_parts) * 4, s>>>(a, ch);  // (the partitions' counters behind)
   LVG_CHECK_LAUNCH();
   k2<<<unsigned(merges), AGG_MERGE_B, smem2, s>>>(a, ch);
+  LVG_CHECK_LAUNCH();
+  agg_place_kernel<<<unsigned(merges), 256, 0, s>>>(a, ch);
   LVG_CHECK_LAUNCH();
 }
 

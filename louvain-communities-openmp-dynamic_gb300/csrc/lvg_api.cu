@@ -518,7 +518,7 @@ int lvg_graph_trim(lvg_graph *g, int level) {
       W.phase_big.release(); W.phase_heavy.release(); W.phase_mv.release(); W.phase_list.release();
       W.ht_soff.release(); W.ht_slg.release(); W.ht_skey.release(); W.ht_scnt.release(); W.ht_n.release();
       W.mpre.release(); W.agg_tdeg.release(); W.agg_plan.release();
-      W.agg_pairs.release(); W.agg_seg.release(); W.agg_lists.release();
+      W.agg_merged.release(); W.agg_seg.release(); W.agg_lists.release();
     }
     if (g->uni)
       for (auto &b : g->uni->stage.buf) b.release();

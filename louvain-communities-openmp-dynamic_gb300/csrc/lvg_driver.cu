@@ -1069,32 +1069,32 @@ Level aggregate(lvg_graph *g, const Level &lv, const uint32_t *com, size_t CN, i
       bytes += (n * elem + 15) / 16 * 16;
       return at;
     };
-    const size_t a_run = place(nrun, 16), a_merge = place(nm, 8), a_poff = place(n11, 8), a_soff = place(n11, 8),
+    const size_t a_run = place(nrun, 16), a_merge = place(nm, 8), a_moff = place(n11, 8), a_soff = place(n11, 8),
                  a_loff = place(n11, 8), a_parts = place(n11, 4);
     W.agg_hplan.ensure(bytes);  // (its last upload was waited for above)
     W.agg_plan.ensure(bytes);
     uint8_t *hp = W.agg_hplan.p;
     auto *runs = reinterpret_cast<uint4 *>(hp + a_run);
     auto *merge = reinterpret_cast<uint2 *>(hp + a_merge);
-    auto *poff = reinterpret_cast<uint64_t *>(hp + a_poff), *soff = reinterpret_cast<uint64_t *>(hp + a_soff);
+    auto *moff = reinterpret_cast<uint64_t *>(hp + a_moff), *soff = reinterpret_cast<uint64_t *>(hp + a_soff);
     auto *loff = reinterpret_cast<uint64_t *>(hp + a_loff);
     auto *parts = reinterpret_cast<uint32_t *>(hp + a_parts);
-    uint64_t c = 0, m = 0, pairs = 0, seg = 0, lists = 0;
+    uint64_t c = 0, m = 0, merged = 0, seg = 0, lists = 0;
     for (size_t j = 0; j < n11; ++j) {
       const uint64_t n = chunks_of(tdeg[j]), R = parts_of(tdeg[j]);
       for (uint64_t k = 0; k < n; k += len)
         runs[c++] = make_uint4(uint32_t(j), uint32_t(k), uint32_t(std::min(len, n - k)), 0u);
       for (uint64_t r = 0; r < R; ++r) merge[m++] = make_uint2(uint32_t(j), uint32_t(r));
-      poff[j] = pairs;
+      moff[j] = merged;
       soff[j] = seg;
       loff[j] = lists;
       parts[j] = uint32_t(R);
       lists += n;
-      pairs += n * AGG_CHUNK;
+      merged += std::min<uint64_t>(tdeg[j], CN);
       seg += n * (R + 1);
     }
     LVG_CUDA(cudaMemcpyAsync(W.agg_plan.p, hp, bytes, cudaMemcpyHostToDevice, s));
-    W.agg_pairs.ensure(pairs);
+    W.agg_merged.ensure(merged);
     W.agg_seg.ensure(seg);
     W.agg_lists.ensure(n11 + lists);
     LVG_CUDA(cudaMemsetAsync(W.agg_lists.p, 0, n11 * sizeof(uint32_t), s));
@@ -1102,11 +1102,11 @@ Level aggregate(lvg_graph *g, const Level &lv, const uint32_t *com, size_t CN, i
     a.count = uint32_t(n11);
     const uint8_t *dp = W.agg_plan.p;
     const AggChunks ch{reinterpret_cast<const uint4 *>(dp + a_run), reinterpret_cast<const uint2 *>(dp + a_merge), list,
-                       reinterpret_cast<const uint32_t *>(dp + a_parts), reinterpret_cast<const uint64_t *>(dp + a_poff),
+                       reinterpret_cast<const uint32_t *>(dp + a_parts), reinterpret_cast<const uint64_t *>(dp + a_moff),
                        reinterpret_cast<const uint64_t *>(dp + a_soff), reinterpret_cast<const uint64_t *>(dp + a_loff),
-                       W.mpre.p, W.agg_pairs.p, W.agg_seg.p, W.agg_lists.p, W.agg_lists.p + n11};
+                       W.mpre.p, W.agg_merged.p, W.agg_seg.p, W.agg_lists.p, W.agg_lists.p + n11};
     launch_aggregate_chunks(a, ch, nrun, nm, uint32_t(max_parts), s);
-    g->stats.aggregate_launches += 2;
+    g->stats.aggregate_launches += 3;
   }
   for (int i = 0; i < 4; ++i) {  // join
     LVG_CUDA(cudaEventRecord(g->join_ev[i], g->aux[i]));

@@ -73,12 +73,12 @@ struct Workspace {
   DBuf<uint32_t> ht_skey, ht_scnt, ht_n;
   HubTabView ht_now;
   // chunked aggregation of the largest communities: the plan (one pinned block,
-  // uploaded in one copy), the chunks' pairs and their groups' bounds
+  // uploaded in one copy), the merged rows and the bounds of the lists' groups
   DBuf<uint64_t> mpre, agg_tdeg;
   DBuf<uint8_t> agg_plan;
   HBuf<uint8_t> agg_hplan;
   HBuf<uint64_t> agg_htdeg;
-  DBuf<uint2> agg_pairs;
+  DBuf<uint2> agg_merged;
   DBuf<uint32_t> agg_seg, agg_lists;
 
   void allocate(size_t S_, size_t X_, cudaStream_t st) {

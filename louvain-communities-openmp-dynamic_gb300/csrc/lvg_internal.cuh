@@ -439,9 +439,10 @@ struct AggArgs {
 // prefix of member degrees in member-list order. Blocks take runs of its
 // chunks and write lists of (community, weight) pairs: nlist[j] of them (at
 // most a list per chunk), list i from chunk f = list_at[list_off[j] + i] on,
-// its pairs at part_off[j] + f * AGG_CHUNK. Its neighbour communities fall into
-// parts[j] hash partitions (at most AGG_MAX_PARTS), by which a list is grouped:
-// the groups' bounds are at seg_off[j] + i * (parts[j] + 1).
+// its pairs in the community's row from entry f * AGG_CHUNK on. Its neighbour
+// communities fall into parts[j] hash partitions (at most AGG_MAX_PARTS), by
+// which a list is grouped: the groups' bounds are at seg_off[j] + i * (parts[j]
+// + 1). The merged row is at merged_off[j] until it takes the lists' place.
 constexpr uint32_t AGG_CHUNK = 4096;
 constexpr uint32_t AGG_PART = 8192;  // distinct communities a partition is meant to hold
 constexpr uint32_t AGG_MAX_PARTS = 20480;
@@ -450,9 +451,9 @@ struct AggChunks {
   const uint2 *merge;        // [merges] (community slot, partition)
   const uint32_t *comm;      // [n]
   const uint32_t *parts;
-  const uint64_t *part_off, *seg_off, *list_off;
+  const uint64_t *merged_off, *seg_off, *list_off;
   const uint64_t *mpre;      // [members+1]
-  uint2 *pairs;
+  uint2 *merged;
   uint32_t *seg, *nlist, *list_at;  // nlist zeroed
 };
 
