@@ -1025,6 +1025,24 @@ Level aggregate(lvg_graph *g, const Level &lv, const uint32_t *com, size_t CN, i
   ensure_aux(g);
   LVG_CUDA(cudaEventRecord(g->fork_ev, s));
   for (int i = 0; i < 4; ++i) LVG_CUDA(cudaStreamWaitEvent(g->aux[i], g->fork_ev, 0));
+  // the join, also when an allocation below fails: what the main stream does
+  // next must not meet kernels of this call on the same buffers
+  struct Join {
+    lvg_graph *g;
+    cudaStream_t s;
+    bool open = true;
+    cudaError_t close() {
+      open = false;
+      cudaError_t first = cudaSuccess;
+      for (int i = 0; i < 4; ++i)
+        for (cudaError_t e : {cudaEventRecord(g->join_ev[i], g->aux[i]), cudaStreamWaitEvent(s, g->join_ev[i], 0)})
+          if (first == cudaSuccess) first = e;
+      return first;
+    }
+    ~Join() {
+      if (open) close();
+    }
+  } join{g, s};
   for (int b = NUM_BINS - 2; b >= 1; --b) {
     const size_t cnt = cb[b + 1] - cb[b];
     if (!cnt) continue;
@@ -1108,10 +1126,7 @@ Level aggregate(lvg_graph *g, const Level &lv, const uint32_t *com, size_t CN, i
     launch_aggregate_chunks(a, ch, nrun, nm, uint32_t(max_parts), s);
     g->stats.aggregate_launches += 3;
   }
-  for (int i = 0; i < 4; ++i) {  // join
-    LVG_CUDA(cudaEventRecord(g->join_ev[i], g->aux[i]));
-    LVG_CUDA(cudaStreamWaitEvent(s, g->join_ev[i], 0));
-  }
+  LVG_CUDA(join.close());
   if (g->profiling) {
     e1 = g->events.record(s);
   }
