@@ -166,7 +166,7 @@ __global__ void fill_f32_kernel(float *p, size_t n, float v) {
 __device__ __forceinline__ void group_add(tot_t *p, uint32_t key, double x, int lane) {
   const unsigned grp = __match_any_sync(0xffffffffu, key);
   double sum = 0.0;
-  for (unsigned r = grp; r; r &= r - 1u) sum += __shfl_sync(grp, x, __ffs(r) - 1);
+  for (unsigned r = key != EMPTY ? grp : 0u; r; r &= r - 1u) sum += __shfl_sync(grp, x, __ffs(r) - 1);
   if (key != EMPTY && (grp & ((1u << lane) - 1u)) == 0u) atomicAdd(p + key, sum);
 }
 
@@ -993,13 +993,25 @@ __global__ void count_flags_kernel(const uint8_t *f, size_t n, unsigned long lon
 // vertices of a warp's round whose communities are equal add their weights
 // first (a large community would take an atomic per member on one address).
 // Ids that are no vertex are flagged (ERR_BAD_ID) and left out.
+// A block takes V vertices at a time, few enough that every SM gets some
+// (mod_vertices), and a weighted row's pieces are longer, since each piece ends
+// in an FP64 reduction over the warp. (Calls on weighted planted partitions of
+// 50000 vertices of degree 300, 20000 of 1500 and 5000 of 2000: 0.19, 0.23 and
+// 0.10 ms, as with a warp per row; with 256 vertices and pieces of 128 entries
+// everywhere 0.46, 0.65 and 0.54. R-MAT scale 22 with weights: 2.6 ms, a warp
+// per row 5.5.)
 constexpr uint32_t MOD_LONG = 128;
 constexpr int MOD_B = 256;
+uint32_t mod_vertices(size_t span) {
+  uint32_t V = MOD_B;
+  while (V > 8 && span / V < size_t(device_sms()) * 8) V /= 2;
+  return V;
+}
 template <bool UNIT>
 __global__ void __launch_bounds__(MOD_B) modularity_kernel(const uint64_t *off, const uint32_t *deg, const uint32_t *key,
                                                            const float *w, const uint8_t *ex, size_t n,
-                                                           const uint32_t *memb, double *ctot64, double *intra,
-                                                           unsigned int *err) {
+                                                           const uint32_t *memb, uint32_t V, double *ctot64,
+                                                           double *intra, unsigned int *err) {
   using A = typename std::conditional<UNIT, unsigned long long, double>::type;
   __shared__ uint32_t s_long[MOD_B];
   __shared__ double s_tot[MOD_B];  // a vertex's weight
@@ -1024,19 +1036,20 @@ __global__ void __launch_bounds__(MOD_B) modularity_kernel(const uint64_t *off, 
       for (int q = 0; q < 4; ++q) {
         if constexpr (UNIT) {
           in += m[q] == c;
-        } else {
-          tot += double(x[q]);
-          if (m[q] == c) in += double(x[q]);
+        } else if (__any_sync(__activemask(), m[q] != EMPTY)) {
+          const double y = double(x[q]);
+          tot += y;
+          if (m[q] == c) in += y;
         }
       }
     }
   };
-  // a block takes 256 vertices at a time: their rows, then their totals
-  for (size_t base = size_t(blockIdx.x) * MOD_B; base < n; base += size_t(gridDim.x) * MOD_B) {
+  // a block takes V vertices at a time: their rows, then their totals
+  for (size_t base = size_t(blockIdx.x) * V; base < n; base += size_t(gridDim.x) * V) {
     if (threadIdx.x == 0) s_n = 0;
     if constexpr (!UNIT) s_tot[threadIdx.x] = 0.0;
     __syncthreads();
-    for (uint32_t r = threadIdx.x / 8; r < MOD_B && base + r < n; r += MOD_B / 8) {
+    for (uint32_t r = threadIdx.x / 8; r < V && base + r < n; r += MOD_B / 8) {
       const size_t u = base + r;
       const uint32_t d = !ex || ex[u] ? deg[u] : 0u, c = memb[u];
       if (d > MOD_LONG) {
@@ -1053,25 +1066,28 @@ __global__ void __launch_bounds__(MOD_B) modularity_kernel(const uint64_t *off, 
     }
     __syncthreads();
     const uint32_t nl = s_n;
-    constexpr uint32_t W = MOD_B / 32;
+    constexpr uint32_t W = MOD_B / 32, PIECE = UNIT ? 128 : 2048;
     for (uint32_t i = 0; i < nl; ++i) {
       const size_t u = base + s_long[i];
       const uint64_t o = off[u];
       const uint32_t d = deg[u], c = memb[u];
       double tot = 0.0;
-      for (uint32_t p = (threadIdx.x / 32 + W - i % W) % W; p * 128u < d; p += W)
-        run(o, p * 128u + lane, min(d, (p + 1) * 128u), 32, c, tot);
+      const uint32_t first = (threadIdx.x / 32 + W - i % W) % W;  // the warp's first piece
+      if (first * PIECE >= d) continue;
+      for (uint32_t p = first; p * PIECE < d; p += W)
+        run(o, p * PIECE + lane, min(d, (p + 1) * PIECE), 32, c, tot);
       if constexpr (!UNIT) {
         tot = warp_sum_d(tot);
-        if (lane == 0 && tot != 0.0) atomicAdd(&s_tot[s_long[i]], tot);
+        if (lane == 0 && d <= PIECE) s_tot[s_long[i]] = tot;
+        else if (lane == 0 && tot != 0.0) atomicAdd(&s_tot[s_long[i]], tot);
       }
     }
     __syncthreads();
-    {
+    if (threadIdx.x - lane < V) {  // (whole warps)
       const size_t u = base + threadIdx.x;
       uint32_t c = EMPTY;
       double x = 0.0;
-      if (u < n) {
+      if (threadIdx.x < V && u < n) {
         c = memb[u];
         if (c >= n) bad = true;
         else if (!ex || ex[u]) x = UNIT ? double(deg[u]) : s_tot[threadIdx.x];
@@ -1414,12 +1430,13 @@ void launch_modularity(const Level &g, const uint32_t *memb, double *ctot64, Cou
   LVG_CUDA(cudaMemsetAsync(&ctr->fp64[1], 0, sizeof(double), s));
   LVG_CUDA(cudaMemsetAsync(ctot64, 0, g.span * sizeof(double), s));
   if (!g.span) return;
-  const int grid = grid_for(g.span, MOD_B);
+  const uint32_t V = mod_vertices(g.span);
+  const int grid = grid_for(g.span, int(V));
   if (g.unit)
-    modularity_kernel<true><<<grid, MOD_B, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, ctot64, &ctr->fp64[1],
-                                                   &ctr->err);
+    modularity_kernel<true><<<grid, MOD_B, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, V, ctot64,
+                                                   &ctr->fp64[1], &ctr->err);
   else
-    modularity_kernel<false><<<grid, MOD_B, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, ctot64,
+    modularity_kernel<false><<<grid, MOD_B, 0, s>>>(g.off, g.deg, g.key, g.w, g.ex, g.span, memb, V, ctot64,
                                                     &ctr->fp64[1], &ctr->err);
   LVG_CHECK_LAUNCH();
 }
