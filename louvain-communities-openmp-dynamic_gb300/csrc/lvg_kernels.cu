@@ -37,61 +37,66 @@ __global__ void degrees_kernel(const uint64_t *off, uint32_t *deg, size_t n) {
 // 32 lanes striding over the row and an xor tree over them (the order of the
 // sum is part of its value), each lane here standing for four of those, which
 // takes 6 FP64 additions a lane beside the row's own instead of 5 on 32 lanes.
-__device__ __forceinline__ double row_sum8(const float *w, uint32_t d, uint32_t sl) {
+// `most`: the longest of the warp's rows (the SM issues an FP64 instruction in 16
+// cycles whether or not a lane has anything to add).
+__device__ __forceinline__ double row_sum8(const float *w, uint32_t d, uint32_t sl, uint32_t most) {
   double acc[4] = {0.0, 0.0, 0.0, 0.0};
-  for (uint32_t j = sl; j < d; j += 32) {
+  for (uint32_t j = 0; j < most; j += 32) {
     float x[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) x[q] = j + 8 * q < d ? __ldcs(w + j + 8 * q) : 0.f;
+    for (int q = 0; q < 4; ++q) x[q] = j + 8 * q + sl < d ? __ldcs(w + j + 8 * q + sl) : 0.f;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) acc[q] += double(x[q]);
+    for (int q = 0; q < 4; ++q)
+      if (j + 8 * q < most) acc[q] += double(x[q]);
   }
   double s = (acc[0] + acc[2]) + (acc[1] + acc[3]);
 #pragma unroll
-  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffu << (threadIdx.x & 24u), s, o);
+  for (int o = 4; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
   return s;
 }
 
 // Calls out(u, sum) once for every vertex u with the FP64 sum of its row's
-// weights (0 where absent): eight lanes per vertex; rows above ROW_LONG
-// entries are put aside and taken a warp each.
-constexpr uint32_t ROW_LONG = 512;
+// weights (0 where absent). A warp takes up to four vertices at a time: first
+// those of its rows that are above ROW_LONG entries, one after the other, then
+// the others with eight lanes each. The four are far apart, so that neighbouring
+// long rows (the first ids of an R-MAT graph) fall to different warps, and no
+// warp waits for another; with a vertex a warp or fewer, all lanes take it. Kernel
+// times (a warp per row / eight lanes a row and the long rows shared by a
+// block's warps): planted partitions of degree 16 (131K vertices) 41 (67 / 37)
+// us, 300 (50K) 86 (84 / 77), 1500 (20K) 117 (117 / 150), 2000 (5K) 43 (45 / 65);
+// R-MAT scale 18 180 (188 / 189), 20 563 (636 / 773) us, 22 2.05 (2.58 / 2.34)
+// ms. FP64 instructions bound the long rows, the longest row's chain of
+// additions R-MAT scale 18.
+constexpr uint32_t ROW_LONG = 128;
 constexpr int ROW_B = 256;
 template <class Out>
 __device__ __forceinline__ void row_sums(const uint64_t *off, const uint32_t *deg, const float *w, const uint8_t *ex,
                                          size_t n, Out out) {
-  __shared__ uint32_t s_long[ROW_B / 8];
-  __shared__ uint32_t s_n;
-  const uint32_t sl = threadIdx.x & 7u;
-  for (size_t base = size_t(blockIdx.x) * (ROW_B / 8); base < n; base += size_t(gridDim.x) * (ROW_B / 8)) {
-    if (threadIdx.x == 0) s_n = 0;
-    __syncthreads();
-    const size_t u = base + threadIdx.x / 8;
+  const uint32_t lane = threadIdx.x & 31u, sl = lane & 7u;
+  const size_t warps = size_t(gridDim.x) * (ROW_B / 32), wid = (size_t(blockIdx.x) * ROW_B + threadIdx.x) / 32;
+  const uint32_t most8 = n <= warps ? 0u : ROW_LONG;  // (with a vertex a warp, all its lanes take it)
+  for (size_t base = wid; base < n; base += 4 * warps) {
+    const size_t u = base + (lane >> 3) * warps;
+    uint32_t d = 0;
+    uint64_t o = 0;
     if (u < n) {
-      const uint32_t d = !ex || ex[u] ? deg[u] : 0u;
-      if (d > ROW_LONG) {
-        if (sl == 0) s_long[atomicAdd(&s_n, 1u)] = uint32_t(u);
-      } else {
-        const double s = row_sum8(w + off[u], d, sl);
-        if (sl == 0) out(u, s);
-      }
+      d = !ex || ex[u] ? deg[u] : 0u;
+      o = off[u];
     }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x / 32; i < s_n; i += ROW_B / 32) {
-      const uint32_t v = s_long[i], d = deg[v];
-      const float *row = w + off[v];
+    for (unsigned rest = __ballot_sync(0xffffffffu, sl == 0 && d > most8); rest; rest &= rest - 1u) {
+      const int of = __ffs(rest) - 1;
+      const uint32_t m = __shfl_sync(0xffffffffu, d, of);
+      const float *row = w + __shfl_sync(0xffffffffu, o, of);
       double s = 0.0;
-      for (uint32_t j = threadIdx.x & 31u; j < d; j += 32 * 8) {  // eight loads in flight
-        float x[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) x[q] = j + 32 * q < d ? __ldcs(row + j + 32 * q) : 0.f;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) s += double(x[q]);
-      }
+#pragma unroll 8
+      for (uint32_t j = lane; j < m; j += 32) s += double(row[j]);
       s = warp_sum_d(s);
-      if ((threadIdx.x & 31u) == 0) out(v, s);
+      if (int(lane) == of) out(u, s);
     }
-    __syncthreads();
+    const bool some = u < n && d <= most8;
+    if (!__any_sync(0xffffffffu, some)) continue;
+    const double s = row_sum8(w + o, some ? d : 0u, sl, __reduce_max_sync(0xffffffffu, some ? d : 0u));
+    if (some && sl == 0) out(u, s);
   }
 }
 
@@ -1178,14 +1183,14 @@ void launch_init_static(const Level &g, uint32_t *ucom, tot_t *utot, tot_t *ctot
   if (g.unit)
     init_unit_kernel<<<grid_for(g.span, 256), 256, 0, s>>>(g.deg, g.ex, g.span, g.gid, g.gbase, ucom, utot, ctot);
   else
-    init_static_kernel<<<grid_for(g.span * 8, ROW_B), ROW_B, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, g.gid, g.gbase,
+    init_static_kernel<<<grid_for(g.span * 32, ROW_B), ROW_B, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, g.gid, g.gbase,
                                                                      ucom, utot, ctot);
   LVG_CHECK_LAUNCH();
 }
 
 void launch_vertex_weights_f64(const Level &g, double *vtot, cudaStream_t s) {
   if (!g.span) return;
-  vertex_weights_f64_kernel<<<grid_for(g.span * 8, ROW_B), ROW_B, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, vtot);
+  vertex_weights_f64_kernel<<<grid_for(g.span * 32, ROW_B), ROW_B, 0, s>>>(g.off, g.deg, g.w, g.ex, g.span, vtot);
   LVG_CHECK_LAUNCH();
 }
 
