@@ -90,36 +90,52 @@ __device__ __forceinline__ void add_gain(const MoveArgs &a, const GraphOf &G, un
   else fix += gain_to_fix(bg);
 }
 
-// A block's counters (all threads, once, at the kernel's end): one atomic each
-// for the whole block. Every block of every launch of a class adds to the same
-// few words: with seven atomics of every warp a launch over the degrees up to 4
-// of a class of R-MAT scale 21 took 51 us, with four of every block it takes 29.
+// A kernel's counters (all threads, once, at its end). Every block of every
+// launch of a class adds to the same few words. BLOCK: one atomic each for the
+// whole block, where a block's warps all have something to add (degrees up to
+// 128: with seven atomics of every warp a launch over the degrees up to 4 of a
+// class of R-MAT scale 21 took 51 us, with four of every block it takes 29).
+// Otherwise by warp, with no barrier and sum that end a block later: of a block
+// that takes a vertex at a time only one warp has counts (naive-dynamic on
+// 50000 vertices of degree 600: 0.50 ms with the barrier, 0.47 without).
+template <bool BLOCK>
 __device__ __forceinline__ void flush_counters(Counters *ctr, int bin, unsigned long long fix, unsigned long long nv,
                                                unsigned long long ne, unsigned long long nm, bool bad,
                                                unsigned long long no = 0) {
-  __shared__ unsigned long long part[32][5];
   unsigned long long v[5] = {fix, nv, ne, nm, no};
 #pragma unroll
   for (int x = 0; x < 5; ++x) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v[x] += __shfl_xor_sync(0xffffffffu, v[x], o);
   }
-  if ((threadIdx.x & 31) == 0) {
+  unsigned long long *to[5] = {&ctr->el_fix, &ctr->bin_vertices[bin], &ctr->bin_edges[bin], &ctr->moves,
+                               &ctr->bin_over[bin]};
+  if constexpr (BLOCK) {
+    __shared__ unsigned long long part[32][5];
+    if ((threadIdx.x & 31) == 0) {
 #pragma unroll
-    for (int x = 0; x < 5; ++x) part[threadIdx.x >> 5][x] = v[x];
+      for (int x = 0; x < 5; ++x) part[threadIdx.x >> 5][x] = v[x];
+    }
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x < 5) {
+      unsigned long long sum = 0;
+      for (uint32_t w = 0; w < blockDim.x / 32; ++w) sum += part[w][threadIdx.x];
+      unsigned long long *p = to[0];
+#pragma unroll
+      for (int x = 1; x < 5; ++x)
+        if (threadIdx.x == uint32_t(x)) p = to[x];
+      if (sum) atomicAdd(p, sum);
+    }
+    if (bad && threadIdx.x == 0) atomicOr(&ctr->err, ERR_TABLE_FULL);
+  } else {
+    bad = __any_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+      for (int x = 0; x < 5; ++x)
+        if (v[x]) atomicAdd(to[x], v[x]);
+      if (bad) atomicOr(&ctr->err, ERR_TABLE_FULL);
+    }
   }
-  const bool anybad = __syncthreads_or(bad);
-  if (threadIdx.x < 5) {
-    unsigned long long sum = 0;
-    for (uint32_t w = 0; w < blockDim.x / 32; ++w) sum += part[w][threadIdx.x];
-    unsigned long long *to = threadIdx.x == 0   ? &ctr->el_fix
-                             : threadIdx.x == 1 ? &ctr->bin_vertices[bin]
-                             : threadIdx.x == 2 ? &ctr->bin_edges[bin]
-                             : threadIdx.x == 3 ? &ctr->moves
-                                                : &ctr->bin_over[bin];
-    if (sum) atomicAdd(to, sum);
-  }
-  if (anybad && threadIdx.x == 0) atomicOr(&ctr->err, ERR_TABLE_FULL);
 }
 
 // Warp-aggregated insertion: the 32 lanes of a converged warp each hold a
@@ -306,7 +322,7 @@ __device__ __forceinline__ void tile_loop(const MoveArgs &a, const uint32_t *lis
     bad |= !ok;
     __syncwarp(m);
   }
-  flush_counters(a.ctr, bin, fix, nv, ne, nm, bad, no);
+  flush_counters<(C <= 256)>(a.ctr, bin, fix, nv, ne, nm, bad, no);
 }
 
 // Tiles with tables of up to 256 slots: registers capped for 8 resident
@@ -698,7 +714,7 @@ __global__ void __launch_bounds__(B) move_big_kernel(MoveArgs a) {
     bad |= !ok;
     __syncthreads();
   }
-  flush_counters(a.ctr, a.bin, fix, nv, ne, nm, bad, no);
+  flush_counters<false>(a.ctr, a.bin, fix, nv, ne, nm, bad, no);
 }
 
 // ------------------------------------------------------------ chunked hubs
@@ -1086,7 +1102,7 @@ __global__ void __launch_bounds__(B) hub_merge_kernel(MoveArgs a) {
     bad |= !ok;
     __syncthreads();
   }
-  flush_counters(a.ctr, a.bin, fix, nv, ne, nm, bad, no);
+  flush_counters<false>(a.ctr, a.bin, fix, nv, ne, nm, bad, no);
 }
 
 // Hub path with resident tables (MoveArgs::ht): one block per hub of the
@@ -1141,7 +1157,7 @@ __global__ void __launch_bounds__(B) hub_table_kernel(MoveArgs a) {
     }
     __syncthreads();
   }
-  flush_counters(a.ctr, NUM_BINS - 1, fix, nv, ne, nm, false, no);
+  flush_counters<false>(a.ctr, NUM_BINS - 1, fix, nv, ne, nm, false, no);
   if (threadIdx.x == 0 && slots) atomicAdd(&a.ctr->ht_slots, slots);
 }
 
