@@ -718,12 +718,37 @@ void reset_hub_scratch(lvg_graph *g) {
   if (W.hub_over.p) LVG_CUDA(cudaMemsetAsync(W.hub_over.p, 0, W.hub_over.n, s));
 }
 
+// Whether a run from a prior over the uploaded level goes launch by launch: the
+// phase kernel spares the launches (0.1-0.3 ms a phase), but has a block of 32
+// warps per SM where the launches' small blocks fill it, and large vertices
+// take it longer. `active` is the share of the vertices that the first iteration
+// looks at; the edges of a degree bin are its vertices times the bin's geometric
+// middle. Measured on both sides (ms, launches / phase kernel; planted
+// partitions, vertices x degree):
+// Asynchronous, naive: 2000 x 300 .20/.14, 10K x 600 .23/.19, 100K x 150 .53/.71,
+// 50K x 300 .50/.55, 300K x 200 1.06/1.24, 200K x 500 1.43/2.83, 9K x 3000
+// .23/.39; power laws with 7M, 13M and 29M edges above degree 128 1.21/.98,
+// .93/1.31, 1.22/2.14. Frontier of 1e-4 and 1e-3 |E|: 300K x 200 .22/.21,
+// .46/.54; 50K x 600 .27/.22, .41/.50; 9K x 3000 .16/.27, .21/.37.
+// Deterministic, naive: 100K x 150 .81/.55, 200K x 500 1.75/1.62, 20K x 1500
+// .43/.38, 300K x 200 1.26/1.38, 100K x 1000 .86/1.14, 9K x 3000 .32/.42; with
+// fractional weights 300K x 200 1.54/1.17, 100K x 1000 1.04/1.50.
+bool prefers_launches(const Level &lv, bool sync, bool whole, double active) {
+  static const double mid[NUM_BINS] = {0, 0, 0, 0, 0, 0, 0, 181, 362, 1025, 4096, 0};
+  double edges[NUM_BINS] = {};
+  for (int b = 7; b < NUM_BINS - 1; ++b)
+    for (int k = 0; k < lv.colors; ++k)
+      edges[b] += active * double(lv.bucket_size(k, b)) * std::min(mid[b], double(lv.bin_maxdeg[b]));
+  if (!sync) return edges[7] + edges[8] + edges[9] + 4 * edges[10] > 8e6;
+  return (whole ? edges[7] : 0.0) + edges[9] + 4 * edges[10] > 32e6;
+}
+
 // Enqueue a level's whole local-moving phase as one launch of the phase
 // kernel (lvg_phase.cu) and the read-back of its counters. False, having
 // enqueued nothing, when the level takes the launch-by-launch path.
 bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const tot_t *tot,
                           const uint8_t *fa, double M, float kr, int L, double E, bool sync, const UnionCall *uc,
-                          bool listed, bool from_prior) {
+                          bool listed, bool from_prior, double active) {
   Workspace &W = *g->ws;
   cudaStream_t s = g->stream;
   if (g->profiling || !g->tuning.level_graphs || L <= 0) return false;
@@ -738,6 +763,8 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   // and with it the outcome by more (1.4 % of the memberships of a scale-22
   // R-MAT graph) than two runs of one order differ (0.2-0.7 %).
   if (P.hubs && from_prior && !sync) return false;
+  if (!P.hubs && from_prior && lv.off == g->base.off && prefers_launches(lv, sync, lv.unit || lv.whole, active))
+    return false;
   if (P.hubs && (g->tuning.hub_chunk > PHASE_HUB_CHUNK || lv.bin_maxdeg[NUM_BINS - 1] > PHASE_MAX_DEGREE)) return false;
   // (a dynamic run's totals begin with the caller's, which can be any numbers)
   const bool small = g->total_weight < 2147483648.0, whole = lv.whole && small;
@@ -827,7 +854,8 @@ struct PhaseEnd {
 int move_phase(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const tot_t *tot, const uint8_t *fa,
                double M, float kr, int L, double E, bool sync, int fused, const UnionCall *uc = nullptr,
                bool iso_clear = false, PhaseEnd *end = nullptr, bool capture = true,
-               const std::function<void()> *tail = nullptr, bool *tail_done = nullptr, bool from_prior = false) {
+               const std::function<void()> *tail = nullptr, bool *tail_done = nullptr, bool from_prior = false,
+               double active = 1.0) {
   if (tail_done) *tail_done = false;
   Workspace &W = *g->ws;
   cudaStream_t s = g->stream;
@@ -844,8 +872,8 @@ int move_phase(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *ctot, const 
     }
     launch_clear_isolated_multi(iso, W.vaff.p, fa, s);
   }
-  if (enqueue_phase_kernel(g, lv, com, ctot, tot, fa, M, kr, L, E, sync, uc, iso_clear && K == 1,
-                           from_prior)) {
+  if (enqueue_phase_kernel(g, lv, com, ctot, tot, fa, M, kr, L, E, sync, uc, iso_clear && K == 1, from_prior,
+                           active)) {
     if (tail) {
       (*tail)();
       if (tail_done) *tail_done = true;
@@ -1185,6 +1213,11 @@ void run(lvg_graph *g, int method, const DBatch &b, StateRef prior, StateRef out
       if (t) t->version = ~0ull;
     }
   } unfinished{tout};
+  // the vertices a first iteration looks at, of all: a frontier run's batch marks
+  // a vertex an entry, and about as many are marked by moves
+  const double active = method == LVG_METHOD_FRONTIER
+                            ? std::min(1.0, 2.0 * double(b.nd + b.ni) / double(std::max<size_t>(1, g->base.order)))
+                            : 1.0;
   int l = 0, p = 0;
   for (int r = 0; r < rep; ++r) {
     g->events.reset();
@@ -1339,7 +1372,7 @@ void run(lvg_graph *g, int method, const DBatch &b, StateRef prior, StateRef out
         HubTabScope hts(g, first && tabs ? tout : nullptr);  // kept up to date by the first pass's moves
         m = move_phase(g, lv, com, ctot, tot, first ? fa : nullptr, M, kr, L, E, sync, fused, nullptr, ends,
                        nullptr, true, first && r == rep - 1 ? &tail : nullptr, &tail_done,
-                       method != LVG_METHOD_STATIC);
+                       method != LVG_METHOD_STATIC, active);
       }
       tl_ev.push_back({a0, tail_done ? tail_ev : g->events.record(s)});
       l += std::max(m, 1);
