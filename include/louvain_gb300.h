@@ -68,7 +68,10 @@ typedef struct lvg_options {
    * methods 8, or the graph's tuned frontier_colors for DF and DS). Vertices
    * are split into classes by a hash of their id and each iteration visits
    * the classes in turn, so most neighbours see each other's moves within
-   * the iteration, as in the reference's sequential sweep. */
+   * the iteration, as in the reference's sequential sweep. On levels whose
+   * graph is dense (the aggregated ones), where most vertices of a class are
+   * neighbours, an asynchronous run decides a class from one state too, and
+   * sweeps aggregated levels over at least 16 classes. */
   int    colors;
 } lvg_options;
 
