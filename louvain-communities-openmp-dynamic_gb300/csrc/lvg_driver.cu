@@ -766,12 +766,13 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   // one class starts from lists of its few marked vertices there
   if ((W.ht_now.key && !(sync && lv.unit)) || listed) return false;
   const HubPlan &P = lv.hub;
-  // Asynchronous runs from a prior on a level with hubs keep the launches: in
-  // which order a class's degree bins see each other's moves differs there,
-  // and with it the outcome by more (1.4 % of the memberships of a scale-22
-  // R-MAT graph) than two runs of one order differ (0.2-0.7 %).
-  if (P.hubs && from_prior && !sync) return false;
-  if (!P.hubs && from_prior && lv.off == g->base.off && prefers_launches(lv, sync, lv.unit || lv.whole, active))
+  // Asynchronous runs from a prior on an uploaded level with hubs keep the
+  // launches: in which order a class's degree bins see each other's moves
+  // differs there, and with it the outcome by more (1.4 % of the memberships of
+  // a scale-22 R-MAT graph) than two runs of one order differ (0.2-0.7 %).
+  const bool uploaded = lv.off == g->base.off;
+  if (P.hubs && from_prior && !sync && uploaded) return false;
+  if (!P.hubs && from_prior && uploaded && prefers_launches(lv, sync, lv.unit || lv.whole, active))
     return false;
   // Where most vertices of a class are neighbours (an aggregated level, whose
   // graph is nearly complete, or an uploaded one as dense), a class of an
@@ -780,7 +781,6 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   // communities that they left, and run after run of 20 iterations ended in 20
   // communities instead of 1100 (temporal drift, 4M vertices: modularity 0.74
   // against 0.7756 launch by launch and 0.7757 so).
-  const bool uploaded = lv.off == g->base.off;
   double cells = double(lv.span) * double(lv.span);  // of the adjacency matrix
   if (uploaded && g->uni) {
     cells = 0.0;
