@@ -726,13 +726,13 @@ void reset_hub_scratch(lvg_graph *g) {
   if (W.hub_over.p) LVG_CUDA(cudaMemsetAsync(W.hub_over.p, 0, W.hub_over.n, s));
 }
 
-// Whether a run from a prior over the uploaded level goes launch by launch: the
-// phase kernel spares the launches (0.1-0.3 ms a phase), but has a block of 32
-// warps per SM where the launches' small blocks fill it, and large vertices
-// take it longer. `active` is the share of the vertices that the first iteration
-// looks at; the edges of a degree bin are its vertices times the bin's geometric
-// middle. Measured on both sides (ms, launches / phase kernel; planted
-// partitions, vertices x degree):
+// Whether a run over the uploaded level goes launch by launch (runs from a prior;
+// deterministic static ones with fractional weights): the phase kernel spares
+// the launches (0.1-0.3 ms a phase), but has a block of 32 warps per SM where the
+// launches' small blocks fill it, and large vertices take it longer. `active` is
+// the share of the vertices that the first iteration looks at; the edges of a
+// degree bin are its vertices times the bin's geometric middle. Measured on both
+// sides (ms, launches / phase kernel; planted partitions, vertices x degree):
 // Asynchronous, naive: 2000 x 300 .20/.14, 10K x 600 .23/.19, 100K x 150 .53/.71,
 // 50K x 300 .50/.55, 300K x 200 1.06/1.24, 200K x 500 1.43/2.83, 9K x 3000
 // .23/.39; power laws with 7M, 13M and 29M edges above degree 128 1.21/.98,
@@ -741,14 +741,17 @@ void reset_hub_scratch(lvg_graph *g) {
 // Deterministic, naive: 100K x 150 .81/.55, 200K x 500 1.75/1.62, 20K x 1500
 // .43/.38, 300K x 200 1.26/1.38, 100K x 1000 .86/1.14, 9K x 3000 .32/.42; with
 // fractional weights 300K x 200 1.54/1.17, 100K x 1000 1.04/1.50.
-bool prefers_launches(const Level &lv, bool sync, bool whole, double active) {
+// Deterministic static runs with fractional weights: 20K x 1500 3.5/2.9, 50K x
+// 600 4.3/4.6, 100K x 1000 6.3/7.8, 9K x 3000 3.8/4.3; with whole ones the phase
+// kernel's integer totals win at every size (9K x 3000 2.5/1.7).
+bool prefers_launches(const Level &lv, bool sync, bool floats, double active) {
   static const double mid[NUM_BINS] = {0, 0, 0, 0, 0, 0, 0, 181, 362, 1025, 4096, 0};
   double edges[NUM_BINS] = {};
   for (int b = 7; b < NUM_BINS - 1; ++b)
     for (int k = 0; k < lv.colors; ++k)
       edges[b] += active * double(lv.bucket_size(k, b)) * std::min(mid[b], double(lv.bin_maxdeg[b]));
   if (!sync) return edges[7] + edges[8] + edges[9] + 4 * edges[10] > 8e6;
-  return (whole ? edges[7] : 0.0) + edges[9] + 4 * edges[10] > 32e6;
+  return (floats ? 0.0 : edges[7]) + edges[9] + 4 * edges[10] > (floats ? 28e6 : 32e6);
 }
 
 // Enqueue a level's whole local-moving phase as one launch of the phase
@@ -772,8 +775,8 @@ bool enqueue_phase_kernel(lvg_graph *g, const Level &lv, uint32_t *com, tot_t *c
   // a scale-22 R-MAT graph) than two runs of one order differ (0.2-0.7 %).
   const bool uploaded = lv.off == g->base.off;
   if (P.hubs && from_prior && !sync && uploaded) return false;
-  if (!P.hubs && from_prior && uploaded && prefers_launches(lv, sync, lv.unit || lv.whole, active))
-    return false;
+  const bool floats = !(lv.unit || lv.whole);
+  if (!P.hubs && uploaded && (from_prior || (sync && floats)) && prefers_launches(lv, sync, floats, active)) return false;
   // Where most vertices of a class are neighbours (an aggregated level, whose
   // graph is nearly complete, or an uploaded one as dense), a class of an
   // asynchronous run is decided from one state too: a vertex that counts its

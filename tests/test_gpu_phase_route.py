@@ -46,3 +46,24 @@ def test_route_and_result(cuda, lvg, n, block, degree, weights, launches):
                 assert np.array_equal(getattr(a, f), getattr(b, f)), f
         else:
             assert g.modularity(a.membership) == pytest.approx(g.modularity(b.membership), abs=0.005)
+
+
+@pytest.mark.parametrize("weights,launches", [("unit", False), ("half", True)])
+def test_static_route_and_result(cuda, lvg, weights, launches):
+    """A deterministic static run on vertices above degree 2048 goes launch by
+    launch when its weights are fractional."""
+    x = lvg.planted_partition(9000, 4500, 3200, 0.9, 7)
+    if weights == "half":
+        u = np.repeat(np.arange(x.span), np.diff(x.offsets).astype(np.int64))
+        x.weights[:] = 0.5 * (1 + (np.minimum(u, x.keys) * 7919 + np.maximum(u, x.keys) * 104729) % 4)
+    out = []
+    for graphs in (1, 0):
+        g = cuda.Graph(x)
+        cuda.set_tuning(g, level_graphs=graphs)
+        out.append(cuda.louvain_static(g, cuda.LouvainOptions(deterministic=True, maxPasses=1)))
+        if graphs:
+            assert (g.stats()["kernel_launches"] > 40) == launches
+    a, b = out
+    assert a.iterations == b.iterations
+    for f in ("membership", "vertexWeight", "communityWeight"):
+        assert np.array_equal(getattr(a, f), getattr(b, f)), f
