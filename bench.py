@@ -576,8 +576,9 @@ def run_gpu(args):
         meth = {"static": lvg.METHOD_STATIC, "nd": lvg.METHOD_NAIVE, "ds": lvg.METHOD_DELTA,
                 "df": lvg.METHOD_FRONTIER}[args.ncu_method]
         # launches one by one (no CUDA graphs: ncu lists the kernels of a
-        # graph's conditional node only as the graph), as ncu serialises them anyway
-        Y.set_profiling(True)
+        # graph's conditional node only as the graph), as ncu serialises them
+        # anyway; a static run launches its phase kernels outside graphs
+        Y.set_profiling(args.ncu_method != "static")
         lvg.run_resident(Y, meth, db, st_prior, st_out, o)  # warm-up
         lvg.profiler_start()
         for _ in range(args.ncu_steps):

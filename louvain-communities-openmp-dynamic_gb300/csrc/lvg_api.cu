@@ -301,7 +301,7 @@ int lvg_graph_clone(lvg_graph *x, lvg_graph **out) {
   std::unique_ptr<lvg_graph> g(new lvg_graph());
   lvg::AcctScope acct_(&g->bytes);
   int rc = lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(x->device));
+    LVG_CUDA(lvg::set_device(x->device));
     g->device = x->device;
     LVG_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
     cudaStream_t s = g->stream;
@@ -361,7 +361,7 @@ int lvg_graph_create_union(lvg_graph *const *graphs, size_t n, lvg_graph **out) 
   lvg::AcctScope acct_(&g->bytes);
   int rc = lvg::guarded([&] {
     using namespace lvg;
-    LVG_CUDA(cudaSetDevice(graphs[0]->device));
+    LVG_CUDA(lvg::set_device(graphs[0]->device));
     g->device = graphs[0]->device;
     LVG_CUDA(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
     cudaStream_t s = g->stream;
@@ -449,7 +449,7 @@ int lvg_static_union(lvg_graph *u, const lvg_options *o, lvg_result *results) {
   if (!u->uni) return lvg::fail(LVG_EINVAL, "not a graph union (lvg_graph_create_union)");
   return lvg::guarded([&] {
     using namespace lvg;
-    LVG_CUDA(cudaSetDevice(u->device));
+    LVG_CUDA(lvg::set_device(u->device));
     lvg_options opt;
     if (o) opt = *o; else lvg_options_default(&opt);
     const auto t0 = std::chrono::steady_clock::now();
@@ -507,7 +507,7 @@ size_t lvg_device_batch_device_bytes(const lvg_device_batch *b) { return b ? b->
 int lvg_graph_trim(lvg_graph *g, int level) {
   if (!g || level < 1 || level > 2) return lvg::fail(LVG_EINVAL, "lvg_graph_trim: bad argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     LVG_CUDA(cudaStreamSynchronize(g->stream));
     lvg::drop_graphs(g);  // the captured iteration refers to the buffers released below
     if (g->ws) {
@@ -593,7 +593,7 @@ int lvg_vertex_weights(lvg_graph *g, double *vtot) {
   lvg::AcctScope acct_(g ? &g->bytes : nullptr);
   if (!g || !vtot) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;
     const size_t S = g->base.span;
@@ -609,7 +609,7 @@ int lvg_community_weights(lvg_graph *g, const uint32_t *membership, const double
   lvg::AcctScope acct_(g ? &g->bytes : nullptr);
   if (!g || !membership || !ctot) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     const size_t S = g->base.span;
     for (size_t u = 0; u < S; ++u)
       if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
@@ -632,7 +632,7 @@ int lvg_modularity(lvg_graph *g, const uint32_t *membership, double M, double R,
   lvg::AcctScope acct_(g ? &g->bytes : nullptr);
   if (!g || !membership || !out) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     const size_t S = g->base.span;
     lvg::ensure_ws(g);
     lvg::Workspace &W = *g->ws;
@@ -655,7 +655,7 @@ int lvg_affected_vertices(lvg_graph *y, int method, const lvg_batch *b, const ui
   lvg::AcctScope acct_(y ? &y->bytes : nullptr);
   if (!y || !flags || method < 0 || method > 3) return lvg::fail(LVG_EINVAL, "bad argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(y->device));
+    LVG_CUDA(lvg::set_device(y->device));
     lvg_options opt;
     if (o) opt = *o; else lvg_options_default(&opt);
     opt.maxPasses = 0;  // initialise and mark only
@@ -689,7 +689,7 @@ int lvg_aggregate(lvg_graph *g, const uint32_t *membership, uint32_t *renumbered
   lvg::AcctScope acct_(g ? &g->bytes : nullptr);
   if (!g || !membership || !renumbered || !num_communities || !offsets) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     const size_t S = g->base.span, X = g->base.edges;
     for (size_t u = 0; u < S; ++u)
       if (membership[u] >= S) throw lvg::Error(LVG_EINVAL, "membership id >= span");
@@ -756,7 +756,7 @@ int lvg_profiler_stop(void) {
 
 int lvg_set_device(int device) {
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(device));
+    LVG_CUDA(lvg::set_device(device));
     return LVG_OK;
   });
 }
@@ -785,7 +785,7 @@ int lvg_state_create(lvg_graph *g, lvg_state **out) {
   std::unique_ptr<lvg_state> st(new lvg_state());
   lvg::AcctScope acct_(&st->bytes);
   int rc = lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     const size_t S = g->base.span;
     st->g = g;
     st->device = g->device;
@@ -805,7 +805,7 @@ int lvg_state_set(lvg_state *st, const uint32_t *q, const double *qvtot, const d
   if (!st) return lvg::fail(LVG_EINVAL, "null state");
   return lvg::guarded([&] {
     lvg_graph *g = st->g;
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg::ensure_ws(g);
     st->ht.version = ~0ull;  // its hub tables described the old membership
     lvg::upload_prior(g, q, qvtot, qctot, st->q.p, st->vt.p, st->ct.p);
@@ -818,7 +818,7 @@ int lvg_state_get(const lvg_state *st, uint32_t *membership, double *vtot, doubl
   if (!st) return lvg::fail(LVG_EINVAL, "null state");
   return lvg::guarded([&] {
     lvg_graph *g = st->g;
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     cudaStream_t s = g->stream;
     const size_t S = g->base.span;
     if (membership) LVG_CUDA(cudaMemcpyAsync(membership, st->q.p, S * 4, cudaMemcpyDeviceToHost, s));
@@ -842,7 +842,7 @@ int lvg_device_batch_create(lvg_graph *g, const lvg_batch *b, lvg_device_batch *
   std::unique_ptr<lvg_device_batch> db(new lvg_device_batch());
   lvg::AcctScope acct_(&db->bytes);
   int rc = lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg::check_batch(g, b, false);
     db->g = g;
     db->device = g->device;
@@ -867,7 +867,7 @@ int lvg_graph_apply_batch(lvg_graph *g, const lvg_batch *b, lvg_batch_buf *tidy)
        (b->num_insertions && (!tidy->ins_src || !tidy->ins_dst || !tidy->ins_w))))
     return lvg::fail(LVG_EINVAL, "lvg_graph_apply_batch: null tidy-batch array");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg::check_batch(g, b, false);
     if (tidy) tidy->num_deletions = tidy->num_insertions = 0;
     if (!b || !(b->num_deletions + b->num_insertions)) return LVG_OK;
@@ -904,7 +904,7 @@ int lvg_graph_apply_device_batch(lvg_graph *g, lvg_device_batch *b) {
   if (b->g != g) return lvg::fail(LVG_EINVAL, "the batch was created on another graph");
   if (b->applied) return lvg::fail(LVG_EINVAL, "the batch has already been applied");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     // the batch becomes the tidied batch (tidyBatchUpdateU's result), which
     // the dynamic methods then take, as main.cxx:108-125 does
     const lvg::DBatch &r = b->b;
@@ -929,7 +929,7 @@ int lvg_graph_apply_device_batch(lvg_graph *g, lvg_device_batch *b) {
 int lvg_graph_download(lvg_graph *g, uint64_t *offsets, uint32_t *keys, float *weights, uint8_t *exists) {
   if (!g || !offsets) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     cudaStream_t s = g->stream;
     const size_t S = g->base.span;
     std::vector<uint64_t> off(S);
@@ -964,7 +964,7 @@ int lvg_device_batch_generate(lvg_graph *g, size_t deletions, size_t insertions,
   std::unique_ptr<lvg_device_batch> db(new lvg_device_batch());
   lvg::AcctScope acct_(&db->bytes);
   int rc = lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     db->g = g;
     db->device = g->device;
     size_t nd = 0, ni = 0;
@@ -987,7 +987,7 @@ int lvg_device_batch_generate(lvg_graph *g, size_t deletions, size_t insertions,
 int lvg_device_batch_download(const lvg_device_batch *b, lvg_batch_buf *out) {
   if (!b || !out) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(b->device));
+    LVG_CUDA(lvg::set_device(b->device));
     const lvg::DBatch &d = b->b;
     cudaStream_t s = b->g->stream;
     auto get = [&](void *dst, const void *src, size_t bytes) {
@@ -1015,7 +1015,7 @@ int lvg_device_batch_set(lvg_device_batch *db, const lvg_batch *b) {
   lvg_graph *g = db->g;
   lvg::AcctScope acct_(&db->bytes);
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg::check_batch(g, b, false);
     lvg::upload_batch(g, b, db->ds, db->dd, db->dw, db->is, db->id, db->iw, db->seg, db->b);
     bool sorted = true;
@@ -1049,7 +1049,7 @@ int lvg_graph_set_tuning(lvg_graph *g, const lvg_tuning *t) {
   lvg::AcctScope acct_(g ? &g->bytes : nullptr);
   if (!g || !t) return lvg::fail(LVG_EINVAL, "null argument");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     LVG_CUDA(cudaStreamSynchronize(g->stream));
     lvg::apply_tuning(g, *t);
     return LVG_OK;
@@ -1066,7 +1066,7 @@ int lvg_autotune(lvg_graph *g, int method, const lvg_device_batch *b, const lvg_
   if ((b && b->g != g) || (prior && prior->g != g)) return lvg::fail(LVG_EINVAL, "state/batch belongs to another graph");
   return lvg::guarded([&] {
     using namespace lvg;
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg_options opt;
     if (o) opt = *o; else lvg_options_default(&opt);
     opt.repeat = 1;
@@ -1224,7 +1224,7 @@ int lvg_run_resident(lvg_graph *g, int method, const lvg_device_batch *b, const 
   if (method == LVG_METHOD_DELTA && b && b->b.max_group == ~size_t(0))
     return lvg::fail(LVG_EINVAL, "delta-screening needs insertions sorted by source vertex");
   return lvg::guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(lvg::set_device(g->device));
     lvg_options opt;
     if (o) opt = *o; else lvg_options_default(&opt);
     lvg::DBatch db;

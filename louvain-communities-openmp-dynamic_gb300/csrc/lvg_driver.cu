@@ -1752,7 +1752,7 @@ int run_host(lvg_graph *g, int method, const lvg_batch *b, const uint32_t *q, co
   AcctScope acct_(g ? &g->bytes : nullptr);
   if (!g || !out) return fail(LVG_EINVAL, "null graph or result");
   return guarded([&] {
-    LVG_CUDA(cudaSetDevice(g->device));
+    LVG_CUDA(set_device(g->device));
     // a copy left in flight by a call that failed
     if (g->copy_stream) LVG_CUDA(cudaStreamSynchronize(g->copy_stream));
     lvg_options opt;

@@ -415,6 +415,7 @@ int fail(int code, const std::string &msg);
 // Runs f, turning exceptions into return codes and last-error messages.
 template <class F>
 int guarded(F &&f) {
+  const CallScope call;
   try {
     g_err.clear();
     return f();

@@ -61,6 +61,32 @@ struct DBuf {
   }
 };
 
+// The calling thread's current device: asked for once in a C-ABI call (CallScope,
+// which set_device() tells of a change), since every launch wants it.
+inline int &call_device() {
+  static thread_local int dev = -2;  // -2: outside of a call, -1: not asked for yet
+  return dev;
+}
+inline int current_device() {
+  int &dev = call_device();
+  if (dev >= 0) return dev;
+  int d = 0;
+  LVG_CUDA(cudaGetDevice(&d));
+  if (dev == -1) dev = d;
+  return d;
+}
+inline cudaError_t set_device(int d) {
+  if (call_device() != -2) call_device() = -1;
+  return cudaSetDevice(d);
+}
+struct CallScope {
+  int outer = call_device();
+  CallScope() { call_device() = -1; }
+  ~CallScope() { call_device() = outer == -2 ? -2 : -1; }
+  CallScope(const CallScope &) = delete;
+  CallScope &operator=(const CallScope &) = delete;
+};
+
 // A value of each device, made by the first call on it: a kernel's attributes
 // and the blocks that fit belong to a device, and handles of one process may
 // live on several (lvg_set_device).
@@ -71,8 +97,7 @@ struct PerDevice {
   T value[KEPT];
   template <class Make>
   T get(Make make) {
-    int dev = 0;
-    LVG_CUDA(cudaGetDevice(&dev));
+    const int dev = current_device();
     if (dev >= KEPT) return make();
     std::call_once(made[dev], [&] { value[dev] = make(); });
     return value[dev];
