@@ -481,7 +481,8 @@ typedef struct lvg_tuning {
   int      level_graphs;       /* 1: a level's local-moving phase runs as one launch with the stop
                                   test on the device: a cooperative kernel that sweeps every
                                   colour class of every iteration, or, on levels it does not serve
-                                  (asynchronous dynamic runs on hubs, hub_chunk above 4096), the iterations
+                                  (asynchronous dynamic runs on hubs, dynamic runs whose work lies
+                                  in large vertices, hub_chunk above 4096), the iterations
                                   after the first as one CUDA graph (a conditional while node)
                                   built for that level; 0: one launch sequence and one
                                   synchronisation per iteration (same results; default 1) */

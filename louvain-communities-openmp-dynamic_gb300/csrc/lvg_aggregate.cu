@@ -18,9 +18,9 @@
 // the members' edge lists are flattened with a tile prefix scan over member
 // degrees, so lanes stay busy whatever the member degrees are; blocks of 64 to
 // 1024 threads with shared tables up to 8192, where a few lanes take a member
-// and warps the pieces of a long row; chunks on many blocks above. Internal edges (into the
-// community itself, the hottest key) are summed privately per lane and added
-// once.
+// and warps the pieces of a long row; chunks on many blocks above. Internal
+// edges (into the community itself, the hottest key) are summed privately per
+// lane and added once.
 #include <type_traits>
 
 #include "lvg_internal.cuh"
@@ -384,8 +384,9 @@ __global__ void __launch_bounds__(B) agg_group_kernel(AggArgs a) {
 // tables: level 0 4.7 -> 2.9 ms, scale 18 2.4 -> 0.1 ms (too few chunks to hide
 // the atomics); a fixed eight lanes per list in the merge took 11 ms where a
 // community has two partitions.
-// Partitions take every bit of the id (two multiply-and-shift rounds), unlike
-// the tables' slots.
+// Partitions take every bit of the id (two multiply-and-shift rounds: lowbias32,
+// published by Chris Wellons), unlike the tables' slots (chunk_slot: the high bits
+// after one multiplication by MurmurHash3's 0x85EBCA6B).
 __device__ __forceinline__ uint32_t part_of(uint32_t c, uint32_t R) {
   c = (c ^ (c >> 16)) * 0x7FEB352Du;
   c = (c ^ (c >> 15)) * 0x846CA68Bu;

@@ -23,19 +23,20 @@
 //      memory;
 //   3. deterministic mode: waits until every block has decided, then commits
 //      its own decisions (community, totals) and marks the movers' neighbours.
-//      Asynchronous mode commits at once.
+//      Asynchronous mode commits at once, on sparse uploaded levels; dense and
+//      aggregated ones are decided as in deterministic mode.
 // Where every weight is 1, or a whole number (the aggregated levels of a
 // unit-weight graph), the tables add with integer shared-memory atomics
 // (native) instead of FP32 ones (a compare-and-swap loop); the sums are exact,
 // so the gains are those of exact FP32 sums.
 //
-// Measured on a GB300, deterministic static runs, launches -> this kernel: 2K
-// vertices 4.1 -> 1.8 ms, 131K-vertex planted partition 13 -> 4.3 ms, R-MAT
-// scale 20 20.4 -> 13.0 ms, scale 23 126 -> 76 ms (its two large levels' moving
-// 44 + 37 -> 21 + 20 ms). A class of a small level takes about 9 us: 1 to list,
-// 3-4 to decide, 1 to commit, 2 a barrier; of a large one, what its gathers
-// take (ncu, scale 21: warps wait at the groups' barriers and on gathers, 19 %
-// of issue slots busy).
+// Measured on a GB300, deterministic static runs, launches -> this kernel with
+// the aggregation beside it: 2K vertices 4.3 -> 1.7 ms, 131K-vertex planted
+// partition 17.5 -> 3.7 ms, R-MAT scale 20 21.7 -> 8.9 ms, scale 23 129 -> 51 ms
+// (its two large levels' moving 44 + 37 -> 17 + 17 ms). A class of a small level
+// takes about 9 us: 1 to list, 3-4 to decide, 1 to commit, 2 a barrier; of a
+// large one, what its gathers take (ncu, scale 20: warps wait at the groups'
+// barriers and on gathers, 22 % of issue slots busy).
 // Tried and dropped: tables of 1.5x instead of 2x to 4x the degree on half
 // blocks (the longest probe of a warp decides: 21 -> 29 ms), one code copy for
 // all group sizes (20.7 -> 21.6 ms), the next vertex's offset and degree
@@ -307,7 +308,8 @@ struct Of {
 // The hash partition (of R) of a hub's community. Every bit of the id takes
 // part (two multiply-and-shift rounds), so that no pattern of ids gathers in
 // one partition; unlike the tables' slots, which are the high bits of one
-// multiplication.
+// multiplication. (The mixer is lowbias32, published by Chris Wellons; the slots'
+// factor is MurmurHash3's 0x85EBCA6B.)
 __device__ __forceinline__ uint32_t hub_part(uint32_t c, uint32_t R) {
   c = (c ^ (c >> 16)) * 0x7FEB352Du;
   c = (c ^ (c >> 15)) * 0x846CA68Bu;
@@ -1097,10 +1099,11 @@ __global__ void __launch_bounds__(PB, 1) phase_kernel(const __grid_constant__ Ph
       } else {
         // light vertices first: they see a class's heavy moves an iteration
         // later and the heavy ones see theirs at once, as in the reference's
-        // sweep most vertices do. (Static runs of R-MAT scale 24: modularity
-        // 0.0598 on average of 65 and 0.0581 at worst, against 0.0586 and
-        // 0.0566 with heavy first and totals through L1, and 0.0596 and 0.0554
-        // for the launches.)
+        // sweep most vertices do. (Static runs of R-MAT scale 24, this level
+        // alone asynchronous: modularity 0.0602 on average of 8 and 0.0594 at
+        // worst; every level so 0.0594 and 0.0576, the launches 0.0596 and
+        // 0.0584; on another graph of the scale heavy first and totals through
+        // L1 0.0586 on average of 65, light first and past L1 0.0598.)
         units();
         fours();
         __syncthreads();
